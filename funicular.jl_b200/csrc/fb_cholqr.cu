@@ -28,8 +28,9 @@ void gram_chunks(int64_t rows, int kA, int kB, bool hermitian, int64_t* chunk_ro
 int gram_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
                           bool hermitian, void* workspace, size_t workspace_bytes, cudaStream_t stream,
                           const ChainStatus* st, int gate, int chunk0, int chunk1);
-int gram_reduce_enqueue(z64* C, int64_t ldc, int64_t rows, int kA, int kB, bool hermitian, z64 alpha, z64 beta,
-                        void* workspace, cudaStream_t stream, const ChainStatus* st, int gate);
+int gram_reduce_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
+                        int kB, bool hermitian, z64 alpha, z64 beta, void* workspace, cudaStream_t stream,
+                        const ChainStatus* st, int gate);
 int trsm_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
                  size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st, int gate);
 size_t trsm_workspace_bytes(int k);
@@ -581,7 +582,7 @@ int fb_zcholqr2_staged(void* const* host_panels, int host_type, const int64_t* h
         FB_TRY(gram_partials_enqueue(Yz, ldy, Yz, ldy, N, k, k, true, gram_ws, gram_bytes, stream, st, GATE_HEALTHY,
                                      B.c0[b], B.c0[b + 1]));
     }
-    FB_TRY(gram_reduce_enqueue(G, k, N, k, k, true, one, zero, gram_ws, stream, st, GATE_HEALTHY));
+    FB_TRY(gram_reduce_enqueue(G, k, Yz, ldy, Yz, ldy, N, k, k, true, one, zero, gram_ws, stream, st, GATE_HEALTHY));
     FB_TRY(potrf_enqueue(G, k, k, N, U, k, nullptr, k, Ra, k, gwork, st, 1, GATE_HEALTHY, stream,
                          shift_unit_roundoff));
     FB_TRY(trsm_enqueue(Yz, ldy, N, k, U, k, trsm_ws, trsm_bytes, stream, st, GATE_HEALTHY));

@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "fb_common.cuh"
+#include "fb_gram_split.cuh"
 #include "fb_tma.cuh"
 
 namespace fb {
@@ -44,6 +45,23 @@ constexpr int GS_BOX_ROWS = 8;          // complex rows per TMA box (128 bytes)
 constexpr int GS_BOXES = GS_ROWS / GS_BOX_ROWS;
 constexpr int G_TILE = 64;              // columns per output tile side, at most
 constexpr int G_MAX_WARPS = 17;         // 16 consumers + the producer
+
+// Set when the split form ran first: its sums and one verdict per tile. The
+// FP64 kernels then return at once unless a verdict refuses the sums. A strict
+// split (the tensor-core entry points) has no FP64 kernels behind it and only
+// an invalid result is refused.
+struct SplitGate {
+    const int* verdict;
+    const double* sums;
+    int ntiles;
+    int strict;
+    __device__ bool accepted() const {
+        if (verdict == nullptr) return false;
+        int any = 0;
+        for (int t = 0; t < ntiles; ++t) any |= verdict[t];
+        return strict ? (any & SPLIT_INVALID) == 0 : any == 0;
+    }
+};
 
 struct GramShape {
     int tw_a, tw_b;      // tile widths in columns (multiples of 8, at most 64)
@@ -85,8 +103,8 @@ template <int PPW>
 __global__ void __launch_bounds__(PPW >= 8 ? 9 * 32 : PPW == 3 ? 13 * 32 : G_MAX_WARPS * 32, 1)
 gram_dmma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  int64_t rows, GramShape sh, GramLaunch ln, z64* __restrict__ partial,
-                 const ChainStatus* st, int gate, int chunk0) {
-    if (gated_off(st, gate)) return;
+                 const ChainStatus* st, int gate, int chunk0, SplitGate split) {
+    if (gated_off(st, gate) || split.accepted()) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // Aligned for the 128-byte swizzle by pointer arithmetic on the shared
     // array itself, so the compiler keeps seeing a shared-memory pointer and
@@ -302,24 +320,11 @@ gram_dmma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
 }
 
-// One warp per entry of C: lane l adds chunks l, l+32, ... in order, then a
-// fixed shuffle tree adds the lanes.
-__global__ void gram_reduce_kernel(z64* __restrict__ C, int64_t ldc, int kA, int kB, GramShape sh,
-                                   const z64* __restrict__ partial, z64 alpha, z64 beta,
-                                   const ChainStatus* st, int gate) {
-    if (gated_off(st, gate)) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t entry = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (entry >= (int64_t)kA * kB) return;
-    const int i = (int)(entry % kA), j = (int)(entry / kA);
-    int si = i, sj = j;
-    bool mirror = false;
-    if (sh.hermitian && i > j) { si = j; sj = i; mirror = true; }
-    const int ti = si / sh.tw_a, tj = sj / sh.tw_b;
-    const int li = si - ti * sh.tw_a, lj = sj - tj * sh.tw_b;
-    int tile;
-    if (sh.hermitian) tile = (ti == tj) ? ti : off_tile_index(sh.nt_a, ti, tj);
-    else tile = ti * sh.nt_b + tj;
+// Entry (li, lj) of a tile summed over the chunks by one warp: lane l adds
+// chunks l, l+32, ... in order, then a fixed shuffle tree adds the lanes (the
+// sum is lane 0's).
+__device__ __forceinline__ z64 gram_chunk_sum(const GramShape& sh, const z64* __restrict__ partial, int tile, int ti,
+                                              int tj, int li, int lj, int lane) {
     const size_t tile_entries = (size_t)(sh.tw_a * sh.tw_b);
     const z64* src = partial + (size_t)tile * sh.nchunks * tile_entries + lj * sh.tw_a + li;
     // A diagonal 8 x 8 block of a folded tile holds S = Re + Im: Re and Im
@@ -339,8 +344,45 @@ __global__ void gram_reduce_kernel(z64* __restrict__ C, int64_t ldc, int kA, int
         s.x += __shfl_down_sync(0xffffffffu, s.x, off);
         s.y += __shfl_down_sync(0xffffffffu, s.y, off);
     }
-    if (lane != 0) return;
     if (sblock) s = (li == lj) ? zmake(s.x, 0.0) : zmake(0.5 * (s.x + s.y), 0.5 * (s.x - s.y));
+    return s;
+}
+
+// One warp per entry of C.
+__global__ void gram_reduce_kernel(z64* __restrict__ C, int64_t ldc, int kA, int kB, GramShape sh,
+                                   const z64* __restrict__ partial, z64 alpha, z64 beta,
+                                   SplitGate split, const ChainStatus* st, int gate) {
+    if (gated_off(st, gate)) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t entry = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (entry >= (int64_t)kA * kB) return;
+    const int i = (int)(entry % kA), j = (int)(entry / kA);
+    int si = i, sj = j;
+    bool mirror = false;
+    if (sh.hermitian && i > j) { si = j; sj = i; mirror = true; }
+    const int ti = si / sh.tw_a, tj = sj / sh.tw_b;
+    const int li = si - ti * sh.tw_a, lj = sj - tj * sh.tw_b;
+    int tile;
+    if (sh.hermitian) tile = (ti == tj) ? ti : off_tile_index(sh.nt_a, ti, tj);
+    else tile = ti * sh.nt_b + tj;
+    z64 s = zmake(0.0, 0.0);
+    const bool from_split = split.accepted();
+    if (split.strict && !from_split) {
+        if (lane == 0) s = zmake(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
+    } else if (from_split) {
+        // Re and Im of a folded tile are the symmetric and antisymmetric parts
+        // of S = Re + Im.
+        const double* t = split.sums + (size_t)tile * SPLIT_TILE_DOUBLES;
+        if (sh.hermitian && ti == tj) {
+            const double a = t[lj * 128 + li], b = t[li * 128 + lj];
+            s = li == lj ? zmake(a, 0.0) : zmake(0.5 * (a + b), 0.5 * (a - b));
+        } else {
+            s = zmake(t[lj * 128 + li], t[lj * 128 + 64 + li]);
+        }
+    } else {
+        s = gram_chunk_sum(sh, partial, tile, ti, tj, li, lj, lane);
+    }
+    if (lane != 0) return;
     if (mirror) s.y = -s.y;
     if (sh.hermitian && i == j) s.y = 0.0;
     z64 out = zmul(alpha, s);
@@ -505,11 +547,11 @@ static int gram_ctas_per_sm(int64_t rows, int kA, int kB, bool hermitian) {
 template <int PPW>
 static int launch_gram_dmma(const CUtensorMap& ma, const CUtensorMap& mb, int64_t rows, const GramShape& sh,
                             const GramLaunch& ln, z64* partial, cudaStream_t stream, const ChainStatus* st, int gate,
-                            int chunk0, int chunk1) {
+                            int chunk0, int chunk1, const SplitGate& split) {
     FB_TRY(set_gram_attr<PPW>(ln.smem));
     dim3 grid(ln.ntiles, chunk1 - chunk0);
     gram_dmma_kernel<PPW><<<grid, (ln.consumers + 1) * 32, ln.smem, stream>>>(ma, mb, rows, sh, ln, partial, st, gate,
-                                                                              chunk0);
+                                                                              chunk0, split);
     FB_LAUNCHED("gram_dmma_kernel");
     return FB_OK;
 }
@@ -522,31 +564,67 @@ static GramShape gram_plan(int64_t rows, int kA, int kB, bool hermitian) {
     return gram_shape(rows, kA, kB, hermitian ? 1 : 0, gram_ctas_per_sm(rows, kA, kB, hermitian));
 }
 
+// Whether the Gram of this shape runs in the split form (fb_ozaki_gram.cu).
+// It costs whole 64 x 64 tiles whatever the columns, and some 20 us more in
+// fixed work than the FP64 kernels (scales, drains, verdict, two more
+// launches), so narrow and short products stay in FP64. Microseconds, FP64 /
+// split, on both sides of the lines drawn here:
+//   folded, 1e6 rows: k = 32 207 / 320, k = 40 367 / 320, k = 64 535 / 326;
+//   folded, k = 64: 1e5 rows 70 / 73, 2e5 rows 122 / 103;
+//   folded, k = 128: 5e4 rows 141 / 136, 1e5 rows 243 / 189;
+//   cross, 1e6 rows: 32 x 32 282 / 511, 40 x 40 507 / 526, 48 x 48 568 / 517,
+//   64 x 64 933 / 563; 64 x 64: 5e4 rows 65 / 64, 1e5 rows 113 / 89.
+static bool gram_takes_split(int64_t rows, int kA, int kB, bool hermitian) {
+    if (rows > ((int64_t)1 << 30)) return false;   // the tile loads' 32-bit coordinates
+    const int a = kA < G_TILE ? kA : G_TILE, b = kB < G_TILE ? kB : G_TILE;
+    if (hermitian) return kA > G_TILE ? rows >= 60000 : (kA > 40 && rows >= 150000);
+    return a * b >= 48 * 48 && rows >= 60000;
+}
+
+// The workspace of a split Gram: the split's own layout, whose partial tiles
+// share their memory with those of the FP64 kernels behind it.
+static size_t split_gram_workspace_bytes(const SplitShape& ss, const GramShape& sh) {
+    const SplitLayout L = split_layout(ss);
+    return std::max(L.total, L.partial + gram_workspace_bytes(sh));
+}
+
+static SplitGate split_gate(const SplitShape& ss, const void* workspace, bool strict) {
+    const SplitLayout L = split_layout(ss);
+    const char* ws = static_cast<const char*>(workspace);
+    return SplitGate{reinterpret_cast<const int*>(ws + L.verdict), reinterpret_cast<const double*>(ws + L.sums),
+                     ss.ntiles, strict ? 1 : 0};
+}
+
+size_t gram_workspace_size(int64_t rows, int kA, int kB, bool hermitian) {
+    const GramShape sh = gram_plan(rows, kA, kB, hermitian);
+    if (!gram_takes_split(rows, kA, kB, hermitian)) return gram_workspace_bytes(sh);
+    return split_gram_workspace_bytes(split_shape(rows, kA, kB, hermitian), sh);
+}
+
 // The row chunks of a Gram: chunk c covers rows [c chunk_rows, (c + 1)
 // chunk_rows). Each chunk's partial tiles depend on its rows alone, so the
 // partials of a chunk range can be computed as soon as those rows are in
 // place (a pipelined upload), with the same bits as one launch over all.
 void gram_chunks(int64_t rows, int kA, int kB, bool hermitian, int64_t* chunk_rows, int* nchunks) {
+    if (gram_takes_split(rows, kA, kB, hermitian)) {
+        const SplitShape ss = split_shape(rows, kA, kB, hermitian);
+        *chunk_rows = ss.chunk_rows;
+        *nchunks = ss.nchunks;
+        return;
+    }
     const GramShape sh = gram_plan(rows, kA, kB, hermitian);
     *chunk_rows = sh.chunk_rows;
     *nchunks = sh.nchunks;
 }
 
-// The partial tiles of chunks [chunk0, chunk1).
-int gram_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
-                          bool hermitian, void* workspace, size_t workspace_bytes, cudaStream_t stream,
-                          const ChainStatus* st, int gate, int chunk0, int chunk1) {
+// The FP64 partial tiles of chunks [chunk0, chunk1).
+static int dmma_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
+                                 bool hermitian, z64* partial, cudaStream_t stream, const ChainStatus* st, int gate,
+                                 int chunk0, int chunk1, const SplitGate& split) {
     GramShape sh = gram_plan(rows, kA, kB, hermitian);
-    size_t need = gram_workspace_bytes(sh);
-    if (workspace_bytes < need || workspace == nullptr) {
-        set_error(FB_ENOMEM, "gram: workspace of %zu bytes is smaller than the %zu bytes this shape needs",
-                  workspace_bytes, need);
-        return FB_ENOMEM;
-    }
     if (chunk0 < 0) chunk0 = 0;
     if (chunk1 > sh.nchunks) chunk1 = sh.nchunks;
     if (chunk0 >= chunk1) return FB_OK;
-    z64* partial = static_cast<z64*>(workspace);
     CUtensorMap ma, mb;
     FB_TRY(encode_panel_map(&ma, A, rows, kA, lda, sh.tw_a));
     FB_TRY(encode_panel_map(&mb, B, rows, kB, ldb, sh.tw_b));
@@ -558,29 +636,65 @@ int gram_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, 
         if (ln.ntiles == 0) continue;
         int status;
         switch (ln.ppw) {
-            case 2: status = launch_gram_dmma<2>(ma, mb, rows, sh, ln, partial, stream, st, gate, chunk0, chunk1); break;
-            case 3: status = launch_gram_dmma<3>(ma, mb, rows, sh, ln, partial, stream, st, gate, chunk0, chunk1); break;
-            case 4: status = launch_gram_dmma<4>(ma, mb, rows, sh, ln, partial, stream, st, gate, chunk0, chunk1); break;
-            default: status = launch_gram_dmma<8>(ma, mb, rows, sh, ln, partial, stream, st, gate, chunk0, chunk1); break;
+#define FB_GRAM_CASE(p) status = launch_gram_dmma<p>(ma, mb, rows, sh, ln, partial, stream, st, gate, chunk0, chunk1, split)
+            case 2: FB_GRAM_CASE(2); break;
+            case 3: FB_GRAM_CASE(3); break;
+            case 4: FB_GRAM_CASE(4); break;
+            default: FB_GRAM_CASE(8); break;
+#undef FB_GRAM_CASE
         }
         FB_TRY(status);
     }
     return FB_OK;
 }
 
-// C <- alpha (sum of the partial tiles of every chunk) + beta C.
-int gram_reduce_enqueue(z64* C, int64_t ldc, int64_t rows, int kA, int kB, bool hermitian, z64 alpha, z64 beta,
-                        void* workspace, cudaStream_t stream, const ChainStatus* st, int gate) {
+// The partial tiles of chunks [chunk0, chunk1).
+int gram_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
+                          bool hermitian, void* workspace, size_t workspace_bytes, cudaStream_t stream,
+                          const ChainStatus* st, int gate, int chunk0, int chunk1) {
+    const size_t need = gram_workspace_size(rows, kA, kB, hermitian);
+    if (workspace_bytes < need || workspace == nullptr) {
+        set_error(FB_ENOMEM, "gram: workspace of %zu bytes is smaller than the %zu bytes this shape needs",
+                  workspace_bytes, need);
+        return FB_ENOMEM;
+    }
+    if (gram_takes_split(rows, kA, kB, hermitian))
+        return split_partials_enqueue(A, lda, B, ldb, rows, kA, kB, split_shape(rows, kA, kB, hermitian), workspace,
+                                      stream, st, gate, chunk0, chunk1);
+    return dmma_partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, static_cast<z64*>(workspace), stream, st,
+                                 gate, chunk0, chunk1, SplitGate{});
+}
+
+static int reduce_enqueue(z64* C, int64_t ldc, const GramShape& sh, int kA, int kB, const z64* partial, z64 alpha,
+                          z64 beta, const SplitGate& split, cudaStream_t stream, const ChainStatus* st, int gate) {
+    const int64_t threads = (int64_t)kA * kB * 32;
+    const int block = 256;
+    const int64_t grid = (threads + block - 1) / block;
+    gram_reduce_kernel<<<(unsigned)grid, block, 0, stream>>>(C, ldc, kA, kB, sh, partial, alpha, beta, split, st, gate);
+    FB_LAUNCHED("gram_reduce_kernel");
+    return FB_OK;
+}
+
+// C <- alpha (sum of the partial tiles of every chunk) + beta C. Of a split
+// Gram: the sums and their verdict, the FP64 kernels over all rows (which
+// return at once when the verdict accepts the sums), and C from one or the
+// other.
+int gram_reduce_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
+                        int kB, bool hermitian, z64 alpha, z64 beta, void* workspace, cudaStream_t stream,
+                        const ChainStatus* st, int gate) {
     GramShape sh = gram_plan(rows, kA, kB, hermitian);
     if (hermitian && sh.nchunks > 0) sh.sdiag = gram_launch(sh, true).sdiag;
     z64* partial = static_cast<z64*>(workspace);
-    int64_t entries = (int64_t)kA * kB;
-    int64_t threads = entries * 32;
-    int block = 256;
-    int64_t grid = (threads + block - 1) / block;
-    gram_reduce_kernel<<<(unsigned)grid, block, 0, stream>>>(C, ldc, kA, kB, sh, partial, alpha, beta, st, gate);
-    FB_LAUNCHED("gram_reduce_kernel");
-    return FB_OK;
+    SplitGate split{};
+    if (gram_takes_split(rows, kA, kB, hermitian)) {
+        const SplitShape ss = split_shape(rows, kA, kB, hermitian);
+        split = split_gate(ss, workspace, false);
+        partial = reinterpret_cast<z64*>(static_cast<char*>(workspace) + split_layout(ss).partial);
+        FB_TRY(split_sum_enqueue(rows, ss, workspace, stream, st, gate));
+        FB_TRY(dmma_partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, partial, stream, st, gate, 0, sh.nchunks,
+                                     split));
+    }
+    return reduce_enqueue(C, ldc, sh, kA, kB, partial, alpha, beta, split, stream, st, gate);
 }
 
 // Shared by fb_zgram and the orthonormalization chain.
@@ -588,20 +702,41 @@ int gram_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z64* B, i
                  int64_t rows, int kA, int kB, z64 alpha, z64 beta, bool hermitian,
                  void* workspace, size_t workspace_bytes, cudaStream_t stream,
                  const ChainStatus* st, int gate) {
-    const GramShape sh = gram_plan(rows, kA, kB, hermitian);
-    const size_t need = gram_workspace_bytes(sh);
-    if (workspace_bytes < need || workspace == nullptr) {
-        set_error(FB_ENOMEM, "gram: workspace of %zu bytes is smaller than the %zu bytes this shape needs",
+    int64_t chunk_rows = 0;
+    int nchunks = 0;
+    gram_chunks(rows, kA, kB, hermitian, &chunk_rows, &nchunks);
+    FB_TRY(gram_partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, workspace, workspace_bytes, stream, st,
+                                 gate, 0, nchunks));
+    return gram_reduce_enqueue(C, ldc, A, lda, B, ldb, rows, kA, kB, hermitian, alpha, beta, workspace, stream, st,
+                               gate);
+}
+
+// The tensor-core entry points: the split form whatever the shape (k <= 64),
+// with no FP64 kernels behind it.
+size_t ozaki_gram_workspace_size(int64_t rows) { return split_layout(split_shape(rows, 64, 64, true)).total; }
+
+int ozaki_gram_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, int64_t rows, int k, z64 alpha, z64 beta,
+                       void* workspace, size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st,
+                       int gate) {
+    if (k < 1 || k > 64) {
+        set_error(FB_ENOTSUP, "the tensor-core Gram handles 1 <= k <= 64, got k = %d", k);
+        return FB_ENOTSUP;
+    }
+    if (rows > ((int64_t)1 << 30)) {
+        set_error(FB_ENOTSUP, "the tensor-core Gram handles at most 2^30 rows, got %lld", (long long)rows);
+        return FB_ENOTSUP;
+    }
+    const size_t need = ozaki_gram_workspace_size(rows);
+    if (!workspace || workspace_bytes < need) {
+        set_error(FB_ENOMEM, "tensor-core gram: workspace of %zu bytes is smaller than the %zu bytes needed",
                   workspace_bytes, need);
         return FB_ENOMEM;
     }
-    FB_TRY(gram_partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, workspace, workspace_bytes, stream, st,
-                                 gate, 0, sh.nchunks));
-    return gram_reduce_enqueue(C, ldc, rows, kA, kB, hermitian, alpha, beta, workspace, stream, st, gate);
-}
-
-size_t gram_workspace_size(int64_t rows, int kA, int kB, bool hermitian) {
-    return gram_workspace_bytes(gram_plan(rows, kA, kB, hermitian));
+    const SplitShape ss = split_shape(rows, k, k, true);
+    FB_TRY(split_partials_enqueue(A, lda, A, lda, rows, k, k, ss, workspace, stream, st, gate, 0, ss.nchunks));
+    FB_TRY(split_sum_enqueue(rows, ss, workspace, stream, st, gate));
+    return reduce_enqueue(C, ldc, gram_plan(rows, k, k, true), k, k, nullptr, alpha, beta,
+                          split_gate(ss, workspace, true), stream, st, gate);
 }
 
 // Scratch for fb_zgram_static, the entry point for callers that cannot
@@ -704,6 +839,24 @@ int fb_zgram_static(fb_z128* C, int64_t ldc, const fb_z128* A, int64_t lda, cons
     return gram_enqueue(reinterpret_cast<z64*>(C), ldc, reinterpret_cast<const z64*>(A), lda,
                         reinterpret_cast<const z64*>(B), ldb, rows, kA, kB, a, b, hermitian,
                         scratch, GRAM_STATIC_SCRATCH_BYTES, stream_of(queue), nullptr, GATE_ALWAYS);
+}
+
+int fb_zgram_tc_workspace_size(int64_t rows, int k, size_t* bytes) {
+    if (!bytes || rows < 0 || k < 0) { set_error(FB_EINVAL, "fb_zgram_tc_workspace_size: bad argument"); return FB_EINVAL; }
+    *bytes = ozaki_gram_workspace_size(rows);
+    return FB_OK;
+}
+
+int fb_zgram_tc(fb_z128* C, int64_t ldc, const fb_z128* A, int64_t lda, int64_t rows, int k, fb_z128 alpha,
+                fb_z128 beta, void* workspace, size_t workspace_bytes, fb_queue_t queue) {
+    if (rows < 0 || k < 0) { set_error(FB_EDIM, "fb_zgram_tc: negative size"); return FB_EDIM; }
+    if (k == 0) return FB_OK;
+    if (!C || (!A && rows > 0)) { set_error(FB_EINVAL, "fb_zgram_tc: NULL matrix"); return FB_EINVAL; }
+    if (ldc < k || (rows > 0 && lda < rows)) { set_error(FB_EDIM, "fb_zgram_tc: leading dimension too small"); return FB_EDIM; }
+    if ((uintptr_t)A & 15) { set_error(FB_EINVAL, "fb_zgram_tc: A must be 16-byte aligned"); return FB_EINVAL; }
+    return ozaki_gram_enqueue(reinterpret_cast<z64*>(C), ldc, reinterpret_cast<const z64*>(A), lda, rows, k,
+                              zmake(alpha.re, alpha.im), zmake(beta.re, beta.im), workspace, workspace_bytes,
+                              stream_of(queue), nullptr, GATE_ALWAYS);
 }
 
 int fb_tune_set_gram_chunks(int64_t rows, int k, int shift) {

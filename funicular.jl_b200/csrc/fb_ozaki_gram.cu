@@ -1,84 +1,95 @@
-// The Gram matrix G = Y^H Y (gram_accumulate!, src/kernels.jl:22-55, with
-// A === B) on the integer tensor cores: an Ozaki-style split of every FP64
-// entry into 8-bit slices whose products are exact in 32-bit integer
-// accumulators, recovered to FP64 with power-of-two weights.
+// Products A^H B of tall skinny ComplexF64 matrices on the integer tensor
+// cores: an Ozaki-style split of every FP64 entry into 8-bit slices whose
+// products are exact in 32-bit integer accumulators, recovered to FP64 with
+// power-of-two weights. fb_gram.cu takes this form of gram_accumulate!
+// (src/kernels.jl:22-55) where it is the faster one and checks afterwards, on
+// the device, that it was also accurate enough (split_sum_kernel).
 //
-// Real form. With W the 2N x k real matrix holding Re Y and Im Y in
-// alternating rows (exactly the interleaved ComplexF64 layout of a column) and
-// JW the same with each (re, im) pair turned into (im, -re):
-//   [W JW]^T W = [Re G ; -Im G]      (a 128 x 64 product for k <= 64).
-// The MMA operand A holds the slices of W and JW, 128 rows, in tensor memory;
-// operand B holds the W slices stacked along N in shared memory, so one MMA
-// of A slice t against B slices 1..7-t lands in the accumulators of the groups
-// g = t + u it feeds. Keeping A in tensor memory halves the shared-memory
-// traffic of the products, which bounds this kernel.
+// Output tiles are 64 x 64 columns; a CTA owns one tile and one chunk of rows.
+//   Folded tile (A === B, on the diagonal). With G = A^H A the real 64 x 64
+//   matrix S = Re G + Im G = V^T W holds all of G (Re and Im are its
+//   symmetric and antisymmetric parts): W is the interleaved (re, im) rows of
+//   A, V the rows (re - im, re + im).
+//   Full tile: [W JW]^T W' = [Re; Im] of A^H B, with JW the rows (-im, re) of
+//   A and W' the interleaved rows of B.
 //
-// Slices. Column j carries a power-of-two scale 2^E_j with |entries| <
-// 2^(E_j - 1); an entry x becomes the integer x_int = rint(x 2^(51 - E_j)),
-// |x_int| <= 2^50, written as seven signed bytes on a grid of 8-bit steps
+// Slices. Column j carries a power-of-two scale 2^E with |entries| <
+// 2^E (1 - 2^-7); an entry x becomes the integer x_int = rint(x 2^(51 - E)),
+// written as seven signed bytes on a grid of 8-bit steps,
 //   x_int = sum_{t=1..7} d_t 2^(52 - 8 t),   d_t in [-128, 127],
-// the last one a multiple of 16 (it carries the lowest 4 bits). One FMA makes
-// them: m = fma(x, 2^(51 - E_j), 2^52 + 2^51 + B) is exact, its 52 mantissa
-// bits are x_int + B + 2^51 with B = 0x80808080808 biasing every digit by
-// half its range, and the bytes of m << 4 are the digits, each plus 128: the
-// slices are read straight out of the double's bit pattern, and its exponent
-// field tells whether x was in range. A product of two entries is
-// 2^(E_a + E_b - 102) sum_{t,u} d_t e_u 2^(104 - 8 (t + u)); the 28 terms
-// with t + u <= 8 are kept, the rest lie below 2^-50 of the leading term. Group g = t + u owns 64 accumulator columns of tensor memory (448 in
-// all), the A slices the next 56.
+// the last a multiple of 16. One FMA makes them: m = fma(x, 2^(51 - E),
+// 2^52 + 2^51 + B) is exact, its 52 mantissa bits are x_int + B + 2^51 with
+// B = 0x80808080808 biasing every digit by half its range, and the bytes of
+// m << 4 are the digits, each plus 128: the slices are read out of the
+// double's bit pattern. V is twice as large and is scaled by half as much.
+// A product of two entries is 2^(E_a + E_b - 102) sum d_t e_u 2^(104 - 8(t+u));
+// the 28 terms with t + u <= 8 are kept (a folded tile also gets three of the
+// six with t + u = 9), the rest lie below 2^-50 of the leading term.
+//
+// MMAs (kind::i8, M = 128, K = 32 bytes = 16 complex rows, one stage).
+//   Full tile: operand A is slice t of W (rows 0-63) and of JW (rows 64-127),
+//   operand B the slices 1..8-t of W' stacked along N; the product lands in
+//   the accumulator blocks of the groups t + u = 2..8 (seven blocks of 64
+//   columns of tensor memory): 1792 columns of N a stage.
+//   Folded tile: S needs 64 rows only, so two slices of V share one operand,
+//   t = 2p + 1 in rows 0-63 and t = 2p + 2 in rows 64-127, against slices
+//   1..7-2p of W; block c then holds group c + 2 in rows 0-63 and c + 3 in
+//   rows 64-127: 1024 columns of N a stage, 0.57 of the full tile's.
 //
 // Scales adapt as the rows stream: a stage with an entry its column's scale
-// cannot hold, or one that would let an int32 accumulator overflow (every
-// 8192 rows), first drains the accumulators into this CTA's FP64 partial in
-// global memory, then rescales with HEADROOM spare bits. The partials of all
-// CTAs are summed in a fixed order by the reduce kernel, so results are
-// deterministic.
+// cannot hold, or one that would let an int32 accumulator overflow, starts a
+// new epoch: the accumulators are first drained into this CTA's FP64 partial
+// tile, then the column's scale grows with HEADROOM spare bits.
 //
-// Rows of A (tensor memory lanes): lane 32q + l holds W column 16q + l for
-// l < 16 and JW column 16q + l - 16 for l >= 16, so one warp writes both rows
-// of a column and its two halves read the same FP64 values (a broadcast).
-//
-// Roles (one CTA per SM, 576 threads): warps 0-15 slice (warp w writes lane
-// quarter w % 4, K bytes 8 (w / 4)..+7 of every A slice) and drain (lane
-// quarter w % 4, accumulator columns 16 (w / 4)..+15 of every group); warp 16
-// issues the MMAs; warp 17 keeps a ring of TMA tile loads in flight. Every
-// wait is bounded.
+// What bounds it and how the work is laid out: a stage of 16 rows costs 512
+// cycles of integer MMA for a folded tile, about as many of 32-bit integer
+// work to cut and transpose the slices, and 709 cycles of HBM time. So nothing
+// may serialize: the decision about scales is made by scanner warps a few
+// stages ahead of the slicers (so slicers never vote), and the slicers form
+// GROUPS groups of four warps that take the stages in turn, each with a slice
+// buffer of its own, so one group's load, cut and store chain overlaps the
+// others' and the MMAs. Every wait is bounded; a failed one stops the CTA and
+// marks its result invalid.
+#include "fb_gram_split.cuh"
 #include "fb_umma.cuh"
 
 namespace fb {
-namespace ozaki {
+namespace split {
 
 constexpr int SLICES = 7;
-constexpr int ROWS = 16;                        // complex rows per stage: K = 32 bytes
-constexpr int FSTAGES = 6;                      // FP64 ring depth
+constexpr int ROWS = SPLIT_STAGE_ROWS;          // complex rows per stage: K = 32 bytes
 constexpr int FBYTES = ROWS * 64 * 16;          // 16 KB: 16 rows x 64 columns
 constexpr int BTILE = SLICES * 64 * 32;         // B: 7 x 64 rows x 32 bytes
-constexpr int SBUFS = 2;
-constexpr int TMEM_COLS = 512;
-constexpr int A_COL = 448;                      // A slice t at tensor memory column A_COL + 8 t
-constexpr int EPOCH_STAGES = 8192 / ROWS;       // int32 headroom: 7 x 2^14 x 2 x 8192 < 2^31
+constexpr int ATILE = 128 * 32;                 // one A operand
+constexpr int TMEM_COLS = 512;                  // 448 used; the allocation is a power of two
 constexpr int HEADROOM = 2;                     // spare exponent bits above the maximum that set a scale
-constexpr int E_UNSET = -4000;                  // column seen only zeros so far
-constexpr int SLICERS = 512;                    // sixteen warps
-constexpr int THREADS = SLICERS + 64;
-// 2^52 + 2^51 + 0x80808080808: the FMA addend that leaves x_int + B + 2^51
-// in the mantissa of a double whose high word starts with 0x433.
-constexpr long long MAGIC_BITS = 0x4338080808080808ll;
+constexpr long long MAGIC_BITS = 0x4338080808080808ll;  // 2^52 + 2^51 + 0x80808080808
 
-constexpr size_t OFF_F = 0;
-constexpr size_t OFF_B = OFF_F + (size_t)FSTAGES * FBYTES;
-constexpr size_t OFF_MAX = OFF_B + (size_t)SBUFS * BTILE;   // uint32 [4][64] column maxima
-constexpr size_t OFF_BAR = OFF_MAX + 4 * 64 * 4;            // mbarriers
-constexpr size_t OFF_MISC = OFF_BAR + 32 * 8;
-constexpr size_t MISC_BYTES = 512;                          // flags, TMEM slot, column exponents
-constexpr size_t SMEM_BYTES = OFF_MISC + MISC_BYTES + 1024;  // + alignment slack
-
-struct Flags {
-    int timeout;
-    int nonfinite;
-    int drains;      // epochs drained, all CTAs together (a statistic)
-    int rescales;    // of them, drains forced by a column outgrowing its scale
+template <bool FULL>
+struct Cfg {
+    static constexpr int SIDES = FULL ? 2 : 1;                 // input tiles per stage
+    static constexpr int GROUPS = FULL ? 3 : 4;                // slicer groups of 128 threads = slice buffers
+    static constexpr int SLOTS = FULL ? 3 : 6;                 // FP64 ring depth
+    static constexpr int NA = FULL ? SLICES : 4;               // A operands per stage
+    static constexpr int SCANNERS = 64 * SIDES;                // scanner threads, one per input column
+    static constexpr int SLICERS = 128 * GROUPS;
+    static constexpr int THREADS = SLICERS + 64 + SCANNERS;
+    static constexpr int BUF = NA * ATILE + BTILE;             // one slice buffer: A operands, then B
+    // int32 headroom: products are at most 2^14, a block gets 7 (full) or 4
+    // (folded) of them per K row and 2 K rows per complex row.
+    static constexpr int EPOCH_STAGES = (FULL ? 8192 : 12288) / ROWS;
+    struct Slot {                                              // what the scanners say about a stage
+        int E[64 * SIDES], Eold[64 * SIDES];
+        int fresh, epoch;
+    };
+    static constexpr size_t OFF_F = 0;
+    static constexpr size_t OFF_S = OFF_F + (size_t)SLOTS * SIDES * FBYTES;
+    static constexpr size_t OFF_SLOT = OFF_S + (size_t)GROUPS * BUF;
+    static constexpr size_t OFF_BAR = (OFF_SLOT + SLOTS * sizeof(Slot) + 15) / 16 * 16;
+    static constexpr size_t OFF_MISC = OFF_BAR + (3 * SLOTS + 2 * GROUPS) * 8;
+    static constexpr size_t SMEM = OFF_MISC + 64 + 1024;       // + alignment slack
 };
+static_assert(Cfg<false>::SMEM <= 227 * 1024 && Cfg<true>::SMEM <= 227 * 1024, "a CTA's shared memory");
 
 __device__ __forceinline__ uint32_t sw32_offset(uint32_t row, uint32_t chunk) {
     return row * 32 + ((chunk ^ ((row >> 2) & 1)) << 4);
@@ -124,423 +135,518 @@ __device__ __forceinline__ void slice_words(const uint64_t (&y)[4], uint32_t (&w
     w[6] = __byte_perm(a01, a23, 0x5410) ^ 0x80808080u;  // byte 0
 }
 
-// Adds the accumulators of the epoch that ended with last_stage into P: row
-// prow, columns 16c..16c+15 of the 128 x 64 partial, read from tensor memory
-// at tcol (this thread's lane, column 16c of group 0). False if the MMAs
-// never finished. Kept out of line: it runs a few times per CTA and would
-// otherwise hold registers across the slicing loop.
-__device__ __noinline__ bool drain_epoch(uint64_t* sl_empty, int last_stage, uint32_t tcol, const int* Es, int prow,
-                                         int c, double* P, bool initialized) {
-    // Every MMA up to last_stage has finished once its commit arrived.
-    if (!mbar_wait(&sl_empty[last_stage % SBUFS], (last_stage / SBUFS) & 1)) return false;
-    umma::fence_after_sync();
-    const int Em = Es[prow & 63];
-    double acc[16];
+// What an operand's K rows are made of, from a complex entry (re, im).
+enum Form { FORM_W, FORM_JW, FORM_V };
+
+// Cuts eight complex rows of one column (v: re, im alternating) into the 16
+// K bytes of every slice and stores slice t at base(t).
+template <Form F, class Base>
+__device__ __forceinline__ void cut(const double (&v)[16], double sc, Base base) {
+    const double magic = __longlong_as_double(MAGIC_BITS);
+    uint32_t w[4][SLICES];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.0;
-#pragma unroll 1
-    for (int g = 0; g < SLICES; ++g) {
-        uint32_t r[16];
-        umma::tmem_ld16(tcol + 64 * g, r);
-        umma::tmem_wait_ld();
-        const double w = pow2(-8 * (g + 2));
+    for (int q = 0; q < 4; ++q) {
+        uint64_t y[4];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[i] = fma((double)(int)r[i], w, acc[i]);
+        for (int r = 0; r < 2; ++r) {
+            const double re = v[4 * q + 2 * r], im = v[4 * q + 2 * r + 1];
+            double a = re, b = im;
+            if (F == FORM_JW) { a = -im; b = re; }
+            if (F == FORM_V) { a = re - im; b = re + im; }
+            y[2 * r] = (uint64_t)__double_as_longlong(fma(a, sc, magic)) << 4;
+            y[2 * r + 1] = (uint64_t)__double_as_longlong(fma(b, sc, magic)) << 4;
+        }
+        slice_words(y, w[q]);
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int n = 16 * c + i;
-        const int En = Es[n];
-        double v = 0.0;
-        if (Em != E_UNSET && En != E_UNSET) v = acc[i] * pow2(Em + En + 2);
-        double* dst = P + (size_t)n * 128 + prow;
-        *dst = initialized ? *dst + v : v;
-    }
-    umma::fence_before_sync();
-    return true;
+    for (int t = 0; t < SLICES; ++t)
+        *reinterpret_cast<uint4*>(base(t)) = make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]);
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
-ozaki_gram_kernel(const __grid_constant__ CUtensorMap tm, int64_t rows, int64_t chunk_rows,
-                  double* __restrict__ partial, Flags* __restrict__ flags, const ChainStatus* st, int gate) {
+// Adds the accumulators into the partial tile P (128 x 64 doubles, column n
+// contiguous): this thread's row `prow`, all 64 columns. EA and EB are the
+// scale exponents of the operands' columns in the epoch that ends. Kept out
+// of line: it runs a few times per CTA and would otherwise hold registers
+// across the slicing loop.
+template <bool FULL>
+__device__ __noinline__ void drain_epoch(uint32_t tmem_lane, const int* EA, const int* EB, int prow, double* P,
+                                         bool initialized) {
+    const int Em = EA[prow & 63];
+    // Weight of block c: 2^(E_a + E_b + 2 - 8 g), V's halved scale one more.
+    const int shift = FULL ? 2 : (prow < 64 ? 3 : 3 - 8);
+    for (int cc = 0; cc < 4; ++cc) {
+        double acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.0;
+#pragma unroll 1
+        for (int c = 0; c < SLICES; ++c) {
+            uint32_t r[16];
+            umma::tmem_ld16(tmem_lane + 64 * c + 16 * cc, r);
+            umma::tmem_wait_ld();
+            const double w = pow2(-8 * (c + 2));
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[i] = fma((double)(int)r[i], w, acc[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int n = 16 * cc + i;
+            const int En = EB[n];
+            double v = 0.0;
+            if (Em != SPLIT_E_UNSET && En != SPLIT_E_UNSET) v = acc[i] * pow2(Em + En + shift);
+            double* dst = P + (size_t)n * 128 + prow;
+            *dst = initialized ? *dst + v : v;
+        }
+    }
+    __threadfence_block();
+}
+
+template <bool FULL>
+__global__ void __launch_bounds__(Cfg<FULL>::THREADS, 1)
+split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int64_t rows,
+                  SplitShape sh, double* __restrict__ partial, SplitStat* __restrict__ stats, const ChainStatus* st,
+                  int gate, int chunk0) {
     if (gated_off(st, gate)) return;
+    using C = Cfg<FULL>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint64_t* fp_full = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-    uint64_t* fp_empty = fp_full + FSTAGES;
-    uint64_t* sl_full = fp_empty + FSTAGES;
-    uint64_t* sl_empty = sl_full + SBUFS;
-    int* misc = reinterpret_cast<int*>(smem + OFF_MISC);
-    volatile int* fresh_flag = misc;           // [SBUFS]
-    volatile int* abort_flag = misc + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 4);
-    int* Es = misc + 8;                        // [64] scale exponents for the drain
-    uint32_t* colmax = reinterpret_cast<uint32_t*>(smem + OFF_MAX);
+    typename C::Slot* slots = reinterpret_cast<typename C::Slot*>(smem + C::OFF_SLOT);
+    uint64_t* fp_full = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);   // a stage's rows have landed
+    uint64_t* fp_empty = fp_full + C::SLOTS;                              // scanned and loaded by its slicers
+    uint64_t* sc_full = fp_empty + C::SLOTS;                              // scanned
+    uint64_t* sl_full = sc_full + C::SLOTS;                               // a group's slices are written
+    uint64_t* sl_empty = sl_full + C::GROUPS;                             // and consumed by the MMAs
+    int* misc = reinterpret_cast<int*>(smem + C::OFF_MISC);
+    volatile int* abort_flag = misc;
+    int* bad_flag = misc + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 2);
+    volatile int* fresh_flag = misc + 4;   // [GROUPS]
 
+    int ti, tj, tile;
+    split_tile_of(sh, FULL, (int)blockIdx.x, ti, tj, tile);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t row0 = (int64_t)blockIdx.x * chunk_rows;
-    const int64_t row_end = min(rows, row0 + chunk_rows);
+    const int chunk = chunk0 + (int)blockIdx.y;
+    const int64_t row0 = (int64_t)chunk * sh.chunk_rows;
+    const int64_t row_end = min(rows, row0 + sh.chunk_rows);
     const int nstages = (int)((row_end - row0 + ROWS - 1) / ROWS);
-    double* P = partial + (size_t)blockIdx.x * (128 * 64);
+    double* P = partial + ((size_t)tile * sh.nchunks + chunk) * SPLIT_TILE_DOUBLES;
+    SplitStat* stat = stats + (size_t)tile * sh.nchunks + chunk;
 
     if (threadIdx.x == 0) {
-        for (int b = 0; b < FSTAGES; ++b) {
+        for (int b = 0; b < C::SLOTS; ++b) {
             mbar_init(&fp_full[b], 1);
-            mbar_init(&fp_empty[b], SLICERS);
+            mbar_init(&fp_empty[b], 4 + C::SCANNERS / 32);
+            mbar_init(&sc_full[b], C::SCANNERS);
         }
-        for (int b = 0; b < SBUFS; ++b) {
-            mbar_init(&sl_full[b], SLICERS);
+        for (int b = 0; b < C::GROUPS; ++b) {
+            mbar_init(&sl_full[b], 4);
             mbar_init(&sl_empty[b], 1);
         }
         *abort_flag = 0;
-        for (int c = 0; c < 64; ++c) Es[c] = E_UNSET;
+        *bad_flag = 0;
         mbar_fence_init();
     }
+    if constexpr (!FULL) {
+        // The last A operand of a folded tile has one slice only: its rows
+        // 64-127 are zero for good.
+        for (int e = threadIdx.x; e < C::GROUPS * (ATILE / 2) / 16; e += blockDim.x) {
+            const int b = e / ((ATILE / 2) / 16), o = e - b * ((ATILE / 2) / 16);
+            reinterpret_cast<uint4*>(smem + C::OFF_S + (size_t)b * C::BUF + 3 * ATILE + ATILE / 2)[o] =
+                make_uint4(0, 0, 0, 0);
+        }
+    }
     if (warp == 0) umma::tmem_alloc(tmem_slot, TMEM_COLS);
+    umma::fence_smem_to_async();
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t taddr = *tmem_slot;
 
-    if (warp == SLICERS / 32 + 1) {
-        // ---- producer: FP64 tiles, two 8-row boxes per stage ----
+    if (warp == C::SLICERS / 32 + 1) {
+        // ---- producer: FP64 tiles, two 8-row boxes per stage and input ----
         if (lane == 0) {
-            tma_prefetch_map(&tm);
-            int issued = 0;
+            tma_prefetch_map(&tmA);
+            if (FULL) tma_prefetch_map(&tmB);
+            int issued = 0, b = 0;
+            uint32_t ph = 0;
             for (int s = 0; s < nstages; ++s) {
-                const int b = s % FSTAGES;
-                if (s >= FSTAGES && !mbar_wait(&fp_empty[b], ((s / FSTAGES) - 1) & 1)) {
-                    atomicExch(&flags->timeout, 1);
+                if (s >= C::SLOTS && !mbar_wait(&fp_empty[b], ph ^ 1u)) {
                     *abort_flag = 1;
                     break;
                 }
                 if (*abort_flag) break;
-                mbar_arrive_expect_tx(&fp_full[b], FBYTES);
+                mbar_arrive_expect_tx(&fp_full[b], C::SIDES * FBYTES);
                 const int x = (int)(2 * (row0 + (int64_t)s * ROWS));
-                unsigned char* dst = smem + OFF_F + (size_t)b * FBYTES;
-                tma_load_2d(dst, &tm, x, 0, &fp_full[b]);
-                tma_load_2d(dst + FBYTES / 2, &tm, x + 16, 0, &fp_full[b]);
+                unsigned char* dst = smem + C::OFF_F + (size_t)b * C::SIDES * FBYTES;
+                tma_load_2d(dst, &tmA, x, 64 * ti, &fp_full[b]);
+                tma_load_2d(dst + FBYTES / 2, &tmA, x + 16, 64 * ti, &fp_full[b]);
+                if (FULL) {
+                    tma_load_2d(dst + FBYTES, &tmB, x, 64 * tj, &fp_full[b]);
+                    tma_load_2d(dst + FBYTES + FBYTES / 2, &tmB, x + 16, 64 * tj, &fp_full[b]);
+                }
                 issued = s + 1;
+                if (++b == C::SLOTS) { b = 0; ph ^= 1u; }
             }
             // After an abort, let the copies still in flight land before the
             // shared memory they write goes away.
-            for (int s = issued > FSTAGES ? issued - FSTAGES : 0; *abort_flag && s < issued; ++s)
-                mbar_wait(&fp_full[s % FSTAGES], (s / FSTAGES) & 1);
+            for (int s = issued > C::SLOTS ? issued - C::SLOTS : 0; *abort_flag && s < issued; ++s)
+                mbar_wait(&fp_full[s % C::SLOTS], (s / C::SLOTS) & 1);
         }
-    } else if (warp == SLICERS / 32) {
+    } else if (warp == C::SLICERS / 32) {
         // ---- MMA issuer ----
         if (lane == 0) {
-            int issued = 0;
+            int issued = 0, g = 0;
+            uint32_t ph = 0;
             for (int s = 0; s < nstages; ++s) {
-                const int b = s % SBUFS;
-                if (!mbar_wait(&sl_full[b], (s / SBUFS) & 1) || *abort_flag) {
-                    atomicExch(&flags->timeout, 1);
+                if (!mbar_wait(&sl_full[g], ph) || *abort_flag) {
                     *abort_flag = 1;
                     break;
                 }
                 umma::fence_after_sync();
-                const bool fresh = fresh_flag[b] != 0;
-                const uint32_t bbase = smem_u32(smem + OFF_B + (size_t)b * BTILE);
+                const bool fresh = fresh_flag[g] != 0;
+                const uint32_t abase = smem_u32(smem + C::OFF_S + (size_t)g * C::BUF);
+                const uint32_t bbase = abase + C::NA * ATILE;
 #pragma unroll
-                for (int t = 0; t < SLICES; ++t) {
-                    const int ntot = 64 * (SLICES - t);
+                for (int a = 0; a < C::NA; ++a) {
+                    const int first = FULL ? a : 2 * a;      // accumulator block of slice 1 of B
+                    const int ntot = 64 * (SLICES - first);
 #pragma unroll
                     for (int off = 0; off < ntot; off += 256) {
                         const int n = ntot - off < 256 ? ntot - off : 256;
-                        umma::mma_s8_tmem_a(taddr + 64 * t + off, taddr + A_COL + 8 * t, desc_sw32(bbase + off * 32),
-                                            umma::idesc_s8s8_s32(128, n), !(fresh && t == 0));
+                        umma::mma_s8(taddr + 64 * first + off, desc_sw32(abase + a * ATILE),
+                                     desc_sw32(bbase + off * 32), umma::idesc_s8s8_s32(128, n), !(fresh && a == 0));
                     }
                 }
-                umma::commit(&sl_empty[b]);
+                umma::commit(&sl_empty[g]);
                 issued = s + 1;
+                if (++g == C::GROUPS) { g = 0; ph ^= 1u; }
             }
             // After an abort, wait for the MMAs in flight before tensor memory
             // is released.
-            if (*abort_flag && issued > 0) mbar_wait(&sl_empty[(issued - 1) % SBUFS], ((issued - 1) / SBUFS) & 1);
+            if (*abort_flag && issued > 0)
+                mbar_wait(&sl_empty[(issued - 1) % C::GROUPS], ((issued - 1) / C::GROUPS) & 1);
+        }
+    } else if (warp < C::SLICERS / 32) {
+        // ---- slicers ----
+        const int g = warp >> 2, q = warp & 3;
+        const int t128 = threadIdx.x & 127;
+        const int j = t128 & 63, kq = t128 >> 6;             // this thread's column and 8-row box
+        const int prow = 32 * q + lane;                      // its row of the accumulators
+        const uint32_t tmem_lane = taddr + ((uint32_t)(32 * q) << 16);
+        unsigned char* abuf = smem + C::OFF_S + (size_t)g * C::BUF;
+        unsigned char* bbuf = abuf + C::NA * ATILE;
+        const uint32_t off_lo = sw32_offset(j, kq), off_hi = sw32_offset(64 + j, kq);
+        // Waits are decided by the whole warp together, so that a warp leaves
+        // the loop as one.
+        auto wait = [&](uint64_t* bar, uint32_t parity) {
+            return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
+        };
+        auto load = [&](const unsigned char* tile_base, double (&v)[16]) {
+            const unsigned char* col = tile_base + (size_t)kq * (FBYTES / 2) + j * 128;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const double2 z = *reinterpret_cast<const double2*>(col + ((r ^ (j & 7)) << 4));
+                v[2 * r] = z.x;
+                v[2 * r + 1] = z.y;
+            }
+        };
+        // Drains the accumulators once the MMAs of `stage` have finished.
+        auto drain = [&](int stage, const int* EA, const int* EB, bool initialized) {
+            if (!wait(&sl_empty[stage % C::GROUPS], (stage / C::GROUPS) & 1)) return false;
+            umma::fence_after_sync();
+            drain_epoch<FULL>(tmem_lane, EA, EB, prow, P, initialized);
+            umma::fence_before_sync();
+            return true;
+        };
+        bool ok = true;
+        uint32_t gph = 1;                                     // parity of this group's previous commit
+        int s = g;
+        for (; s < nstages; s += C::GROUPS) {
+            const int b = s % C::SLOTS;
+            const uint32_t ph = (s / C::SLOTS) & 1;
+            if (!wait(&sc_full[b], ph) || !wait(&fp_full[b], ph) || *abort_flag) { ok = false; break; }
+            const typename C::Slot& slot = slots[b];
+            const bool fresh = slot.fresh != 0;
+            // This group's buffer is free once its previous stage's MMAs are
+            // done (waited for before a drain, too: it leaves the barrier of
+            // stage s - 1 at most one phase behind).
+            if (s >= C::GROUPS && !wait(&sl_empty[g], gph)) { ok = false; break; }
+            // A new epoch: the MMAs of the one before it all precede this
+            // stage's, which wait for this group.
+            if (fresh && s > 0 &&
+                !drain(s - 1, slot.Eold, slot.Eold + (FULL ? 64 : 0), slot.epoch > 1)) { ok = false; break; }
+            const unsigned char* f = smem + C::OFF_F + (size_t)b * C::SIDES * FBYTES;
+            const int EA = slot.E[j], EB = slot.E[(FULL ? 64 : 0) + j];
+            const double sca = EA == SPLIT_E_UNSET ? 0.0 : pow2((FULL ? 51 : 50) - EA);
+            const double scb = EB == SPLIT_E_UNSET ? 0.0 : pow2(51 - EB);
+            auto release = [&]() {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&fp_empty[b]);
+            };
+            double v[16];
+            if constexpr (FULL) {
+                load(f + FBYTES, v);
+                cut<FORM_W>(v, scb, [&](int t) { return bbuf + off_lo + t * (64 * 32); });
+                load(f, v);
+                release();
+                cut<FORM_W>(v, sca, [&](int t) { return abuf + t * ATILE + off_lo; });
+                cut<FORM_JW>(v, sca, [&](int t) { return abuf + t * ATILE + off_hi; });
+            } else {
+                load(f, v);
+                release();
+                cut<FORM_W>(v, scb, [&](int t) { return bbuf + off_lo + t * (64 * 32); });
+                cut<FORM_V>(v, sca, [&](int t) { return abuf + (t >> 1) * ATILE + ((t & 1) ? off_hi : off_lo); });
+            }
+            if (t128 == 0) fresh_flag[g] = fresh ? 1 : 0;
+            umma::fence_smem_to_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sl_full[g]);
+            gph ^= 1u;
+        }
+        if (!ok) *abort_flag = 1;
+        // The group of the last stage drains the last epoch.
+        if (ok && nstages > 0 && s - C::GROUPS == nstages - 1) {
+            const typename C::Slot& slot = slots[(nstages - 1) % C::SLOTS];
+            if (!drain(nstages - 1, slot.E, slot.E + (FULL ? 64 : 0), slot.epoch > 0)) *abort_flag = 1;
         }
     } else {
-        // ---- slicers and drains: warps 0..15 ----
-        const int tid = threadIdx.x;
-        const int q = warp & 3, kq = warp >> 2;
-        const bool jw = lane >= 16;
-        const int j = 16 * q + (lane & 15);                  // this thread's column
-        const int prow = (jw ? 64 : 0) + j;                  // its row of the 128 x 64 partial
-        const uint32_t lane_base = (uint32_t)(32 * q) << 16;
-        int E = E_UNSET;            // scale exponent of column j
-        int epoch_start = 0;
-        bool initialized = false;   // P written at least once
-        bool bad = false;
-
-        // A CTA-uniform OR over the slicer threads; also a barrier.
+        // ---- scanners: scales, a few stages ahead of the slicers ----
+        const int c = (int)threadIdx.x - C::SLICERS - 64;    // input column: A's 0-63, then B's
         auto any = [](bool p) -> bool {
-            uint32_t qq;
+            uint32_t r;
             asm volatile(
                 "{\n\t.reg .pred a, b;\n\t"
                 "setp.ne.u32 a, %1, 0;\n\t"
                 "barrier.cta.red.or.pred b, 1, %2, a;\n\t"
                 "selp.u32 %0, 1, 0, b;\n\t}"
-                : "=r"(qq)
-                : "r"((uint32_t)p), "n"(SLICERS)
+                : "=r"(r)
+                : "r"((uint32_t)p), "n"(C::SCANNERS)
                 : "memory");
-            return qq != 0;
+            return r != 0;
         };
-        auto fail = [&]() {
-            atomicExch(&flags->timeout, 1);
-            *abort_flag = 1;
-        };
-        auto drain = [&](int last_stage) -> bool {
-            const bool ok = drain_epoch(sl_empty, last_stage, taddr + lane_base + 16 * kq, Es, prow, kq, P, initialized);
-            initialized = true;
-            return ok;
-        };
-        // Complex rows 4 (kq & 1) .. + 3 of column j in box kq / 2 of stage st.
-        auto load = [&](int st, double (&vv)[8]) -> bool {
-            const int fb = st % FSTAGES;
-            if (!mbar_wait(&fp_full[fb], (st / FSTAGES) & 1)) return false;
-            const unsigned char* box = smem + OFF_F + (size_t)fb * FBYTES + (size_t)(kq >> 1) * (FBYTES / 2) + j * 128;
+        int E = SPLIT_E_UNSET;
+        // |x| < 2^E (1 - 2^-7) in terms of the high word of x; while the
+        // scale is unset every normal number is past it.
+        uint32_t limit = 0x00100000u;
+        uint32_t tiny = 0;                                   // bits of subnormal entries under an unset scale
+        bool bad = false;
+        double sq[4] = {0.0, 0.0, 0.0, 0.0};
+        int b = 0, epoch = -1, epoch_start = 0;
+        uint32_t ph = 0;
+        for (int s = 0; s < nstages; ++s) {
+            const bool landed = mbar_wait(&fp_full[b], ph);
+            const bool stop = !landed || *abort_flag;
+            const unsigned char* col =
+                smem + C::OFF_F + ((size_t)b * C::SIDES + (c >> 6)) * FBYTES + (c & 63) * 128;
+            uint32_t mx = 0, low = 0;
+            if (!stop) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int rr = 4 * (kq & 1) + r;
-                const double2 z = *reinterpret_cast<const double2*>(box + ((rr ^ (j & 7)) << 4));
-                vv[2 * r] = z.x;
-                vv[2 * r + 1] = z.y;
-            }
-            mbar_arrive(&fp_empty[fb]);
-            return true;
-        };
-
-        // Every decision that can end the loop is taken by all slicer threads
-        // together (any), so none of them is ever left waiting at a barrier:
-        // one barrier per stage in the common case. A failed wait elsewhere
-        // is recorded and stops the loop at the next stage's barrier.
-        const double magic = __longlong_as_double(MAGIC_BITS);
-        bool timed_out = false;
-        int s = 0;
-        for (; s < nstages; ++s) {
-            const int sb = s % SBUFS;
-            double v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = 0.0;
-            const bool landed = load(s, v);
-            // Scale and split: W rows take re0 im0 re1 im1 .., JW rows
-            // im0 -re0 im1 -re1 .., four K values to a word. A result whose
-            // high word does not start 0x433 was out of range.
-            double sc = (E == E_UNSET || bad) ? 0.0 : pow2(51 - E);
-            uint64_t t[8];
-            uint32_t range = 0;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const double first = jw ? v[2 * c + 1] : v[2 * c];
-                const double second = jw ? v[2 * c] : v[2 * c + 1];
-                t[2 * c] = (uint64_t)__double_as_longlong(fma(first, sc, magic));
-                t[2 * c + 1] = (uint64_t)__double_as_longlong(fma(second, jw ? -sc : sc, magic));
-                range |= ((uint32_t)(t[2 * c] >> 32) ^ 0x43300000u) | ((uint32_t)(t[2 * c + 1] >> 32) ^ 0x43300000u);
-            }
-            bool out_of_range = (range & 0xFFF00000u) != 0;
-            if (E == E_UNSET) {
-                uint32_t nz = 0;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) nz |= (uint32_t)(__double_as_longlong(v[i]) >> 32) & 0x7FF00000u;
-                out_of_range = nz != 0;
-            }
-            const bool epoch_full = s - epoch_start >= EPOCH_STAGES;
-            const bool stop = !landed || timed_out || *abort_flag;
-            bool fresh = s == 0;
-            if (any(stop || out_of_range || epoch_full)) {
-                if (any(stop)) { fail(); break; }
-                // The column maxima: the high word of |x| orders magnitudes
-                // by exponent, and Inf and NaN above every finite value.
-                uint32_t mx = 0;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) mx = max(mx, (uint32_t)(__double_as_longlong(v[i]) >> 32) & 0x7FFFFFFFu);
-                if (!jw) colmax[kq * 64 + j] = mx;
-                asm volatile("bar.sync 1, %0;" ::"n"(SLICERS) : "memory");
-                const uint32_t cm = max(max(colmax[j], colmax[64 + j]), max(colmax[128 + j], colmax[192 + j]));
-                if (cm >= 0x7FF00000u) bad = true;
-                // A column outgrows its scale when its maximum is no longer
-                // below 2^(E - 1); the new scale leaves HEADROOM bits above it.
-                const int need = cm >= 0x00100000u ? (int)(cm >> 20) - 1023 + 2 + HEADROOM : E_UNSET;
-                const bool over = need != E_UNSET && (E == E_UNSET || (int)(cm >> 20) - 1023 >= E - 1);
-                const bool any_over = any(over);
-                if (any_over || epoch_full) {
-                    const bool drained = s > epoch_start ? drain(s - 1) : true;
-                    if (tid == 0 && s > epoch_start) {
-                        atomicAdd(&flags->drains, 1);
-                        if (any_over) atomicAdd(&flags->rescales, 1);
-                    }
-                    if (any(!drained)) { fail(); break; }
-                    if (over) E = E == E_UNSET ? need : max(E, need);
-                    if (kq == 0 && !jw) Es[j] = E;
-                    epoch_start = s;
-                    fresh = true;
-                    if (any_over) {
-                        sc = (E == E_UNSET || bad) ? 0.0 : pow2(51 - E);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const double first = jw ? v[2 * c + 1] : v[2 * c];
-                            const double second = jw ? v[2 * c] : v[2 * c + 1];
-                            t[2 * c] = (uint64_t)__double_as_longlong(fma(first, sc, magic));
-                            t[2 * c + 1] = (uint64_t)__double_as_longlong(fma(second, jw ? -sc : sc, magic));
-                        }
-                    }
+                for (int r = 0; r < ROWS; ++r) {
+                    const double2 z =
+                        *reinterpret_cast<const double2*>(col + (r >> 3) * (FBYTES / 2) + (((r & 7) ^ (c & 7)) << 4));
+                    mx = max(mx, (uint32_t)__double2hiint(z.x) & 0x7FFFFFFFu);
+                    mx = max(mx, (uint32_t)__double2hiint(z.y) & 0x7FFFFFFFu);
+                    low |= (uint32_t)__double2loint(z.x) | (uint32_t)__double2loint(z.y);
+                    sq[r & 1] = fma(z.x, z.x, sq[r & 1]);
+                    sq[2 + (r & 1)] = fma(z.y, z.y, sq[2 + (r & 1)]);
                 }
             }
-            uint32_t w0[SLICES], w1[SLICES];
-            {
-                const uint64_t y0[4] = {t[0] << 4, t[1] << 4, t[2] << 4, t[3] << 4};
-                const uint64_t y1[4] = {t[4] << 4, t[5] << 4, t[6] << 4, t[7] << 4};
-                slice_words(y0, w0);
-                slice_words(y1, w1);
+            bool over = mx >= limit;
+            if (mx >= 0x7FF00000u) { bad = true; over = false; }   // Inf or NaN
+            if (E == SPLIT_E_UNSET && mx < 0x00100000u) tiny |= mx | low;
+            const bool epoch_full = s - epoch_start >= C::EPOCH_STAGES;
+            const int Eold = E;
+            bool any_over = false;
+            if (any(over || stop)) {
+                if (any(stop)) {
+                    *abort_flag = 1;
+                    break;
+                }
+                any_over = true;
+                if (over) {
+                    // The maximum lies in [2^e, 2^(e + 1)), e = the exponent:
+                    // the scale leaves HEADROOM bits above that.
+                    E = (int)(mx >> 20) - 1023 + 1 + HEADROOM;
+                    // The limit's exponent stays in range: a scale past it is
+                    // refused afterwards by split_sum_kernel anyway.
+                    limit = ((uint32_t)min(max(E - 1 + 1023, 1), 0x7FE) << 20) | 0xFC000u;
+                }
             }
-            // The MMAs of stage s - 1 still read A and, two stages back, B:
-            // wait for them, then write this stage's slices.
-            if (s >= 1 && !mbar_wait(&sl_empty[(s - 1) % SBUFS], ((s - 1) / SBUFS) & 1)) timed_out = true;
-            umma::fence_after_sync();
-            unsigned char* bbuf = smem + OFF_B + (size_t)sb * BTILE;
-            const uint32_t boff = sw32_offset(j, kq >> 1) + (kq & 1) * 8;
-#pragma unroll
-            for (int tt = 0; tt < SLICES; ++tt) {
-                umma::tmem_st2(taddr + lane_base + A_COL + 8 * tt + 2 * kq, w0[tt], w1[tt]);
-                if (!jw) *reinterpret_cast<uint2*>(bbuf + boff + tt * (64 * 32)) = make_uint2(w0[tt], w1[tt]);
+            const bool fresh = s == 0 || any_over || epoch_full;
+            if (fresh) {
+                ++epoch;
+                epoch_start = s;
             }
-            umma::tmem_wait_st();
-            umma::fence_smem_to_async();
-            umma::fence_before_sync();
-            if (tid == 0) fresh_flag[sb] = fresh ? 1 : 0;
-            mbar_arrive(&sl_full[sb]);
+            slots[b].E[c] = E;
+            slots[b].Eold[c] = Eold;
+            if (c == 0) {
+                slots[b].fresh = fresh ? 1 : 0;
+                slots[b].epoch = epoch;
+            }
+            mbar_arrive(&sc_full[b]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&fp_empty[b]);
+            if (++b == C::SLOTS) { b = 0; ph ^= 1u; }
         }
-        if (s == nstages && nstages > 0) {
-            if (any(!drain(nstages - 1))) fail();
-            if (tid == 0) atomicAdd(&flags->drains, 1);
-        }
-        if (bad) atomicExch(&flags->nonfinite, 1);
+        if (bad) *bad_flag = 1;
+        stat->E[c] = E;
+        stat->tiny[c] = E == SPLIT_E_UNSET && tiny != 0 ? 1 : 0;
+        stat->sumsq[c] = (sq[0] + sq[1]) + (sq[2] + sq[3]);
     }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
+    if (threadIdx.x == 0) stat->invalid = (*abort_flag || *bad_flag) ? 1 : 0;
     if (warp == 0) umma::tmem_dealloc(taddr, TMEM_COLS);
 }
 
-// G = alpha (sum over CTAs) + beta C: Re G[a][b] = P[b][a], Im G[a][b] =
-// -P[b][64 + a]. Re comes out symmetric to the bit (its slice products are
-// symmetric integers); Im is made antisymmetric to the bit by taking half the
-// difference of the two mirrored sums, since the slices of -x are not the
-// negated slices of x and so the kept products differ in their last bits.
-__global__ void ozaki_gram_reduce_kernel(z64* __restrict__ C, int64_t ldc, int k, int nctas,
-                                         const double* __restrict__ partial, const Flags* __restrict__ flags,
-                                         z64 alpha, z64 beta, const ChainStatus* st, int gate) {
+// Blocks 0..63 of a tile: its columns summed over the chunks in a fixed order
+// (four interleaved runs of chunks, then the four), a folded tile's two halves
+// added. Block 64: the tile's verdict.
+//
+// The verdict compares what the slices leave out with what the column weighs.
+// With scale 2^E an entry is off by at most 2^(E - 51) (V: 2^(E - 50)), which
+// reaches G_ij as an error of about 2^(E_j - 50) / sqrt(12) ||a_i||; the
+// products left out (three digit pairs a K row, digits of standard deviation
+// 74) add about sqrt(6 N) 74^2 2^(E_i + E_j - 70). Both stay below
+// 2^-54 ||a_i|| ||a_j||, under the rounding of the FP64 sums themselves, when
+//     ||a_j||^2 >= 4^E_j max(21.4, 0.21 sqrt(N)),
+// which the kernel checks per column (N Gaussian rows give about 2 N / 400).
+// A spike that dwarfs the rest of its column fails it, as do Inf and NaN, a
+// scale whose products could leave the FP64 range, and a wait that gave up:
+// the caller then computes the tile in FP64 instead.
+constexpr int SUM_THREADS = 512;
+
+__global__ void __launch_bounds__(SUM_THREADS)
+split_sum_kernel(SplitShape sh, int64_t rows, const double* __restrict__ partial, const SplitStat* __restrict__ stats,
+                 double* __restrict__ sums, int* __restrict__ verdict, const ChainStatus* st, int gate) {
     if (gated_off(st, gate)) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t entry = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (entry >= (int64_t)k * k) return;
-    const int a = (int)(entry % k), b = (int)(entry / k);
-    double re = 0.0, im_ab = 0.0, im_ba = 0.0;
-    for (int c = lane; c < nctas; c += 32) {
-        const double* p = partial + (size_t)c * (128 * 64);
-        re += p[(size_t)b * 128 + a];
-        im_ab -= p[(size_t)b * 128 + 64 + a];
-        im_ba -= p[(size_t)a * 128 + 64 + b];
+    __shared__ double red[SUM_THREADS];
+    __shared__ int redE[SUM_THREADS];
+    __shared__ int flags;
+    const int tile = blockIdx.y, tid = threadIdx.x;
+    const int m = tid & 127, part = tid >> 7;
+    const bool full = !sh.hermitian || tile >= sh.nt_a;
+    if (blockIdx.x < 64) {
+        const double* p = partial + (size_t)tile * sh.nchunks * SPLIT_TILE_DOUBLES + blockIdx.x * 128 + m;
+        double s = 0.0;
+#pragma unroll 8
+        for (int c = part; c < sh.nchunks; c += 4) s += p[(size_t)c * SPLIT_TILE_DOUBLES];
+        red[tid] = s;
+        __syncthreads();
+        if (tid >= 128) return;
+        s = (red[tid] + red[128 + tid]) + (red[256 + tid] + red[384 + tid]);
+        if (!full) {
+            __syncthreads();
+            red[tid] = s;
+            __syncthreads();
+            if (tid >= 64) return;
+            s += red[64 + tid];
+        }
+        sums[(size_t)tile * SPLIT_TILE_DOUBLES + blockIdx.x * 128 + m] = s;
+        return;
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        re += __shfl_down_sync(0xffffffffu, re, off);
-        im_ab += __shfl_down_sync(0xffffffffu, im_ab, off);
-        im_ba += __shfl_down_sync(0xffffffffu, im_ba, off);
+    if (tid == 0) flags = 0;
+    __syncthreads();
+    const int columns = full ? 128 : 64;
+    int E = SPLIT_E_UNSET, mine = 0;
+    double s = 0.0;
+    for (int c = part; c < sh.nchunks; c += 4) {
+        const SplitStat& x = stats[(size_t)tile * sh.nchunks + c];
+        if (m == 0 && x.invalid) mine |= SPLIT_INVALID;
+        if (m < columns) {
+            E = max(E, x.E[m]);
+            s += x.sumsq[m];
+            if (x.tiny[m]) mine |= SPLIT_INACCURATE;
+        }
     }
-    if (lane != 0) return;
-    double im = a == b ? 0.0 : 0.5 * (im_ab - im_ba);
-    if (flags->timeout || flags->nonfinite) re = im = __longlong_as_double(0x7ff8000000000000ll);
-    z64 out = zmul(alpha, zmake(re, im));
-    z64* dst = C + a + (int64_t)b * ldc;
-    if (beta.x != 0.0 || beta.y != 0.0) zmac(out, beta, *dst);
-    *dst = out;
+    red[tid] = s;
+    redE[tid] = E;
+    __syncthreads();
+    if (tid < columns) {
+        s = (red[tid] + red[128 + tid]) + (red[256 + tid] + red[384 + tid]);
+        E = max(max(redE[tid], redE[128 + tid]), max(redE[256 + tid], redE[384 + tid]));
+        if (E != SPLIT_E_UNSET &&
+            !(E >= -450 && E <= 450 && s >= fmax(21.4, 0.21 * sqrt((double)rows)) * pow2(2 * E)))
+            mine |= SPLIT_INACCURATE;
+    }
+    if (mine) atomicOr(&flags, mine);
+    __syncthreads();
+    if (tid == 0) verdict[tile] = flags;
 }
 
-struct Shape {
-    int nctas;
-    int64_t chunk_rows;
-};
-
-static Shape shape_of(int64_t rows) {
-    Shape s{};
-    const int64_t sms = sm_count();
-    const int64_t stages = (rows + ROWS - 1) / ROWS;
-    const int64_t per = (stages + sms - 1) / sms;
-    s.chunk_rows = per * ROWS;
-    s.nctas = s.chunk_rows > 0 ? (int)((rows + s.chunk_rows - 1) / s.chunk_rows) : 0;
-    return s;
+template <bool FULL>
+static int launch(const CUtensorMap& ma, const CUtensorMap& mb, int64_t rows, const SplitShape& sh, int ntiles,
+                  double* partial, SplitStat* stats, cudaStream_t stream, const ChainStatus* st, int gate, int chunk0,
+                  int chunk1) {
+    using C = Cfg<FULL>;
+    FB_CUDA(cudaFuncSetAttribute(split_gram_kernel<FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM),
+            "cudaFuncSetAttribute(split_gram_kernel)");
+    split_gram_kernel<FULL><<<dim3((unsigned)ntiles, (unsigned)(chunk1 - chunk0)), C::THREADS, C::SMEM, stream>>>(
+        ma, mb, rows, sh, partial, stats, st, gate, chunk0);
+    FB_LAUNCHED("split_gram_kernel");
+    return FB_OK;
 }
 
-}  // namespace ozaki
+}  // namespace split
 
-size_t ozaki_gram_workspace_size(int64_t rows) {
-    const ozaki::Shape s = ozaki::shape_of(rows);
-    return align_up(sizeof(ozaki::Flags), 256) + (size_t)(s.nctas > 0 ? s.nctas : 1) * 128 * 64 * sizeof(double);
+// One chunk per SM for the launch with fewer tiles, in whole stages.
+SplitShape split_shape(int64_t rows, int kA, int kB, bool hermitian) {
+    SplitShape sh{};
+    sh.nt_a = (kA + 63) / 64;
+    sh.nt_b = (kB + 63) / 64;
+    sh.hermitian = hermitian ? 1 : 0;
+    sh.ntiles = hermitian ? sh.nt_a * (sh.nt_a + 1) / 2 : sh.nt_a * sh.nt_b;
+    int smallest = sh.ntiles;
+    if (hermitian && sh.nt_a > 1) smallest = std::min(sh.nt_a, sh.nt_a * (sh.nt_a - 1) / 2);
+    const int64_t stages = (rows + SPLIT_STAGE_ROWS - 1) / SPLIT_STAGE_ROWS;
+    const int64_t target = std::max<int64_t>(1, sm_count() / smallest);
+    sh.chunk_rows = std::max<int64_t>(1, (stages + target - 1) / target) * SPLIT_STAGE_ROWS;
+    sh.nchunks = (int)((rows + sh.chunk_rows - 1) / sh.chunk_rows);
+    return sh;
 }
 
-// C = alpha A^H A + beta C for a rows x k matrix A, k <= 64, on the integer
-// tensor cores. workspace: ozaki_gram_workspace_size(rows) bytes.
-int ozaki_gram_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, int64_t rows, int k, z64 alpha, z64 beta,
-                       void* workspace, size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st,
-                       int gate) {
-    if (k < 1 || k > 64) {
-        set_error(FB_ENOTSUP, "the tensor-core Gram handles 1 <= k <= 64, got k = %d", k);
-        return FB_ENOTSUP;
-    }
-    if (rows > ((int64_t)1 << 30)) {
-        set_error(FB_ENOTSUP, "the tensor-core Gram handles at most 2^30 rows, got %lld", (long long)rows);
-        return FB_ENOTSUP;
-    }
-    const size_t need = ozaki_gram_workspace_size(rows);
-    if (!workspace || workspace_bytes < need) {
-        set_error(FB_ENOMEM, "tensor-core gram: workspace of %zu bytes is smaller than the %zu bytes needed",
-                  workspace_bytes, need);
-        return FB_ENOMEM;
-    }
-    const ozaki::Shape s = ozaki::shape_of(rows);
-    ozaki::Flags* flags = static_cast<ozaki::Flags*>(workspace);
-    double* partial = reinterpret_cast<double*>(static_cast<char*>(workspace) + align_up(sizeof(ozaki::Flags), 256));
-    FB_CUDA(cudaMemsetAsync(flags, 0, sizeof(ozaki::Flags), stream), "cudaMemsetAsync");
-    if (s.nctas > 0) {
-        CUtensorMap tm;
-        FB_TRY(encode_panel_map(&tm, A, rows, k, lda, 64));
-        FB_CUDA(cudaFuncSetAttribute(ozaki::ozaki_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)ozaki::SMEM_BYTES), "cudaFuncSetAttribute");
-        ozaki::ozaki_gram_kernel<<<s.nctas, ozaki::THREADS, ozaki::SMEM_BYTES, stream>>>(
-            tm, rows, s.chunk_rows, partial, flags, st, gate);
-        FB_LAUNCHED("ozaki_gram_kernel");
-    } else {
-        FB_CUDA(cudaMemsetAsync(partial, 0, 128 * 64 * sizeof(double), stream), "cudaMemsetAsync");
-    }
-    const int64_t threads = (int64_t)k * k * 32;
-    ozaki::ozaki_gram_reduce_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(
-        C, ldc, k, s.nctas > 0 ? s.nctas : 1, partial, flags, alpha, beta, st, gate);
-    FB_LAUNCHED("ozaki_gram_reduce_kernel");
+SplitLayout split_layout(const SplitShape& sh) {
+    SplitLayout L{};
+    const size_t parts = (size_t)sh.ntiles * (size_t)(sh.nchunks > 0 ? sh.nchunks : 1);
+    L.verdict = 0;
+    L.sums = align_up((size_t)sh.ntiles * sizeof(int), 256);
+    L.stats = L.sums + (size_t)sh.ntiles * SPLIT_TILE_DOUBLES * sizeof(double);
+    L.partial = align_up(L.stats + parts * sizeof(SplitStat), 256);
+    L.total = L.partial + parts * SPLIT_TILE_DOUBLES * sizeof(double);
+    return L;
+}
+
+int split_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
+                           const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st, int gate,
+                           int chunk0, int chunk1) {
+    if (chunk0 < 0) chunk0 = 0;
+    if (chunk1 > sh.nchunks) chunk1 = sh.nchunks;
+    if (chunk0 >= chunk1) return FB_OK;
+    const SplitLayout L = split_layout(sh);
+    char* ws = static_cast<char*>(workspace);
+    double* partial = reinterpret_cast<double*>(ws + L.partial);
+    SplitStat* stats = reinterpret_cast<SplitStat*>(ws + L.stats);
+    CUtensorMap ma, mb;
+    FB_TRY(encode_panel_map(&ma, A, rows, kA, lda, 64));
+    FB_TRY(encode_panel_map(&mb, B, rows, kB, ldb, 64));
+    const int full = sh.hermitian ? sh.ntiles - sh.nt_a : sh.ntiles;
+    if (sh.hermitian)
+        FB_TRY(split::launch<false>(ma, mb, rows, sh, sh.nt_a, partial, stats, stream, st, gate, chunk0, chunk1));
+    if (full > 0)
+        FB_TRY(split::launch<true>(ma, mb, rows, sh, full, partial, stats, stream, st, gate, chunk0, chunk1));
+    return FB_OK;
+}
+
+int split_sum_enqueue(int64_t rows, const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st,
+                      int gate) {
+    const SplitLayout L = split_layout(sh);
+    char* ws = static_cast<char*>(workspace);
+    split::split_sum_kernel<<<dim3(65, (unsigned)sh.ntiles), split::SUM_THREADS, 0, stream>>>(
+        sh, rows, reinterpret_cast<const double*>(ws + L.partial), reinterpret_cast<const SplitStat*>(ws + L.stats),
+        reinterpret_cast<double*>(ws + L.sums), reinterpret_cast<int*>(ws + L.verdict), st, gate);
+    FB_LAUNCHED("split_sum_kernel");
     return FB_OK;
 }
 
 }  // namespace fb
 
-using namespace fb;
-
-extern "C" {
-
-int fb_zgram_tc_workspace_size(int64_t rows, int k, size_t* bytes) {
-    if (!bytes || rows < 0 || k < 0) { set_error(FB_EINVAL, "fb_zgram_tc_workspace_size: bad argument"); return FB_EINVAL; }
-    *bytes = ozaki_gram_workspace_size(rows);
-    return FB_OK;
-}
-
-int fb_zgram_tc(fb_z128* C, int64_t ldc, const fb_z128* A, int64_t lda, int64_t rows, int k, fb_z128 alpha,
-                fb_z128 beta, void* workspace, size_t workspace_bytes, fb_queue_t queue) {
-    if (rows < 0 || k < 0) { set_error(FB_EDIM, "fb_zgram_tc: negative size"); return FB_EDIM; }
-    if (k == 0) return FB_OK;
-    if (!C || (!A && rows > 0)) { set_error(FB_EINVAL, "fb_zgram_tc: NULL matrix"); return FB_EINVAL; }
-    if (ldc < k || (rows > 0 && lda < rows)) { set_error(FB_EDIM, "fb_zgram_tc: leading dimension too small"); return FB_EDIM; }
-    if ((uintptr_t)A & 15) { set_error(FB_EINVAL, "fb_zgram_tc: A must be 16-byte aligned"); return FB_EINVAL; }
-    return ozaki_gram_enqueue(reinterpret_cast<z64*>(C), ldc, reinterpret_cast<const z64*>(A), lda, rows, k,
-                              zmake(alpha.re, alpha.im), zmake(beta.re, beta.im), workspace, workspace_bytes,
-                              stream_of(queue), nullptr, GATE_ALWAYS);
-}
-
-}  // extern "C"
