@@ -42,14 +42,23 @@
 // tile, then the column's scale grows with HEADROOM spare bits.
 //
 // What bounds it and how the work is laid out: a stage of 16 rows costs 512
-// cycles of integer MMA for a folded tile, about as many of 32-bit integer
-// work to cut and transpose the slices, and 709 cycles of HBM time. So nothing
-// may serialize: the decision about scales is made by scanner warps a few
-// stages ahead of the slicers (so slicers never vote), and the slicers form
-// GROUPS groups of four warps that take the stages in turn, each with a slice
-// buffer of its own, so one group's load, cut and store chain overlaps the
-// others' and the MMAs. Every wait is bounded; a failed one stops the CTA and
-// marks its result invalid.
+// cycles of integer MMA for a folded tile, about 600 of 32-bit integer work to
+// cut and transpose the slices, 709 of HBM time, and shared memory traffic:
+// the tile coming in, its rows read once by the slicers, the W slices written
+// and read back by the MMAs. Operand A therefore lives in tensor memory (two
+// buffers of it beside the accumulators for a folded tile, one for a full
+// one): with A in shared memory too, and separate warps reading every entry
+// once more for the scales, that traffic alone took 1190 cycles a stage and
+// bound the kernel. Nothing may serialize either: the slicers form GROUPS
+// groups that take the stages in turn, so one group's load, cut and store
+// chain overlaps the others' and the MMAs; a group publishes its stage's
+// column maxima, a decider warp turns them into scales in stage order, and no
+// slicer ever waits on another group's slicing. Every wait is bounded; a
+// failed one stops the CTA and marks its result invalid. Measured: 2.80 ms for
+// 10^7 x 64 folded (5.18 on the FP64 tensor cores), 5.70 ms for 64 x 64 cross
+// products (9.20); the integer pipe is 62 % busy, HBM 56 %.
+#include <type_traits>
+
 #include "fb_gram_split.cuh"
 #include "fb_umma.cuh"
 
@@ -60,36 +69,41 @@ constexpr int SLICES = 7;
 constexpr int ROWS = SPLIT_STAGE_ROWS;          // complex rows per stage: K = 32 bytes
 constexpr int FBYTES = ROWS * 64 * 16;          // 16 KB: 16 rows x 64 columns
 constexpr int BTILE = SLICES * 64 * 32;         // B: 7 x 64 rows x 32 bytes
-constexpr int ATILE = 128 * 32;                 // one A operand
-constexpr int TMEM_COLS = 512;                  // 448 used; the allocation is a power of two
+constexpr int TMEM_COLS = 512;
 constexpr int HEADROOM = 2;                     // spare exponent bits above the maximum that set a scale
 constexpr long long MAGIC_BITS = 0x4338080808080808ll;  // 2^52 + 2^51 + 0x80808080808
 
 template <bool FULL>
 struct Cfg {
     static constexpr int SIDES = FULL ? 2 : 1;                 // input tiles per stage
-    static constexpr int GROUPS = FULL ? 3 : 4;                // slicer groups of 128 threads = slice buffers
-    static constexpr int SLOTS = FULL ? 3 : 6;                 // FP64 ring depth
-    static constexpr int NA = FULL ? SLICES : 4;               // A operands per stage
-    static constexpr int SCANNERS = 64 * SIDES;                // scanner threads, one per input column
-    static constexpr int SLICERS = 128 * GROUPS;
-    static constexpr int THREADS = SLICERS + 64 + SCANNERS;
-    static constexpr int BUF = NA * ATILE + BTILE;             // one slice buffer: A operands, then B
+    static constexpr int GROUPS = FULL ? 2 : 4;                // slicer groups = B buffers
+    static constexpr int GWARPS = 4 * SIDES;                   // warps of a group: a set of four per input tile
+    static constexpr int SLOTS = FULL ? 6 : 10;                // FP64 ring depth
+    static constexpr int NA = FULL ? SLICES : 4;               // A operands per stage, 8 columns of tensor memory each
+    static constexpr int ABUFS = FULL ? 1 : 2;                 // stages of A operands held
+    static constexpr int COLUMNS = 64 * SIDES;                 // input columns
+    static constexpr int SLICERS = 32 * GWARPS * GROUPS;
+    static constexpr int THREADS = SLICERS + 96;           // and the issuer, producer and decider warps
     // int32 headroom: products are at most 2^14, a block gets 7 (full) or 4
     // (folded) of them per K row and 2 K rows per complex row.
     static constexpr int EPOCH_STAGES = (FULL ? 8192 : 12288) / ROWS;
-    struct Slot {                                              // what the scanners say about a stage
-        int E[64 * SIDES], Eold[64 * SIDES];
+    struct Stage {                                             // of the stage a group is working on
+        uint32_t colmax[64 * SIDES];                           // slicers: high words of the column maxima
+        int E[64 * SIDES], Eold[64 * SIDES];                   // decider: scales of this stage and the one before
         int fresh, epoch;
+        int mma_fresh;                                         // fresh, kept by the slicers until the MMAs are issued
     };
     static constexpr size_t OFF_F = 0;
-    static constexpr size_t OFF_S = OFF_F + (size_t)SLOTS * SIDES * FBYTES;
-    static constexpr size_t OFF_SLOT = OFF_S + (size_t)GROUPS * BUF;
-    static constexpr size_t OFF_BAR = (OFF_SLOT + SLOTS * sizeof(Slot) + 15) / 16 * 16;
-    static constexpr size_t OFF_MISC = OFF_BAR + (3 * SLOTS + 2 * GROUPS) * 8;
+    static constexpr size_t OFF_B = OFF_F + (size_t)SLOTS * SIDES * FBYTES;
+    static constexpr size_t OFF_STAGE = OFF_B + (size_t)GROUPS * BTILE;
+    static constexpr size_t OFF_BAR = (OFF_STAGE + GROUPS * sizeof(Stage) + 15) / 16 * 16;
+    static constexpr size_t OFF_MISC = OFF_BAR + (2 * SLOTS + 4 * GROUPS) * 8;
     static constexpr size_t SMEM = OFF_MISC + 64 + 1024;       // + alignment slack
 };
 static_assert(Cfg<false>::SMEM <= 227 * 1024 && Cfg<true>::SMEM <= 227 * 1024, "a CTA's shared memory");
+constexpr int A_COL = 64 * SLICES;                             // tensor memory column of the first A operand
+static_assert(A_COL + 8 * Cfg<false>::NA * Cfg<false>::ABUFS <= TMEM_COLS, "accumulators and A operands");
+static_assert(A_COL + 8 * Cfg<true>::NA * Cfg<true>::ABUFS <= TMEM_COLS, "accumulators and A operands");
 
 __device__ __forceinline__ uint32_t sw32_offset(uint32_t row, uint32_t chunk) {
     return row * 32 + ((chunk ^ ((row >> 2) & 1)) << 4);
@@ -135,32 +149,37 @@ __device__ __forceinline__ void slice_words(const uint64_t (&y)[4], uint32_t (&w
     w[6] = __byte_perm(a01, a23, 0x5410) ^ 0x80808080u;  // byte 0
 }
 
+// The largest high word of |x| over eight values, taken as single-precision
+// magnitudes, which order like the words themselves and whose comparison
+// drops the sign for free. A word past single precision's range (|x| >= 2^1017,
+// Inf, NaN) propagates as a NaN, 0x7FFFFFFF.
+__device__ __forceinline__ uint32_t max_hi(const double (&v)[8]) {
+    float m = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(fabsf(__int_as_float(__double2hiint(v[e])))));
+    return (uint32_t)__float_as_int(m);
+}
+
 // What an operand's K rows are made of, from a complex entry (re, im).
 enum Form { FORM_W, FORM_JW, FORM_V };
 
-// Cuts eight complex rows of one column (v: re, im alternating) into the 16
-// K bytes of every slice and stores slice t at base(t).
-template <Form F, class Base>
-__device__ __forceinline__ void cut(const double (&v)[16], double sc, Base base) {
+// Cuts two complex rows of one column (re, im, re, im) into the four K bytes
+// of every slice.
+template <Form F>
+__device__ __forceinline__ void cut(const double* v, double sc, uint32_t (&w)[SLICES]) {
     const double magic = __longlong_as_double(MAGIC_BITS);
-    uint32_t w[4][SLICES];
+    uint64_t y[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uint64_t y[4];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const double re = v[4 * q + 2 * r], im = v[4 * q + 2 * r + 1];
-            double a = re, b = im;
-            if (F == FORM_JW) { a = -im; b = re; }
-            if (F == FORM_V) { a = re - im; b = re + im; }
-            y[2 * r] = (uint64_t)__double_as_longlong(fma(a, sc, magic)) << 4;
-            y[2 * r + 1] = (uint64_t)__double_as_longlong(fma(b, sc, magic)) << 4;
-        }
-        slice_words(y, w[q]);
+    for (int r = 0; r < 2; ++r) {
+        const double re = v[2 * r], im = v[2 * r + 1];
+        double a = re, b = im;
+        if (F == FORM_JW) { a = -im; b = re; }
+        if (F == FORM_V) { a = re - im; b = re + im; }
+        y[2 * r] = (uint64_t)__double_as_longlong(fma(a, sc, magic)) << 4;
+        y[2 * r + 1] = (uint64_t)__double_as_longlong(fma(b, sc, magic)) << 4;
     }
-#pragma unroll
-    for (int t = 0; t < SLICES; ++t)
-        *reinterpret_cast<uint4*>(base(t)) = make_uint4(w[0][t], w[1][t], w[2][t], w[3][t]);
+    slice_words(y, w);
 }
 
 // Adds the accumulators into the partial tile P (128 x 64 doubles, column n
@@ -174,6 +193,7 @@ __device__ __noinline__ void drain_epoch(uint32_t tmem_lane, const int* EA, cons
     const int Em = EA[prow & 63];
     // Weight of block c: 2^(E_a + E_b + 2 - 8 g), V's halved scale one more.
     const int shift = FULL ? 2 : (prow < 64 ? 3 : 3 - 8);
+#pragma unroll 1
     for (int cc = 0; cc < 4; ++cc) {
         double acc[16];
 #pragma unroll
@@ -209,21 +229,22 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     using C = Cfg<FULL>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    typename C::Slot* slots = reinterpret_cast<typename C::Slot*>(smem + C::OFF_SLOT);
+    typename C::Stage* stages = reinterpret_cast<typename C::Stage*>(smem + C::OFF_STAGE);
     uint64_t* fp_full = reinterpret_cast<uint64_t*>(smem + C::OFF_BAR);   // a stage's rows have landed
-    uint64_t* fp_empty = fp_full + C::SLOTS;                              // scanned and loaded by its slicers
-    uint64_t* sc_full = fp_empty + C::SLOTS;                              // scanned
-    uint64_t* sl_full = sc_full + C::SLOTS;                               // a group's slices are written
+    uint64_t* fp_empty = fp_full + C::SLOTS;                              // and are in its slicers' registers
+    uint64_t* mx_full = fp_empty + C::SLOTS;                              // a group's column maxima are published
+    uint64_t* sc_full = mx_full + C::GROUPS;                              // and its scales
+    uint64_t* sl_full = sc_full + C::GROUPS;                              // its slices are written
     uint64_t* sl_empty = sl_full + C::GROUPS;                             // and consumed by the MMAs
     int* misc = reinterpret_cast<int*>(smem + C::OFF_MISC);
     volatile int* abort_flag = misc;
     int* bad_flag = misc + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 2);
-    volatile int* fresh_flag = misc + 4;   // [GROUPS]
 
     int ti, tj, tile;
     split_tile_of(sh, FULL, (int)blockIdx.x, ti, tj, tile);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // Taken from one lane, so that the branches on it are known to be uniform.
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int chunk = chunk0 + (int)blockIdx.y;
     const int64_t row0 = (int64_t)chunk * sh.chunk_rows;
     const int64_t row_end = min(rows, row0 + sh.chunk_rows);
@@ -234,32 +255,24 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     if (threadIdx.x == 0) {
         for (int b = 0; b < C::SLOTS; ++b) {
             mbar_init(&fp_full[b], 1);
-            mbar_init(&fp_empty[b], 4 + C::SCANNERS / 32);
-            mbar_init(&sc_full[b], C::SCANNERS);
+            mbar_init(&fp_empty[b], C::GWARPS);
         }
         for (int b = 0; b < C::GROUPS; ++b) {
-            mbar_init(&sl_full[b], 4);
+            mbar_init(&mx_full[b], C::GWARPS);
+            mbar_init(&sc_full[b], 1);
+            mbar_init(&sl_full[b], C::GWARPS);
             mbar_init(&sl_empty[b], 1);
         }
         *abort_flag = 0;
         *bad_flag = 0;
         mbar_fence_init();
     }
-    if constexpr (!FULL) {
-        // The last A operand of a folded tile has one slice only: its rows
-        // 64-127 are zero for good.
-        for (int e = threadIdx.x; e < C::GROUPS * (ATILE / 2) / 16; e += blockDim.x) {
-            const int b = e / ((ATILE / 2) / 16), o = e - b * ((ATILE / 2) / 16);
-            reinterpret_cast<uint4*>(smem + C::OFF_S + (size_t)b * C::BUF + 3 * ATILE + ATILE / 2)[o] =
-                make_uint4(0, 0, 0, 0);
-        }
-    }
     if (warp == 0) umma::tmem_alloc(tmem_slot, TMEM_COLS);
-    umma::fence_smem_to_async();
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t taddr = *tmem_slot;
+    double sumsq[2] = {0.0, 0.0};                            // of a slicer's two columns
 
     if (warp == C::SLICERS / 32 + 1) {
         // ---- producer: FP64 tiles, two 8-row boxes per stage and input ----
@@ -302,9 +315,9 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                     break;
                 }
                 umma::fence_after_sync();
-                const bool fresh = fresh_flag[g] != 0;
-                const uint32_t abase = smem_u32(smem + C::OFF_S + (size_t)g * C::BUF);
-                const uint32_t bbase = abase + C::NA * ATILE;
+                const bool fresh = *(volatile int*)&stages[g].mma_fresh != 0;
+                const uint32_t atmem = taddr + A_COL + 8 * C::NA * (s % C::ABUFS);
+                const uint32_t bbase = smem_u32(smem + C::OFF_B + (size_t)g * BTILE);
 #pragma unroll
                 for (int a = 0; a < C::NA; ++a) {
                     const int first = FULL ? a : 2 * a;      // accumulator block of slice 1 of B
@@ -312,8 +325,8 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
                     for (int off = 0; off < ntot; off += 256) {
                         const int n = ntot - off < 256 ? ntot - off : 256;
-                        umma::mma_s8(taddr + 64 * first + off, desc_sw32(abase + a * ATILE),
-                                     desc_sw32(bbase + off * 32), umma::idesc_s8s8_s32(128, n), !(fresh && a == 0));
+                        umma::mma_s8_tmem_a(taddr + 64 * first + off, atmem + 8 * a, desc_sw32(bbase + off * 32),
+                                            umma::idesc_s8s8_s32(128, n), !(fresh && a == 0));
                     }
                 }
                 umma::commit(&sl_empty[g]);
@@ -327,176 +340,274 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         }
     } else if (warp < C::SLICERS / 32) {
         // ---- slicers ----
-        const int g = warp >> 2, q = warp & 3;
-        const int t128 = threadIdx.x & 127;
-        const int j = t128 & 63, kq = t128 >> 6;             // this thread's column and 8-row box
-        const int prow = 32 * q + lane;                      // its row of the accumulators
-        const uint32_t tmem_lane = taddr + ((uint32_t)(32 * q) << 16);
-        unsigned char* abuf = smem + C::OFF_S + (size_t)g * C::BUF;
-        unsigned char* bbuf = abuf + C::NA * ATILE;
-        const uint32_t off_lo = sw32_offset(j, kq), off_hi = sw32_offset(64 + j, kq);
-        // Waits are decided by the whole warp together, so that a warp leaves
-        // the loop as one.
-        auto wait = [&](uint64_t* bar, uint32_t parity) {
-            return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
-        };
-        auto load = [&](const unsigned char* tile_base, double (&v)[16]) {
-            const unsigned char* col = tile_base + (size_t)kq * (FBYTES / 2) + j * 128;
+        // Warp q of a set of four cuts columns 16 q .. 16 q + 15 of its input
+        // tile, lane (c8, i) columns m0 = 16 q + c8 and m0 + 8, rows 2 i and
+        // 2 i + 1 of both 8-row boxes: words i and 4 + i of a column's 32 K
+        // bytes. That is the layout of a 16-lane store to tensor memory,
+        // whose lanes c8 and c8 + 8 take the two halves of an A operand (two
+        // slices of V, or W and JW) of one column: accumulator lane
+        // 32 q + 16 n + c8 (+ 8) belongs to column 16 q + 8 n + c8.
+        const int g = warp / C::GWARPS, w = warp - g * C::GWARPS;
+        typename C::Stage& stage = stages[g];
+        auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity); };
+        // Until the MMAs of stage s are done. The barrier is at most one
+        // phase behind: this group has waited for its own previous stage,
+        // which is later than the one before s on that barrier.
+        auto wait_mma = [&](int s) { return wait(&sl_empty[s % C::GROUPS], (s / C::GROUPS) & 1); };
+        const int c8 = lane >> 2, i = lane & 3;
+
+        auto slicer = [&](auto side_tag) -> bool {
+            constexpr int SIDE = decltype(side_tag)::value;
+            constexpr int NC = 2;                             // columns a lane
+            constexpr bool TO_B = !FULL || SIDE == 1;         // cuts operand B
+            constexpr bool TO_A = SIDE == 0;
+            const int q = w & 3, m0 = 16 * q + c8;
+            unsigned char* bbuf = smem + C::OFF_B + (size_t)g * BTILE;
+            const uint32_t tmem_lane = taddr + ((uint32_t)(32 * q) << 16);
+            const int prow = ((lane >> 3) & 1) * 64 + 16 * q + 8 * (lane >> 4) + (lane & 7);
+            double v[NC][8];
+            // This warp's rows of stage s into registers, and its columns'
+            // maxima published: the high word of |x| orders magnitudes by
+            // exponent, and Inf and NaN above every finite value. A column of
+            // nothing but numbers below the high word's range reports 1.
+            auto load = [&](int s) -> bool {
+                const int b = s % C::SLOTS;
+                if (!wait(&fp_full[b], (s / C::SLOTS) & 1)) return false;
+                const unsigned char* f = smem + C::OFF_F + ((size_t)b * C::SIDES + SIDE) * FBYTES;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const double2 z = *reinterpret_cast<const double2*>(col + ((r ^ (j & 7)) << 4));
-                v[2 * r] = z.x;
-                v[2 * r + 1] = z.y;
+                for (int n = 0; n < NC; ++n)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const int m = m0 + 8 * n, row = 2 * i + (r & 1);
+                        const double2 z = *reinterpret_cast<const double2*>(f + (r >> 1) * (FBYTES / 2) + m * 128 +
+                                                                            ((row ^ (m & 7)) << 4));
+                        v[n][2 * r] = z.x;
+                        v[n][2 * r + 1] = z.y;
+                    }
+                return true;
+            };
+            auto publish = [&](int s) {
+#pragma unroll
+                for (int n = 0; n < NC; ++n) {
+                    uint32_t mx = max_hi(v[n]);
+                    if (mx == 0) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) mx |= __double2loint(v[n][e]) != 0 ? 1u : 0u;
+                    }
+                    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                    if (i == 0) stage.colmax[64 * SIDE + m0 + 8 * n] = mx;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&mx_full[g]);
+            };
+            // Sums of squares of the leading digits, in units of
+            // 4^(E - 7) of the scale they were cut with.
+            int E[NC], digits[NC];
+#pragma unroll
+            for (int n = 0; n < NC; ++n) { E[n] = SPLIT_E_UNSET; digits[n] = 0; }
+            auto fold = [&](int n) {
+                if (E[n] != SPLIT_E_UNSET) sumsq[n] += (double)digits[n] * pow2(2 * (E[n] - 7));
+                digits[n] = 0;
+            };
+            auto drain = [&](int s, const int* EA, const int* EB, bool initialized) -> bool {
+                if (!wait_mma(s)) return false;
+                umma::fence_after_sync();
+                drain_epoch<FULL>(tmem_lane, EA, EB, prow, P, initialized);
+                umma::fence_before_sync();
+                return true;
+            };
+            uint32_t gph = 0;                                 // parity of this group's stage count
+            int s = g;
+            if (s < nstages) {
+                if (!load(s)) return false;
+                publish(s);
             }
-        };
-        // Drains the accumulators once the MMAs of `stage` have finished.
-        auto drain = [&](int stage, const int* EA, const int* EB, bool initialized) {
-            if (!wait(&sl_empty[stage % C::GROUPS], (stage / C::GROUPS) & 1)) return false;
-            umma::fence_after_sync();
-            drain_epoch<FULL>(tmem_lane, EA, EB, prow, P, initialized);
-            umma::fence_before_sync();
+            for (; s < nstages; s += C::GROUPS, gph ^= 1u) {
+                if (!wait(&sc_full[g], gph) || __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+                const bool fresh = __any_sync(0xffffffffu, stage.fresh != 0);
+                // This group's B buffer is free once its previous stage's
+                // MMAs are done.
+                if (s >= C::GROUPS && !wait(&sl_empty[g], gph ^ 1u)) return false;
+                // A new epoch: the MMAs of the one before it all precede this
+                // stage's, which wait for this group. (The rows are read
+                // again, so that no register holds them across the drain.)
+                if (TO_A && fresh && s > 0) {
+                    if (!drain(s - 1, stage.Eold, stage.Eold + (FULL ? 64 : 0), stage.epoch > 1) || !load(s))
+                        return false;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&fp_empty[s % C::SLOTS]);
+                double sc[NC];
+#pragma unroll
+                for (int n = 0; n < NC; ++n) {
+                    const int En = stage.E[64 * SIDE + m0 + 8 * n];
+                    if (En != E[n] || (s / C::GROUPS) % 4096 == 0) {   // digits: 2^17 a stage at most
+                        fold(n);
+                        E[n] = En;
+                    }
+                    sc[n] = En == SPLIT_E_UNSET ? 0.0 : pow2(51 - En);
+                }
+                if constexpr (TO_B) {
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) {
+                        const int m = m0 + 8 * n;
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            uint32_t wd[SLICES];
+                            cut<FORM_W>(v[n] + 4 * x, sc[n], wd);
+                            digits[n] = __dp4a((int)wd[0], (int)wd[0], digits[n]);
+                            unsigned char* b0 = bbuf + sw32_offset(m, x) + 4 * i;
+#pragma unroll
+                            for (int t = 0; t < SLICES; ++t) *reinterpret_cast<uint32_t*>(b0 + t * (64 * 32)) = wd[t];
+                        }
+                    }
+                }
+                if constexpr (TO_A) {
+                    uint32_t lo[NC][2][SLICES], hi[FULL ? NC : 1][2][SLICES];
+#pragma unroll
+                    for (int n = 0; n < NC; ++n)
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            if constexpr (FULL) {
+                                cut<FORM_W>(v[n] + 4 * x, sc[n], lo[n][x]);
+                                cut<FORM_JW>(v[n] + 4 * x, sc[n], hi[n][x]);
+                                digits[n] = __dp4a((int)lo[n][x][0], (int)lo[n][x][0], digits[n]);
+                            } else {
+                                cut<FORM_V>(v[n] + 4 * x, 0.5 * sc[n], lo[n][x]);
+                            }
+                        }
+                    if (s >= C::ABUFS && !wait_mma(s - C::ABUFS)) return false;
+                    umma::fence_after_sync();
+                    const uint32_t at = tmem_lane + A_COL + 8 * C::NA * (s % C::ABUFS);
+#pragma unroll
+                    for (int n = 0; n < NC; ++n)
+#pragma unroll
+                        for (int a = 0; a < C::NA; ++a) {
+                            const uint32_t col = at + 8 * a + ((uint32_t)(16 * n) << 16);
+                            if constexpr (FULL)
+                                umma::tmem_st_16x128b_x2(col, lo[n][0][a], hi[n][0][a], lo[n][1][a], hi[n][1][a]);
+                            else
+                                umma::tmem_st_16x128b_x2(col, lo[n][0][2 * a], a < 3 ? lo[n][0][2 * a + 1] : 0,
+                                                         lo[n][1][2 * a], a < 3 ? lo[n][1][2 * a + 1] : 0);
+                        }
+                    umma::tmem_wait_st();
+                }
+                if (w == 0 && lane == 0) stage.mma_fresh = fresh ? 1 : 0;
+                umma::fence_smem_to_async();
+                umma::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sl_full[g]);
+                // The next stage's rows and maxima go out before this group
+                // comes back to it, so its scales are settled by then.
+                if (s + C::GROUPS < nstages) {
+                    if (!load(s + C::GROUPS)) return false;
+                    publish(s + C::GROUPS);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NC; ++n) fold(n);
+            // The group of the last stage drains the last epoch.
+            if (TO_A && s - C::GROUPS == nstages - 1)
+                return drain(nstages - 1, stage.E, stage.E + (FULL ? 64 : 0), stage.epoch > 0);
             return true;
         };
-        bool ok = true;
-        uint32_t gph = 1;                                     // parity of this group's previous commit
-        int s = g;
-        for (; s < nstages; s += C::GROUPS) {
-            const int b = s % C::SLOTS;
-            const uint32_t ph = (s / C::SLOTS) & 1;
-            if (!wait(&sc_full[b], ph) || !wait(&fp_full[b], ph) || *abort_flag) { ok = false; break; }
-            const typename C::Slot& slot = slots[b];
-            const bool fresh = slot.fresh != 0;
-            // This group's buffer is free once its previous stage's MMAs are
-            // done (waited for before a drain, too: it leaves the barrier of
-            // stage s - 1 at most one phase behind).
-            if (s >= C::GROUPS && !wait(&sl_empty[g], gph)) { ok = false; break; }
-            // A new epoch: the MMAs of the one before it all precede this
-            // stage's, which wait for this group.
-            if (fresh && s > 0 &&
-                !drain(s - 1, slot.Eold, slot.Eold + (FULL ? 64 : 0), slot.epoch > 1)) { ok = false; break; }
-            const unsigned char* f = smem + C::OFF_F + (size_t)b * C::SIDES * FBYTES;
-            const int EA = slot.E[j], EB = slot.E[(FULL ? 64 : 0) + j];
-            const double sca = EA == SPLIT_E_UNSET ? 0.0 : pow2((FULL ? 51 : 50) - EA);
-            const double scb = EB == SPLIT_E_UNSET ? 0.0 : pow2(51 - EB);
-            auto release = [&]() {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&fp_empty[b]);
-            };
-            double v[16];
-            if constexpr (FULL) {
-                load(f + FBYTES, v);
-                cut<FORM_W>(v, scb, [&](int t) { return bbuf + off_lo + t * (64 * 32); });
-                load(f, v);
-                release();
-                cut<FORM_W>(v, sca, [&](int t) { return abuf + t * ATILE + off_lo; });
-                cut<FORM_JW>(v, sca, [&](int t) { return abuf + t * ATILE + off_hi; });
-            } else {
-                load(f, v);
-                release();
-                cut<FORM_W>(v, scb, [&](int t) { return bbuf + off_lo + t * (64 * 32); });
-                cut<FORM_V>(v, sca, [&](int t) { return abuf + (t >> 1) * ATILE + ((t & 1) ? off_hi : off_lo); });
-            }
-            if (t128 == 0) fresh_flag[g] = fresh ? 1 : 0;
-            umma::fence_smem_to_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sl_full[g]);
-            gph ^= 1u;
-        }
+        bool ok;
+        if constexpr (FULL) ok = w < 4 ? slicer(std::integral_constant<int, 0>{}) : slicer(std::integral_constant<int, 1>{});
+        else ok = slicer(std::integral_constant<int, 0>{});
         if (!ok) *abort_flag = 1;
-        // The group of the last stage drains the last epoch.
-        if (ok && nstages > 0 && s - C::GROUPS == nstages - 1) {
-            const typename C::Slot& slot = slots[(nstages - 1) % C::SLOTS];
-            if (!drain(nstages - 1, slot.E, slot.E + (FULL ? 64 : 0), slot.epoch > 0)) *abort_flag = 1;
-        }
     } else {
-        // ---- scanners: scales, a few stages ahead of the slicers ----
-        const int c = (int)threadIdx.x - C::SLICERS - 64;    // input column: A's 0-63, then B's
-        auto any = [](bool p) -> bool {
-            uint32_t r;
-            asm volatile(
-                "{\n\t.reg .pred a, b;\n\t"
-                "setp.ne.u32 a, %1, 0;\n\t"
-                "barrier.cta.red.or.pred b, 1, %2, a;\n\t"
-                "selp.u32 %0, 1, 0, b;\n\t}"
-                : "=r"(r)
-                : "r"((uint32_t)p), "n"(C::SCANNERS)
-                : "memory");
-            return r != 0;
-        };
-        int E = SPLIT_E_UNSET;
+        // ---- decider: the scales, in stage order ----
+        // Lane l decides input columns l, l + 32, ... (A's 0-63, then B's).
         // |x| < 2^E (1 - 2^-7) in terms of the high word of x; while the
         // scale is unset every normal number is past it.
-        uint32_t limit = 0x00100000u;
-        uint32_t tiny = 0;                                   // bits of subnormal entries under an unset scale
-        bool bad = false;
-        double sq[4] = {0.0, 0.0, 0.0, 0.0};
-        int b = 0, epoch = -1, epoch_start = 0;
+        constexpr int NC = C::COLUMNS / 32;
+        int E[NC];
+        uint32_t limit[NC];
+        bool tiny[NC], bad = false;
+#pragma unroll
+        for (int x = 0; x < NC; ++x) {
+            E[x] = SPLIT_E_UNSET;
+            limit[x] = 0x00100000u;
+            tiny[x] = false;
+        }
+        int g = 0, epoch = -1, epoch_start = 0;
         uint32_t ph = 0;
         for (int s = 0; s < nstages; ++s) {
-            const bool landed = mbar_wait(&fp_full[b], ph);
-            const bool stop = !landed || *abort_flag;
-            const unsigned char* col =
-                smem + C::OFF_F + ((size_t)b * C::SIDES + (c >> 6)) * FBYTES + (c & 63) * 128;
-            uint32_t mx = 0, low = 0;
-            if (!stop) {
-#pragma unroll
-                for (int r = 0; r < ROWS; ++r) {
-                    const double2 z =
-                        *reinterpret_cast<const double2*>(col + (r >> 3) * (FBYTES / 2) + (((r & 7) ^ (c & 7)) << 4));
-                    mx = max(mx, (uint32_t)__double2hiint(z.x) & 0x7FFFFFFFu);
-                    mx = max(mx, (uint32_t)__double2hiint(z.y) & 0x7FFFFFFFu);
-                    low |= (uint32_t)__double2loint(z.x) | (uint32_t)__double2loint(z.y);
-                    sq[r & 1] = fma(z.x, z.x, sq[r & 1]);
-                    sq[2 + (r & 1)] = fma(z.y, z.y, sq[2 + (r & 1)]);
-                }
+            typename C::Stage& stage = stages[g];
+            if (!mbar_wait_warp(&mx_full[g], ph) || __any_sync(0xffffffffu, *abort_flag != 0)) {
+                *abort_flag = 1;
+                break;
             }
-            bool over = mx >= limit;
-            if (mx >= 0x7FF00000u) { bad = true; over = false; }   // Inf or NaN
-            if (E == SPLIT_E_UNSET && mx < 0x00100000u) tiny |= mx | low;
-            const bool epoch_full = s - epoch_start >= C::EPOCH_STAGES;
-            const int Eold = E;
-            bool any_over = false;
-            if (any(over || stop)) {
-                if (any(stop)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                any_over = true;
-                if (over) {
+            uint32_t mx[NC];
+            bool over[NC], mine = false;
+#pragma unroll
+            for (int x = 0; x < NC; ++x) {
+                mx[x] = stage.colmax[32 * x + lane];
+                over[x] = mx[x] >= limit[x];
+                if (mx[x] >= 0x7FF00000u) { bad = true; over[x] = false; }   // Inf, NaN or next to them
+                if (E[x] == SPLIT_E_UNSET && mx[x] != 0 && mx[x] < 0x00100000u) tiny[x] = true;
+                mine = mine || over[x];
+                stage.Eold[32 * x + lane] = E[x];
+            }
+            const bool any_over = __any_sync(0xffffffffu, mine);
+            if (any_over) {
+#pragma unroll
+                for (int x = 0; x < NC; ++x) {
+                    if (!over[x]) continue;
                     // The maximum lies in [2^e, 2^(e + 1)), e = the exponent:
                     // the scale leaves HEADROOM bits above that.
-                    E = (int)(mx >> 20) - 1023 + 1 + HEADROOM;
+                    E[x] = (int)(mx[x] >> 20) - 1023 + 1 + HEADROOM;
                     // The limit's exponent stays in range: a scale past it is
                     // refused afterwards by split_sum_kernel anyway.
-                    limit = ((uint32_t)min(max(E - 1 + 1023, 1), 0x7FE) << 20) | 0xFC000u;
+                    limit[x] = ((uint32_t)min(max(E[x] - 1 + 1023, 1), 0x7FE) << 20) | 0xFC000u;
                 }
             }
-            const bool fresh = s == 0 || any_over || epoch_full;
+            const bool fresh = s == 0 || any_over || s - epoch_start >= C::EPOCH_STAGES;
             if (fresh) {
                 ++epoch;
                 epoch_start = s;
             }
-            slots[b].E[c] = E;
-            slots[b].Eold[c] = Eold;
-            if (c == 0) {
-                slots[b].fresh = fresh ? 1 : 0;
-                slots[b].epoch = epoch;
+#pragma unroll
+            for (int x = 0; x < NC; ++x) stage.E[32 * x + lane] = E[x];
+            if (lane == 0) {
+                stage.fresh = fresh ? 1 : 0;
+                stage.epoch = epoch;
             }
-            mbar_arrive(&sc_full[b]);
             __syncwarp();
-            if (lane == 0) mbar_arrive(&fp_empty[b]);
-            if (++b == C::SLOTS) { b = 0; ph ^= 1u; }
+            if (lane == 0) mbar_arrive(&sc_full[g]);
+            if (++g == C::GROUPS) { g = 0; ph ^= 1u; }
         }
         if (bad) *bad_flag = 1;
-        stat->E[c] = E;
-        stat->tiny[c] = E == SPLIT_E_UNSET && tiny != 0 ? 1 : 0;
-        stat->sumsq[c] = (sq[0] + sq[1]) + (sq[2] + sq[3]);
+#pragma unroll
+        for (int x = 0; x < NC; ++x) {
+            stat->E[32 * x + lane] = E[x];
+            stat->tiny[32 * x + lane] = E[x] == SPLIT_E_UNSET && tiny[x] ? 1 : 0;
+        }
     }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     if (threadIdx.x == 0) stat->invalid = (*abort_flag || *bad_flag) ? 1 : 0;
     if (warp == 0) umma::tmem_dealloc(taddr, TMEM_COLS);
+    // The columns' sums of squares, over the four lanes of a column, then the
+    // groups in order (the ring is free by now).
+    double* sq = reinterpret_cast<double*>(smem + C::OFF_F);
+    if (warp < C::SLICERS / 32) {
+        const int g = warp / C::GWARPS, w = warp - g * C::GWARPS;
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            sumsq[n] += __shfl_xor_sync(0xffffffffu, sumsq[n], 1);
+            sumsq[n] += __shfl_xor_sync(0xffffffffu, sumsq[n], 2);
+            if ((lane & 3) == 0) sq[g * C::COLUMNS + 16 * w + 8 * n + (lane >> 2)] = sumsq[n];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < C::COLUMNS) {
+        double t = 0.0;
+        for (int g = 0; g < C::GROUPS; ++g) t += sq[g * C::COLUMNS + threadIdx.x];
+        stat->sumsq[threadIdx.x] = t;
+    }
 }
 
 // Blocks 0..63 of a tile: its columns summed over the chunks in a fixed order
@@ -509,8 +620,10 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // products left out (three digit pairs a K row, digits of standard deviation
 // 74) add about sqrt(6 N) 74^2 2^(E_i + E_j - 70). Both stay below
 // 2^-54 ||a_i|| ||a_j||, under the rounding of the FP64 sums themselves, when
-//     ||a_j||^2 >= 4^E_j max(21.4, 0.21 sqrt(N)),
-// which the kernel checks per column (N Gaussian rows give about 2 N / 400).
+//     ||a_j||^2 >= 4^E_j max(21.4, 0.21 sqrt(N)).
+// The kernel knows ||a_j||^2 from the leading digits, whose rounding can raise
+// it by a third where they are small, so it checks 1.4 times that (N Gaussian
+// rows have at least about 2 N / 576).
 // A spike that dwarfs the rest of its column fails it, as do Inf and NaN, a
 // scale whose products could leave the FP64 range, and a wait that gave up:
 // the caller then computes the tile in FP64 instead.
@@ -566,7 +679,7 @@ split_sum_kernel(SplitShape sh, int64_t rows, const double* __restrict__ partial
         s = (red[tid] + red[128 + tid]) + (red[256 + tid] + red[384 + tid]);
         E = max(max(redE[tid], redE[128 + tid]), max(redE[256 + tid], redE[384 + tid]));
         if (E != SPLIT_E_UNSET &&
-            !(E >= -450 && E <= 450 && s >= fmax(21.4, 0.21 * sqrt((double)rows)) * pow2(2 * E)))
+            !(E >= -450 && E <= 450 && s >= fmax(30.0, 0.3 * sqrt((double)rows)) * pow2(2 * E)))
             mine |= SPLIT_INACCURATE;
     }
     if (mine) atomicOr(&flags, mine);

@@ -12,6 +12,7 @@ namespace fb {
 
 // A wait gives up after this long; a healthy wait takes microseconds.
 constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;
+constexpr long long WAIT_LIMIT_CYCLES = 4000000000ll;   // the same at 2 GHz
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -54,12 +55,29 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Waits for the phase with the given parity to complete; false after
-// WAIT_LIMIT_NS without it.
+// WAIT_LIMIT_CYCLES without it. The limit is counted in SM cycles: reading the
+// global timer in the polling loop goes through the same queue as the other
+// warps' shared-memory and barrier operations and holds them up for hundreds
+// of cycles each.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = globaltimer_ns();
+    const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity)) {
-        if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) return false;
+        if (clock64() - t0 > WAIT_LIMIT_CYCLES) return false;
+    }
+    return true;
+}
+
+// mbar_wait by a whole converged warp, every lane polling and the warp
+// deciding together. The branch is then uniform: lanes that left a polling
+// loop of their own at different turns would stay apart until the code joins
+// again, which where a failed wait leaves the loop is past its end, and every
+// instruction between would issue once per group of lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        if (__any_sync(0xffffffffu, clock64() - t0 > WAIT_LIMIT_CYCLES)) return false;
     }
     return true;
 }

@@ -124,10 +124,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "memory");
 }
 
-// Thread t of the warp writes two consecutive 32-bit columns of lane
-// (taddr lane + t).
-__device__ __forceinline__ void tmem_st2(uint32_t taddr, uint32_t r0, uint32_t r1) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(r0), "r"(r1) : "memory");
+// 16 lanes (from the address's lane on) x 8 consecutive 32-bit columns:
+// thread t writes lanes t / 4 (a0, a1) and t / 4 + 8 (b0, b1), columns t % 4
+// (a0, b0) and 4 + t % 4 (a1, b1).
+__device__ __forceinline__ void tmem_st_16x128b_x2(uint32_t taddr, uint32_t a0, uint32_t b0, uint32_t a1,
+                                                   uint32_t b1) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};"
+                 ::"r"(taddr), "r"(a0), "r"(b0), "r"(a1), "r"(b1) : "memory");
 }
 
 __device__ __forceinline__ void tmem_wait_st() {
