@@ -435,6 +435,10 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 if (TO_A && fresh && s > 0) {
                     if (!drain(s - 1, stage.Eold, stage.Eold + (FULL ? 64 : 0), stage.epoch > 1) || !load(s))
                         return false;
+#pragma unroll
+                    for (int n = 0; n < NC; ++n)
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) hold_loaded(v[n][e]);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&fp_empty[s % C::SLOTS]);

@@ -86,6 +86,28 @@ int encode_panel_map(CUtensorMap* map, const void* base, int64_t rows, int64_t c
     return FB_OK;
 }
 
+int encode_grid_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, int64_t nz, int64_t cols, int64_t ld,
+                    int box_x, int box_y) {
+    auto encode = tensor_map_encoder();
+    if (!encode) {
+        set_error(FB_ECUDA, "the driver does not provide cuTensorMapEncodeTiled");
+        return FB_ECUDA;
+    }
+    cuuint64_t dims[4] = {(cuuint64_t)(2 * nx), (cuuint64_t)ny, (cuuint64_t)nz, (cuuint64_t)cols};
+    cuuint64_t strides[3] = {(cuuint64_t)(nx * 16), (cuuint64_t)(nx * ny * 16), (cuuint64_t)(ld * 16)};
+    cuuint32_t box[4] = {(cuuint32_t)(2 * box_x), (cuuint32_t)box_y, 1u, 1u};
+    cuuint32_t elem[4] = {1u, 1u, 1u, 1u};
+    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(base), dims, strides, box, elem,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error(FB_ECUDA, "cuTensorMapEncodeTiled failed (%d) for %lld columns on a %lld x %lld x %lld grid, ld %lld",
+                  (int)r, (long long)cols, (long long)nx, (long long)ny, (long long)nz, (long long)ld);
+        return FB_ECUDA;
+    }
+    return FB_OK;
+}
+
 }  // namespace fb
 
 using namespace fb;

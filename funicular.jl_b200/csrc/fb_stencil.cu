@@ -9,6 +9,7 @@
 // are read from DRAM once. Two kernels: by 2.5-D tiles (the default), and a
 // thread per output entry for column counts past the grid limit.
 #include "fb_common.cuh"
+#include "fb_tma.cuh"
 
 namespace fb {
 
@@ -41,68 +42,102 @@ __global__ void __launch_bounds__(128) laplace7_kernel(z64* __restrict__ Y, int6
     }
 }
 
-// The same operator by 2.5-D tiles: a block owns a 32 x 8 tile of an x-y
-// plane of one column and marches it along a range of z. Each thread keeps
-// its point's values at z - 1, z and z + 1 in registers, with the plane at
-// z + 2 already loading (one new plane read a step, two steps ahead of its
-// use), and the x and y neighbours come from the current plane staged in
-// shared memory with a one-point halo (its edge points read from L2, where
-// the neighbouring tiles marching beside this one have brought them). Every
-// input is read from DRAM about once. The z range of a column is cut into
-// zchunks pieces, enough for the grid to fill the GPU when there are few
-// columns.
-constexpr int LT_X = 32, LT_Y = 8;
+// The same operator by 2.5-D tiles: a block owns a 32 x 16 tile of an x-y
+// plane of one column and marches it along a range of z. A producer warp keeps
+// a ring of planes in flight with TMA, each the tile with a one-point halo (a
+// 4-D box at (x0 - 1, y0 - 1, z, column); points outside the grid read as zero,
+// which is the boundary condition); a thread takes its four neighbours in the
+// plane from there and its own point of the planes below and above from
+// registers. Every input is read from DRAM about once: the halos come from L2,
+// where the neighbouring tiles marching beside this one have brought them.
+// HBM-bound, so what counts is bytes in flight: the ring holds 78 KB a block
+// and two blocks run on an SM, against one 16-byte load a thread and two block
+// barriers a plane when each thread loaded its own points. 64 columns on the
+// 215^3 grid: 3.86 ms, 5280 GB/s (5.31 ms, 3830 before); 3 columns on 342^3:
+// 0.66 ms, 5780 GB/s. Three blocks with six slots (0.74 ms, 32 registers a
+// thread) and 8-row tiles (0.70 ms, more halo) were slower. The z range of a
+// column is cut into zchunks pieces, enough for the grid to fill the GPU when
+// there are few columns.
+constexpr int LT_X = 32, LT_Y = 16, LT_SLOTS = 8;
+constexpr int LT_ROW = LT_X + 2;
+constexpr int LT_PLANE = (LT_ROW * (LT_Y + 2) * 16 + 127) / 128 * 128;   // bytes of a ring slot
+constexpr int LT_BOX_BYTES = LT_ROW * (LT_Y + 2) * 16;
+constexpr int LT_WARPS = LT_X * LT_Y / 32;
+constexpr size_t LT_SMEM = (size_t)LT_SLOTS * LT_PLANE + 2 * LT_SLOTS * sizeof(uint64_t) + 128;
 
-__global__ void __launch_bounds__(LT_X * LT_Y)
-laplace7_tiled_kernel(z64* __restrict__ Y, int64_t ldy, const z64* __restrict__ X, int64_t ldx, int nx, int ny,
-                      int nz, z64 shift, int zchunks) {
-    __shared__ z64 tile[LT_Y + 2][LT_X + 2];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int gx = blockIdx.x * LT_X + tx, gy = blockIdx.y * LT_Y + ty;
+__global__ void __launch_bounds__(LT_X * LT_Y + 32, 2)
+laplace7_tiled_kernel(const __grid_constant__ CUtensorMap tm, z64* __restrict__ Y, int64_t ldy, int nx, int ny, int nz,
+                      z64 shift, int zchunks) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)LT_SLOTS * LT_PLANE);
+    uint64_t* empty = full + LT_SLOTS;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), tx = threadIdx.x & 31;
     const int c = blockIdx.z / zchunks, zc = blockIdx.z - c * zchunks;
     const int z0 = (int)((int64_t)nz * zc / zchunks), z1 = (int)((int64_t)nz * (zc + 1) / zchunks);
-    const z64* x = X + (int64_t)c * ldx;
-    z64* y = Y + (int64_t)c * ldy;
-    const int64_t plane = (int64_t)nx * ny;
-    const bool inside = gx < nx && gy < ny;
-    const int64_t col_off = (int64_t)gy * nx + gx;
-    const double dr = 6.0 + shift.x, di = shift.y;
-    const z64 zero = zmake(0.0, 0.0);
-    auto at = [&](int xx, int yy, int zz) -> z64 {
-        return (xx >= 0 && xx < nx && yy >= 0 && yy < ny && zz >= 0 && zz < nz)
-                   ? x[(int64_t)zz * plane + (int64_t)yy * nx + xx] : zero;
-    };
-    auto plane_at = [&](int zz) -> z64 { return (inside && zz >= 0 && zz < nz) ? x[(int64_t)zz * plane + col_off] : zero; };
-    z64 below = plane_at(z0 - 1);
-    z64 cur = plane_at(z0);
-    z64 above = plane_at(z0 + 1);
-    z64 ahead = plane_at(z0 + 2);
-    // Halo: the columns x0 - 1 and x0 + 32 (lanes 0..7 of the first two
-    // warps) and the rows y0 - 1 and y0 + 8 (the next two warps); each such
-    // thread loads its halo point one plane ahead.
-    int hx = -2, hy = -2, hr = 0, hc = 0;
-    if (ty == 0 && tx < LT_Y) { hx = blockIdx.x * LT_X - 1; hy = blockIdx.y * LT_Y + tx; hr = tx + 1; hc = 0; }
-    if (ty == 1 && tx < LT_Y) { hx = blockIdx.x * LT_X + LT_X; hy = blockIdx.y * LT_Y + tx; hr = tx + 1; hc = LT_X + 1; }
-    if (ty == 2) { hx = gx; hy = blockIdx.y * LT_Y - 1; hr = 0; hc = tx + 1; }
-    if (ty == 3) { hx = gx; hy = blockIdx.y * LT_Y + LT_Y; hr = LT_Y + 1; hc = tx + 1; }
-    const bool halo = hx != -2;
-    z64 hval = halo ? at(hx, hy, z0) : zero;
-    for (int z = z0; z < z1; ++z) {
-        tile[ty + 1][tx + 1] = cur;
-        if (halo) tile[hr][hc] = hval;
-        __syncthreads();
-        if (inside) {
-            const z64 a = tile[ty + 1][tx], b = tile[ty + 1][tx + 2], d = tile[ty][tx + 1], e = tile[ty + 2][tx + 1];
-            const double sx = a.x + b.x + d.x + e.x + below.x + above.x;
-            const double sy = a.y + b.y + d.y + e.y + below.y + above.y;
-            y[(int64_t)z * plane + col_off] = zmake(dr * cur.x - di * cur.y - sx, dr * cur.y + di * cur.x - sy);
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < LT_SLOTS; ++b) {
+            mbar_init(&full[b], 1);
+            mbar_init(&empty[b], LT_WARPS);
         }
-        __syncthreads();
+        mbar_fence_init();
+    }
+    __syncthreads();
+    // Planes z0 - 1 .. z1, plane z0 - 1 + i in slot i % LT_SLOTS.
+    const int planes = z1 - z0 + 2;
+    if (warp == LT_WARPS) {
+        if (tx == 0) {
+            tma_prefetch_map(&tm);
+            int b = 0, issued = 0;
+            uint32_t ph = 0;
+            for (int i = 0; i < planes; ++i) {
+                if (i >= LT_SLOTS && !mbar_wait(&empty[b], ph ^ 1u)) break;
+                mbar_arrive_expect_tx(&full[b], LT_BOX_BYTES);
+                tma_load_4d(smem + (size_t)b * LT_PLANE, &tm, 2 * ((int)blockIdx.x * LT_X - 1),
+                            (int)blockIdx.y * LT_Y - 1, z0 - 1 + i, c, &full[b]);
+                if (++b == LT_SLOTS) { b = 0; ph ^= 1u; }
+                issued = i + 1;
+            }
+            // The block's shared memory must not go away under a copy that
+            // the other warps gave up on.
+            for (int i = issued > LT_SLOTS ? issued - LT_SLOTS : 0; i < issued; ++i)
+                mbar_wait(&full[i % LT_SLOTS], (i / LT_SLOTS) & 1);
+        }
+        return;
+    }
+    const int gx = blockIdx.x * LT_X + tx, gy = blockIdx.y * LT_Y + warp;
+    const bool inside = gx < nx && gy < ny;
+    const int64_t plane = (int64_t)nx * ny;
+    z64* y = Y + (int64_t)c * ldy + (int64_t)z0 * plane + (int64_t)gy * nx + gx;
+    const double dr = 6.0 + shift.x, di = shift.y;
+    const unsigned char* mine = smem + (((warp + 1) * LT_ROW + tx + 1) << 4);
+    auto point = [&](int b, int off) { return *reinterpret_cast<const z64*>(mine + b * LT_PLANE + (off << 4)); };
+    z64 below, cur;
+    bool ok = mbar_wait_warp(&full[0], 0) && mbar_wait_warp(&full[1], 0);
+    below = point(0, 0);
+    cur = point(1, 0);
+    hold_loaded(below.x);
+    __syncwarp();
+    if (tx == 0) mbar_arrive(&empty[0]);
+    int b = 1, nb = 2;
+    uint32_t ph = 0;
+    for (int z = z0; z < z1; ++z) {
+        ok = ok && mbar_wait_warp(&full[nb], ph);
+        const z64 above = point(nb, 0);
+        const z64 l = point(b, -1), r = point(b, 1), d = point(b, -LT_ROW), u = point(b, LT_ROW);
+        double sx = l.x + r.x + d.x + u.x + below.x + above.x;
+        double sy = l.y + r.y + d.y + u.y + below.y + above.y;
+        hold_loaded(sx);
+        hold_loaded(sy);
+        __syncwarp();
+        if (tx == 0) mbar_arrive(&empty[b]);
+        if (!ok) sx = __longlong_as_double(0x7ff8000000000000ll);   // a plane never came: no silent wrong answer
+        if (inside) *y = zmake(dr * cur.x - di * cur.y - sx, dr * cur.y + di * cur.x - sy);
+        y += plane;
         below = cur;
         cur = above;
-        above = ahead;
-        ahead = plane_at(z + 3);
-        if (halo) hval = at(hx, hy, z + 1);
+        b = nb;
+        if (++nb == LT_SLOTS) { nb = 0; ph ^= 1u; }
     }
 }
 
@@ -138,16 +173,20 @@ int fb_zlaplace7_apply(fb_z128* Y, int64_t ldy, const fb_z128* X, int64_t ldx, i
     }
     if ((int64_t)ny * nz > INT32_MAX) { set_error(FB_ENOTSUP, "fb_zlaplace7_apply: ny * nz must fit in 32 bits"); return FB_ENOTSUP; }
     const int64_t tiles = (int64_t)((nx + LT_X - 1) / LT_X) * ((ny + LT_Y - 1) / LT_Y);
-    // z pieces: enough blocks for eight a SM, each piece at least 16 planes.
-    int64_t zchunks = ((int64_t)sm_count() * 8 + tiles * cols - 1) / (tiles * cols);
+    // z pieces: enough blocks for three rounds of two a SM, each piece at
+    // least 16 planes (a piece reads two planes more than it writes).
+    int64_t zchunks = ((int64_t)sm_count() * 6 + tiles * cols - 1) / (tiles * cols);
     if (zchunks > nz / 16) zchunks = nz / 16;
     if (zchunks < 1) zchunks = 1;
-    if (cols * zchunks <= 65535 && (ny + LT_Y - 1) / LT_Y <= 65535) {
+    if (cols * zchunks <= 65535 && (ny + LT_Y - 1) / LT_Y <= 65535 && nx < (1 << 30)) {
+        CUtensorMap tm;
+        FB_TRY(encode_grid_map(&tm, X, nx, ny, nz, cols, ldx, LT_ROW, LT_Y + 2));
+        FB_CUDA(cudaFuncSetAttribute(laplace7_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LT_SMEM),
+                "cudaFuncSetAttribute(laplace7_tiled_kernel)");
         const dim3 grid((unsigned)((nx + LT_X - 1) / LT_X), (unsigned)((ny + LT_Y - 1) / LT_Y),
                         (unsigned)(cols * zchunks));
-        laplace7_tiled_kernel<<<grid, dim3(LT_X, LT_Y), 0, stream_of(queue)>>>(
-            reinterpret_cast<z64*>(Y), ldy, reinterpret_cast<const z64*>(X), ldx, nx, ny, nz, zmake(shift.re, shift.im),
-            (int)zchunks);
+        laplace7_tiled_kernel<<<grid, LT_X * LT_Y + 32, LT_SMEM, stream_of(queue)>>>(
+            tm, reinterpret_cast<z64*>(Y), ldy, nx, ny, nz, zmake(shift.re, shift.im), (int)zchunks);
         FB_LAUNCHED("laplace7_tiled_kernel");
         return FB_OK;
     }

@@ -68,6 +68,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return true;
 }
 
+// A value that comes from shared memory is in its register before anything
+// after this point in program order runs. A warp that gives a buffer back with
+// mbar_arrive needs it: the arrival and a load still on its way take different
+// paths, and a copy into the buffer could otherwise overtake the load.
+__device__ __forceinline__ void hold_loaded(double& v) { asm volatile("" : "+d"(v)::"memory"); }
+
 // mbar_wait by a whole converged warp, every lane polling and the warp
 // deciding together. The branch is then uniform: lanes that left a polling
 // loop of their own at different turns would stay apart until the code joins
@@ -91,6 +97,14 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
+// The same from a 4-D map.
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar))
+        : "memory");
+}
+
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -108,5 +122,12 @@ __device__ __forceinline__ void dmma_884(double& d0, double& d1, double a, doubl
 // (128 bytes, the 128-byte swizzle span) by box_cols columns; rows and
 // columns past the matrix read as zero.
 int encode_panel_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_cols);
+
+// Host: a 4-D tensor map over `cols` columns of ComplexF64 grid functions on
+// nx x ny x nz points (column c at base + c ld, x fastest), seen as FP64
+// pairs. A box is box_x by box_y points of one plane; points outside the grid
+// read as zero.
+int encode_grid_map(CUtensorMap* map, const void* base, int64_t nx, int64_t ny, int64_t nz, int64_t cols, int64_t ld,
+                    int box_x, int box_y);
 
 }  // namespace fb
