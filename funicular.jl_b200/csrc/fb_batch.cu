@@ -463,10 +463,10 @@ __device__ void factor_step(const PbInst& I, int pass, unsigned char* smem, doub
         }
         __syncthreads();
         auto g = [&](int i, int j) { return Gs[i * kp + j]; };
-        const double gnorm = hermitian_fro(g, k, red);
+        auto at = [&](int i, int j) -> z64& { return W[i * k + j]; };
         bool shifted = false;
-        double shift = 0.0;
-        const bool ok = factor_shifted(g, k, I.N, gnorm, 0.0, W, shifted, shift);
+        double shift = 0.0, gnorm = 0.0;
+        const bool ok = factor_shifted(g, k, I.N, 0.0, at, red, gnorm, shifted, shift);
         if (tid == 0) {
             st->shifted[pass] = shifted ? 1 : 0;
             st->shift[pass] = shift;

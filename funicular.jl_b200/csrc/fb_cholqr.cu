@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "fb_common.cuh"
+#include "fb_solve.cuh"
 
 namespace fb {
 
@@ -31,20 +32,35 @@ int gram_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, 
 int gram_reduce_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
                         int kB, bool hermitian, z64 alpha, z64 beta, void* workspace, cudaStream_t stream,
                         const ChainStatus* st, int gate);
-int trsm_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
-                 size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st, int gate);
+int trsm_prepare_enqueue(int k, const z64* R, int64_t ldr, void* workspace, size_t workspace_bytes,
+                         cudaStream_t stream, const ChainStatus* st, int gate);
+int trsm_solve_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
+                       cudaStream_t stream, const ChainStatus* st, int gate);
 size_t trsm_workspace_bytes(int k);
 size_t potrf_gwork_bytes(int k);
 size_t ozaki_gram_workspace_size(int64_t rows);
 int ozaki_gram_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, int64_t rows, int k, z64 alpha, z64 beta,
                        void* workspace, size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st,
                        int gate);
-int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t ldu,
-                  const z64* Rin, int64_t ldrin, z64* Rout, int64_t ldrout, z64* gwork,
-                  ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u);
+int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t ldu, z64* gwork,
+                  ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u, TrsmPlan* plan,
+                  double* frag);
+int compose_r_enqueue(z64* R, int64_t ldr, int k, const z64* U1, int64_t ldu1, const z64* U2, int64_t ldu2,
+                      const z64* U3, int64_t ldu3, const ChainStatus* st, cudaStream_t stream);
+
+// One pass's factor and everything its solves need in trsm_ws: up to 64
+// columns the Cholesky's own launch leaves the solve plan there.
+static int factor_enqueue(const z64* G, int k, int64_t N, z64* U, z64* gwork, void* trsm_ws, size_t trsm_bytes,
+                          ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u) {
+    const bool one = k <= TR_KMAX;
+    FB_TRY(potrf_enqueue(G, k, k, N, U, k, gwork, st, pass, gate, stream, forced_u,
+                         one ? static_cast<TrsmPlan*>(trsm_ws) : nullptr,
+                         one ? reinterpret_cast<double*>(static_cast<char*>(trsm_ws) + TR_PLAN_BYTES) : nullptr));
+    return one ? FB_OK : trsm_prepare_enqueue(k, U, k, trsm_ws, trsm_bytes, stream, st, gate);
+}
 
 struct CholqrLayout {
-    size_t status, G, U, Ra, Rb, gwork, trsm, gram, total;
+    size_t status, G, U[3], gwork, trsm, gram, total;
 };
 
 static CholqrLayout cholqr_layout(int64_t N, int k) {
@@ -54,9 +70,7 @@ static CholqrLayout cholqr_layout(int64_t N, int k) {
     const size_t kk = (size_t)k * k * sizeof(z64);
     L.status = take(sizeof(ChainStatus));
     L.G = take(kk);
-    L.U = take(kk);
-    L.Ra = take(kk);
-    L.Rb = take(kk);
+    for (int p = 0; p < 3; ++p) L.U[p] = take(kk);
     L.gwork = take(potrf_gwork_bytes(k));
     L.trsm = take(trsm_workspace_bytes(k));
     // One workspace serves both forms: the Gram scratch is the larger of the
@@ -66,19 +80,6 @@ static CholqrLayout cholqr_layout(int64_t N, int k) {
     L.gram = take(g64 > gtc ? g64 : gtc);
     L.total = off;
     return L;
-}
-
-// Copies R of the last pass that ran into the caller's R.
-__global__ void select_r_kernel(z64* __restrict__ R, int64_t ldr, const z64* __restrict__ Ra,
-                                const z64* __restrict__ Rb, int k, const ChainStatus* st) {
-    if (st->failed) return;
-    const bool third = (st->shifted[1] | st->shifted[2]) != 0;
-    const z64* src = third ? Ra : Rb;
-    const int64_t kk = (int64_t)k * k;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < kk; e += (int64_t)gridDim.x * blockDim.x) {
-        int j = (int)(e / k), i = (int)(e - (int64_t)j * k);
-        R[i + (int64_t)j * ldr] = src[e];
-    }
 }
 
 }  // namespace fb
@@ -117,9 +118,8 @@ static int cholqr2_chain(fb_z128* Y, int64_t ldy, int64_t N, int k, fb_z128* R, 
     char* ws = static_cast<char*>(workspace);
     ChainStatus* st = status ? status : reinterpret_cast<ChainStatus*>(ws + L.status);
     z64* G = reinterpret_cast<z64*>(ws + L.G);
-    z64* U = reinterpret_cast<z64*>(ws + L.U);
-    z64* Ra = reinterpret_cast<z64*>(ws + L.Ra);
-    z64* Rb = reinterpret_cast<z64*>(ws + L.Rb);
+    z64* U[3];
+    for (int p = 0; p < 3; ++p) U[p] = reinterpret_cast<z64*>(ws + L.U[p]);
     z64* gwork = reinterpret_cast<z64*>(ws + L.gwork);
     void* gram_ws = ws + L.gram;
     void* trsm_ws = ws + L.trsm;
@@ -130,9 +130,6 @@ static int cholqr2_chain(fb_z128* Y, int64_t ldy, int64_t N, int k, fb_z128* R, 
     const z64 one = zmake(1.0, 0.0), zero = zmake(0.0, 0.0);
 
     FB_CUDA(cudaMemsetAsync(st, 0, sizeof(ChainStatus), stream), "cudaMemsetAsync");
-    // R accumulates as Ra = R1, Rb = R2 R1, Ra = R3 R2 R1.
-    const z64* rin[4] = {nullptr, nullptr, Ra, Rb};
-    z64* rout[4] = {nullptr, Ra, Rb, Ra};
     for (int pass = 1; pass <= 3; ++pass) {
         const int gate = pass == 3 ? GATE_THIRD : GATE_HEALTHY;
         if (tensor)
@@ -142,13 +139,11 @@ static int cholqr2_chain(fb_z128* Y, int64_t ldy, int64_t N, int k, fb_z128* R, 
                                 gate));
         // The shifted CholeskyQR3 shifts pass 1 unconditionally; that marks
         // the pass as shifted, so the third pass runs and R = R3 R2 R1.
-        FB_TRY(potrf_enqueue(G, k, k, N, U, k, rin[pass], k, rout[pass], k, gwork, st, pass, gate, stream,
-                             pass == 1 ? forced_u : 0.0));
-        FB_TRY(trsm_enqueue(Yz, ldy, N, k, U, k, trsm_ws, trsm_bytes, stream, st, gate));
+        FB_TRY(factor_enqueue(G, k, N, U[pass - 1], gwork, trsm_ws, trsm_bytes, st, pass, gate, stream,
+                              pass == 1 ? forced_u : 0.0));
+        FB_TRY(trsm_solve_enqueue(Yz, ldy, N, k, U[pass - 1], k, trsm_ws, stream, st, gate));
     }
-    int blocks = (int)((int64_t)k * k + 255) / 256;
-    select_r_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<z64*>(R), ldr, Ra, Rb, k, st);
-    FB_LAUNCHED("select_r_kernel");
+    FB_TRY(compose_r_enqueue(reinterpret_cast<z64*>(R), ldr, k, U[0], k, U[1], k, U[2], k, st, stream));
 
     if (info) {
         FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
@@ -510,9 +505,8 @@ int fb_zcholqr2_staged(void* const* host_panels, int host_type, const int64_t* h
     char* ws = static_cast<char*>(workspace);
     ChainStatus* st = reinterpret_cast<ChainStatus*>(ws + L.status);
     z64* G = reinterpret_cast<z64*>(ws + L.G);
-    z64* U = reinterpret_cast<z64*>(ws + L.U);
-    z64* Ra = reinterpret_cast<z64*>(ws + L.Ra);
-    z64* Rb = reinterpret_cast<z64*>(ws + L.Rb);
+    z64* U[3];
+    for (int p = 0; p < 3; ++p) U[p] = reinterpret_cast<z64*>(ws + L.U[p]);
     z64* gwork = reinterpret_cast<z64*>(ws + L.gwork);
     void* gram_ws = ws + L.gram;
     void* trsm_ws = ws + L.trsm;
@@ -583,12 +577,12 @@ int fb_zcholqr2_staged(void* const* host_panels, int host_type, const int64_t* h
                                      B.c0[b], B.c0[b + 1]));
     }
     FB_TRY(gram_reduce_enqueue(G, k, Yz, ldy, Yz, ldy, N, k, k, true, one, zero, gram_ws, stream, st, GATE_HEALTHY));
-    FB_TRY(potrf_enqueue(G, k, k, N, U, k, nullptr, k, Ra, k, gwork, st, 1, GATE_HEALTHY, stream,
-                         shift_unit_roundoff));
-    FB_TRY(trsm_enqueue(Yz, ldy, N, k, U, k, trsm_ws, trsm_bytes, stream, st, GATE_HEALTHY));
+    FB_TRY(factor_enqueue(G, k, N, U[0], gwork, trsm_ws, trsm_bytes, st, 1, GATE_HEALTHY, stream,
+                          shift_unit_roundoff));
+    FB_TRY(trsm_solve_enqueue(Yz, ldy, N, k, U[0], k, trsm_ws, stream, st, GATE_HEALTHY));
     FB_TRY(gram_enqueue(G, k, Yz, ldy, Yz, ldy, N, k, k, one, zero, true, gram_ws, gram_bytes, stream, st,
                         GATE_HEALTHY));
-    FB_TRY(potrf_enqueue(G, k, k, N, U, k, Ra, k, Rb, k, gwork, st, 2, GATE_HEALTHY, stream, 0.0));
+    FB_TRY(factor_enqueue(G, k, N, U[1], gwork, trsm_ws, trsm_bytes, st, 2, GATE_HEALTHY, stream, 0.0));
     // Whether a third pass runs (or the chain stopped) decides which solve is
     // the last: read the status once here.
     ChainStatus hs;
@@ -596,10 +590,10 @@ int fb_zcholqr2_staged(void* const* host_panels, int host_type, const int64_t* h
     FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     const bool third = !hs.failed && (hs.shifted[1] | hs.shifted[2]);
     if (third) {
-        FB_TRY(trsm_enqueue(Yz, ldy, N, k, U, k, trsm_ws, trsm_bytes, stream, st, GATE_HEALTHY));
+        FB_TRY(trsm_solve_enqueue(Yz, ldy, N, k, U[1], k, trsm_ws, stream, st, GATE_HEALTHY));
         FB_TRY(gram_enqueue(G, k, Yz, ldy, Yz, ldy, N, k, k, one, zero, true, gram_ws, gram_bytes, stream, st,
                             GATE_HEALTHY));
-        FB_TRY(potrf_enqueue(G, k, k, N, U, k, Rb, k, Ra, k, gwork, st, 3, GATE_HEALTHY, stream, 0.0));
+        FB_TRY(factor_enqueue(G, k, N, U[2], gwork, trsm_ws, trsm_bytes, st, 3, GATE_HEALTHY, stream, 0.0));
         FB_CUDA(cudaMemcpyAsync(&hs, st, sizeof(ChainStatus), cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync");
         FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     }
@@ -611,7 +605,7 @@ int fb_zcholqr2_staged(void* const* host_panels, int host_type, const int64_t* h
         for (int b = 0; b < nb; ++b) {
             int64_t r0, r1;
             B.rows(b, N, &r0, &r1);
-            FB_TRY(trsm_enqueue(Yz + r0, ldy, r1 - r0, k, U, k, trsm_ws, trsm_bytes, stream, st, GATE_HEALTHY));
+            FB_TRY(trsm_solve_enqueue(Yz + r0, ldy, r1 - r0, k, U[third ? 2 : 1], k, trsm_ws, stream, st, GATE_HEALTHY));
             if (narrow) {
                 if (b >= 2) FB_CUDA(cudaStreamWaitEvent(stream, sent[b - 2], 0), "cudaStreamWaitEvent");
                 FB_TRY(fb_convert_copy(stage[b & 1], FB_C64, sld, Yz + r0, FB_C128, ldy, r1 - r0, k, queue));
@@ -626,9 +620,7 @@ int fb_zcholqr2_staged(void* const* host_panels, int host_type, const int64_t* h
         }
         FB_CUDA(cudaStreamWaitEvent(stream, sent[nb - 1], 0), "cudaStreamWaitEvent");
     }
-    int blocks = (int)((int64_t)k * k + 255) / 256;
-    select_r_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<z64*>(R), ldr, Ra, Rb, k, st);
-    FB_LAUNCHED("select_r_kernel");
+    FB_TRY(compose_r_enqueue(reinterpret_cast<z64*>(R), ldr, k, U[0], k, U[1], k, U[2], k, st, stream));
     FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     int inf = 0;
     const int status = fb_zcholqr2_query(st, &inf, passes, nullptr);

@@ -12,6 +12,7 @@ namespace fb {
 constexpr int SPLIT_STAGE_ROWS = 16;              // complex rows per stage; chunks are whole stages
 constexpr int SPLIT_TILE_DOUBLES = 128 * 64;      // a partial or summed tile, column n of it contiguous
 constexpr int SPLIT_E_UNSET = -4000;              // scale of a column that has only zeros so far
+constexpr int SPLIT_E_TINY = -3999;               // and of one that has nothing above the subnormals
 constexpr int SPLIT_INVALID = 1;                  // Inf, NaN or a wait that gave up: the sums mean nothing
 constexpr int SPLIT_INACCURATE = 2;               // the slices may leave out more than FP64 rounding would
 
@@ -24,12 +25,10 @@ struct SplitShape {
 };
 
 // What a CTA reports about its chunk: per input column (A's 64, then B's) the
-// last scale exponent, the sum of squares, and whether only subnormal entries
-// were seen.
+// last scale exponent and the sum of squares.
 struct SplitStat {
     double sumsq[128];
     int E[128];
-    int tiny[128];
     int invalid;
     int pad[3];
 };

@@ -585,8 +585,7 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (bad) *bad_flag = 1;
 #pragma unroll
         for (int x = 0; x < NC; ++x) {
-            stat->E[32 * x + lane] = E[x];
-            stat->tiny[32 * x + lane] = E[x] == SPLIT_E_UNSET && tiny[x] ? 1 : 0;
+            stat->E[32 * x + lane] = E[x] == SPLIT_E_UNSET && tiny[x] ? SPLIT_E_TINY : E[x];
         }
     }
     umma::fence_before_sync();
@@ -614,9 +613,12 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
 }
 
-// Blocks 0..63 of a tile: its columns summed over the chunks in a fixed order
-// (four interleaved runs of chunks, then the four), a folded tile's two halves
-// added. Block 64: the tile's verdict.
+// Blocks 0..127 of a tile: half a column each (a folded tile: a column, its
+// two halves added) summed over the chunks in a fixed order, eight interleaved
+// runs of chunks, then the eight. Block 128: the tile's verdict. The partial
+// tiles are in L2, so the loads' latency is what counts: ten are in flight a
+// thread (21 us at 148 chunks with the loads of the sums and of the verdict waiting
+// for one another, 7 to 10 now).
 //
 // The verdict compares what the slices leave out with what the column weighs.
 // With scale 2^E an entry is off by at most 2^(E - 51) (V: 2^(E - 50)), which
@@ -641,41 +643,60 @@ split_sum_kernel(SplitShape sh, int64_t rows, const double* __restrict__ partial
     __shared__ int redE[SUM_THREADS];
     __shared__ int flags;
     const int tile = blockIdx.y, tid = threadIdx.x;
-    const int m = tid & 127, part = tid >> 7;
     const bool full = !sh.hermitian || tile >= sh.nt_a;
-    if (blockIdx.x < 64) {
-        const double* p = partial + (size_t)tile * sh.nchunks * SPLIT_TILE_DOUBLES + blockIdx.x * 128 + m;
+    if (blockIdx.x < 128) {
+        if (!full && blockIdx.x >= 64) return;
+        const int n = full ? blockIdx.x >> 1 : blockIdx.x, half = full ? blockIdx.x & 1 : 0;
+        const int m = tid & 63, run = tid >> 6;
+        const double* p = partial + (size_t)tile * sh.nchunks * SPLIT_TILE_DOUBLES + n * 128 + half * 64 + m;
         double s = 0.0;
-#pragma unroll 8
-        for (int c = part; c < sh.nchunks; c += 4) s += p[(size_t)c * SPLIT_TILE_DOUBLES];
+        for (int c0 = run; c0 < sh.nchunks; c0 += 80) {
+            double v[10], w[10];
+#pragma unroll
+            for (int q = 0; q < 10; ++q) {
+                const double* c = p + (size_t)min(c0 + 8 * q, sh.nchunks - 1) * SPLIT_TILE_DOUBLES;
+                v[q] = c[0];
+                w[q] = c[full ? 0 : 64];
+            }
+#pragma unroll
+            for (int q = 0; q < 10; ++q)
+                if (c0 + 8 * q < sh.nchunks) s += full ? v[q] : v[q] + w[q];
+        }
         red[tid] = s;
         __syncthreads();
-        if (tid >= 128) return;
-        s = (red[tid] + red[128 + tid]) + (red[256 + tid] + red[384 + tid]);
-        if (!full) {
-            __syncthreads();
-            red[tid] = s;
-            __syncthreads();
-            if (tid >= 64) return;
-            s += red[64 + tid];
-        }
-        sums[(size_t)tile * SPLIT_TILE_DOUBLES + blockIdx.x * 128 + m] = s;
+        if (tid >= 64) return;
+        s = 0.0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) s += red[64 * r + tid];
+        sums[(size_t)tile * SPLIT_TILE_DOUBLES + n * 128 + half * 64 + m] = s;
         return;
     }
+    const int m = tid & 127, part = tid >> 7;
     if (tid == 0) flags = 0;
     __syncthreads();
     const int columns = full ? 128 : 64;
     int E = SPLIT_E_UNSET, mine = 0;
     double s = 0.0;
-    for (int c = part; c < sh.nchunks; c += 4) {
-        const SplitStat& x = stats[(size_t)tile * sh.nchunks + c];
-        if (m == 0 && x.invalid) mine |= SPLIT_INVALID;
-        if (m < columns) {
-            E = max(E, x.E[m]);
-            s += x.sumsq[m];
-            if (x.tiny[m]) mine |= SPLIT_INACCURATE;
+    const SplitStat* x = stats + (size_t)tile * sh.nchunks;
+    for (int c = tid; c < sh.nchunks; c += SUM_THREADS)
+        if (x[c].invalid) mine |= SPLIT_INVALID;
+    if (m < columns)
+        for (int c0 = part; c0 < sh.nchunks; c0 += 40) {
+            double v[10];
+            int e[10];
+#pragma unroll
+            for (int q = 0; q < 10; ++q) {
+                const int c = min(c0 + 4 * q, sh.nchunks - 1);   // the last one again past the end
+                v[q] = x[c].sumsq[m];
+                e[q] = x[c].E[m];
+            }
+#pragma unroll
+            for (int q = 0; q < 10; ++q) {
+                s += c0 + 4 * q < sh.nchunks ? v[q] : 0.0;
+                if (e[q] == SPLIT_E_TINY) mine |= SPLIT_INACCURATE;
+                E = max(E, e[q] == SPLIT_E_TINY ? SPLIT_E_UNSET : e[q]);
+            }
         }
-    }
     red[tid] = s;
     redE[tid] = E;
     __syncthreads();
@@ -758,7 +779,7 @@ int split_sum_enqueue(int64_t rows, const SplitShape& sh, void* workspace, cudaS
                       int gate) {
     const SplitLayout L = split_layout(sh);
     char* ws = static_cast<char*>(workspace);
-    split::split_sum_kernel<<<dim3(65, (unsigned)sh.ntiles), split::SUM_THREADS, 0, stream>>>(
+    split::split_sum_kernel<<<dim3(129, (unsigned)sh.ntiles), split::SUM_THREADS, 0, stream>>>(
         sh, rows, reinterpret_cast<const double*>(ws + L.partial), reinterpret_cast<const SplitStat*>(ws + L.stats),
         reinterpret_cast<double*>(ws + L.sums), reinterpret_cast<int*>(ws + L.verdict), st, gate);
     FB_LAUNCHED("split_sum_kernel");

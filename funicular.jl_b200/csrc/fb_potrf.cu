@@ -2,12 +2,14 @@
 // k x k Cholesky of a Hermitian Gram matrix, the shifted retry, and the
 // R2 * R product of cholqr2! (src/panelblas.jl:133,136), all FP64.
 //
-// The factorization is right-looking on the upper triangle, held in shared
-// memory when it fits (k <= 112) and in workspace memory otherwise. Pivot
-// test as LAPACK's zpotrf makes it: the factorization fails as soon as a
-// pivot is not > 0 (this also catches NaN). On failure the matrix is reloaded
-// with s = 11 N k eps(Float64) ||G||_F added to the diagonal and factored
-// again; a second failure is reported, not shifted further.
+// The factor is held in shared memory: for k <= 64 in the solve plan's layout,
+// so that the orthonormalization chain gets the plan of its next triangular
+// solve from the same launch; as a packed upper triangle up to k = 160; in
+// workspace memory beyond. Pivot test as LAPACK's zpotrf makes it: the
+// factorization fails as soon as a pivot is not > 0 (this also catches NaN).
+// On failure the matrix is reloaded with s = 11 N k eps(Float64) ||G||_F added
+// to the diagonal and factored again; a second failure is reported, not
+// shifted further.
 //
 // The shifted CholeskyQR3 of Fukaya, Kannan, Nakatsukasa, Zhang and Yamamoto
 // (SIAM J. Sci. Comput. 2020) shifts its first pass unconditionally: with a
@@ -19,25 +21,32 @@
 namespace fb {
 
 constexpr int POTRF_THREADS = 512;
-constexpr int POTRF_SMEM_MAX_K = 112;
+constexpr int POTRF_PACKED_MAX_K = 160;
 
+// Where the factor lives while it is made.
+enum FactorStore { STORE_PLAN, STORE_PACKED, STORE_GLOBAL };
+
+template <FactorStore S>
 __global__ void __launch_bounds__(POTRF_THREADS, 1)
 potrf_kernel(const z64* __restrict__ G, int64_t ldg, int k, int64_t N,
-             z64* __restrict__ U, int64_t ldu, const z64* __restrict__ Rin, int64_t ldrin,
-             z64* __restrict__ Rout, int64_t ldrout, z64* __restrict__ gwork,
-             ChainStatus* st, int pass, int gate, double forced_u) {
+             z64* __restrict__ U, int64_t ldu, z64* __restrict__ gwork,
+             ChainStatus* st, int pass, int gate, double forced_u, TrsmPlan* plan, double* __restrict__ frag) {
     if (gated_off(st, gate)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red_scratch[33];
-    const bool in_smem = k <= POTRF_SMEM_MAX_K;
-    z64* W = in_smem ? reinterpret_cast<z64*>(smem_raw) : gwork;  // row-major k x k, upper part used
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int kk = k * k;
+    constexpr int LD = TR_PREP_LD;
+    z64* W = S == STORE_GLOBAL ? gwork : reinterpret_cast<z64*>(smem_raw);
+    const int tid = threadIdx.x;
+    const int warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+    auto at = [&](int i, int j) -> z64& {
+        if (S == STORE_PLAN) return W[i * LD + j];
+        if (S == STORE_PACKED) return W[i * k - i * (i + 1) / 2 + j];
+        return W[(int64_t)i * k + j];
+    };
     auto g = [&](int i, int j) { return G[i + (int64_t)j * ldg]; };
-    const double gnorm = hermitian_fro(g, k, red_scratch);
+    double gnorm = 0.0, shift = 0.0;
     bool shifted = false;
-    double shift = 0.0;
-    const bool ok = factor_shifted(g, k, N, gnorm, forced_u, W, shifted, shift);
+    const bool ok = factor_shifted(g, k, N, forced_u, at, red_scratch, gnorm, shifted, shift);
 
     if (tid == 0 && st) {
         st->shifted[pass] = shifted ? 1 : 0;
@@ -47,38 +56,112 @@ potrf_kernel(const z64* __restrict__ G, int64_t ldg, int k, int64_t N,
     }
     if (!ok) return;
 
-    for (int e = tid; e < kk; e += nt) {
-        int j = e / k, i = e - j * k;  // column-major walk of U: coalesced stores
-        U[i + (int64_t)j * ldu] = (i <= j) ? W[i * k + j] : zmake(0.0, 0.0);
-    }
-    if (Rout) {
-        for (int e = tid; e < kk; e += nt) {
-            int j = e / k, i = e - j * k;
-            z64 acc = zmake(0.0, 0.0);
-            if (i <= j) {
-                if (Rin) {
-                    for (int m = i; m <= j; ++m) zmac(acc, W[i * k + m], Rin[m + (int64_t)j * ldrin]);
-                } else {
-                    acc = W[i * k + j];
-                }
+    for (int j = warp; j < k; j += nwarps)
+        for (int i = lane; i < k; i += 32) U[i + (int64_t)j * ldu] = (i <= j) ? at(i, j) : zmake(0.0, 0.0);
+    if (S == STORE_PLAN && plan) {
+        __syncthreads();
+        z64* Xs = W + TR_KMAX * LD;
+        const int KP = (k + TR_NB - 1) / TR_NB * TR_NB;
+        for (int i = warp; i < KP; i += nwarps)
+            for (int j = lane; j < KP; j += 32) {
+                if (j >= k || i >= k || i > j) W[i * LD + j] = zmake(i == j ? 1.0 : 0.0, 0.0);
+                Xs[i * LD + j] = zmake(0.0, 0.0);
             }
-            Rout[i + (int64_t)j * ldrout] = acc;
+        __syncthreads();
+        solve_plan(W, Xs, k, plan, frag);
+    }
+}
+
+// R = U3 U2 U1 column by column: the product of the passes' factors, run once
+// after the last pass instead of inside each pass's one-CTA factor step. A
+// block per column; 32 rows a warp and, where that leaves warps, the sum over
+// the columns of U cut into `parts` interleaved runs, added in order. U3
+// counts only if a third pass ran, U1 may be NULL (R = U2). Latency-bound:
+// eight loads a thread in flight.
+constexpr int COMPOSE_THREADS = 512;
+
+__global__ void __launch_bounds__(COMPOSE_THREADS)
+compose_r_kernel(z64* __restrict__ R, int64_t ldr, int k, const z64* __restrict__ U1, int64_t ldu1,
+                 const z64* __restrict__ U2, int64_t ldu2, const z64* __restrict__ U3, int64_t ldu3,
+                 const ChainStatus* st) {
+    if (st->failed) return;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    z64* t = reinterpret_cast<z64*>(smem_raw);   // the column so far
+    z64* red = t + k;                            // COMPOSE_THREADS partial sums
+    const int j = blockIdx.x;
+    if (!U1) {
+        for (int i = threadIdx.x; i < k; i += blockDim.x) R[i + (int64_t)j * ldr] = U2[i + (int64_t)j * ldu2];
+        return;
+    }
+    const bool third = U3 != nullptr && (st->shifted[1] | st->shifted[2]) != 0;
+    const int span = k < COMPOSE_THREADS ? (k + 31) / 32 * 32 : COMPOSE_THREADS;
+    const int parts = COMPOSE_THREADS / span;
+    const int part = threadIdx.x / span, lane = threadIdx.x - part * span;
+    for (int i = threadIdx.x; i < k; i += blockDim.x) t[i] = U1[i + (int64_t)j * ldu1];
+    __syncthreads();
+    for (int f = 0; f < (third ? 2 : 1); ++f) {
+        const z64* U = f ? U3 : U2;
+        const int64_t ldu = f ? ldu3 : ldu2;
+        for (int i0 = 0; i0 < k; i0 += span) {
+            const int i = i0 + lane;
+            z64 acc = zmake(0.0, 0.0);
+            if (part < parts && i < k)
+                for (int m0 = part; m0 <= j; m0 += 8 * parts) {
+                    z64 u[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) u[q] = U[i + (int64_t)min(m0 + q * parts, j) * ldu];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int m = m0 + q * parts;
+                        if (m >= i && m <= j) zmac(acc, u[q], t[m]);
+                    }
+                }
+            // Rows i0 .. i0 + span of the result need t's rows from i0 on
+            // only, so t can be overwritten strip by strip.
+            red[threadIdx.x] = acc;
+            __syncthreads();
+            if (part == 0 && i < k) {
+                for (int p = 1; p < parts; ++p) {
+                    acc.x += red[p * span + lane].x;
+                    acc.y += red[p * span + lane].y;
+                }
+                t[i] = acc;
+                if (f == (third ? 1 : 0)) R[i + (int64_t)j * ldr] = acc;
+            }
+            __syncthreads();
         }
     }
 }
 
-size_t potrf_gwork_bytes(int k) { return k > POTRF_SMEM_MAX_K ? (size_t)k * k * sizeof(z64) : 0; }
+int compose_r_enqueue(z64* R, int64_t ldr, int k, const z64* U1, int64_t ldu1, const z64* U2, int64_t ldu2,
+                      const z64* U3, int64_t ldu3, const ChainStatus* st, cudaStream_t stream) {
+    const size_t smem = (size_t)(k + COMPOSE_THREADS) * sizeof(z64);
+    if (smem > 48 * 1024)
+        FB_CUDA(cudaFuncSetAttribute(compose_r_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                "cudaFuncSetAttribute(compose_r_kernel)");
+    compose_r_kernel<<<k, COMPOSE_THREADS, smem, stream>>>(R, ldr, k, U1, ldu1, U2, ldu2, U3, ldu3, st);
+    FB_LAUNCHED("compose_r_kernel");
+    return FB_OK;
+}
 
-int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t ldu,
-                  const z64* Rin, int64_t ldrin, z64* Rout, int64_t ldrout, z64* gwork,
-                  ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u) {
-    size_t smem = k <= POTRF_SMEM_MAX_K ? (size_t)k * k * sizeof(z64) : 0;
-    if (smem > 0) {
-        FB_CUDA(cudaFuncSetAttribute(potrf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "cudaFuncSetAttribute(potrf_kernel)");
-    }
-    potrf_kernel<<<1, POTRF_THREADS, smem, stream>>>(G, ldg, k, N, U, ldu, Rin, ldrin, Rout, ldrout, gwork, st,
-                                                     pass, gate, forced_u);
+size_t potrf_gwork_bytes(int k) { return k > POTRF_PACKED_MAX_K ? (size_t)k * k * sizeof(z64) : 0; }
+
+// plan and frag, when given (k <= 64 only), also receive the solve plan of U:
+// what trsm_prepare_enqueue would make of it.
+int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t ldu, z64* gwork,
+                  ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u, TrsmPlan* plan,
+                  double* frag) {
+#define FB_POTRF(store, smem)                                                                                        \
+    do {                                                                                                             \
+        FB_CUDA(cudaFuncSetAttribute(potrf_kernel<store>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)), \
+                "cudaFuncSetAttribute(potrf_kernel)");                                                               \
+        potrf_kernel<store><<<1, POTRF_THREADS, (smem), stream>>>(G, ldg, k, N, U, ldu, gwork, st, pass, gate,       \
+                                                                  forced_u, plan, frag);                             \
+    } while (0)
+    if (k <= TR_KMAX) FB_POTRF(STORE_PLAN, (size_t)2 * TR_KMAX * TR_PREP_LD * sizeof(z64));
+    else if (k <= POTRF_PACKED_MAX_K) FB_POTRF(STORE_PACKED, (size_t)k * (k + 1) / 2 * sizeof(z64));
+    else FB_POTRF(STORE_GLOBAL, 0);
+#undef FB_POTRF
     FB_LAUNCHED("potrf_kernel");
     return FB_OK;
 }
@@ -124,9 +207,12 @@ static int potrf_call(fb_z128* U, int64_t ldu, const fb_z128* G, int64_t ldg, in
     ChainStatus* st = static_cast<ChainStatus*>(workspace);
     z64* gwork = reinterpret_cast<z64*>(static_cast<char*>(workspace) + align_up(sizeof(ChainStatus), 256));
     FB_CUDA(cudaMemsetAsync(st, 0, sizeof(ChainStatus), stream), "cudaMemsetAsync");
-    FB_TRY(potrf_enqueue(reinterpret_cast<const z64*>(G), ldg, k, N, reinterpret_cast<z64*>(U), ldu,
-                         reinterpret_cast<const z64*>(Rin), ldrin, reinterpret_cast<z64*>(Rout), ldrout, gwork, st,
-                         1, GATE_ALWAYS, stream, forced_u));
+    z64* Uz = reinterpret_cast<z64*>(U);
+    FB_TRY(potrf_enqueue(reinterpret_cast<const z64*>(G), ldg, k, N, Uz, ldu, gwork, st, 1, GATE_ALWAYS, stream, forced_u,
+                         nullptr, nullptr));
+    if (Rout)
+        FB_TRY(compose_r_enqueue(reinterpret_cast<z64*>(Rout), ldrout, k, reinterpret_cast<const z64*>(Rin), ldrin, Uz,
+                                 ldu, nullptr, 0, st, stream));
     ChainStatus host{};
     FB_CUDA(cudaMemcpyAsync(&host, st, sizeof host, cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync");
     FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");

@@ -17,8 +17,10 @@ namespace fb {
 
 constexpr int TB_COLS = 64;  // columns of a block of the blocked solve
 
+int trsm_prep_enqueue(const z64* R, int64_t ldr, int k, void* workspace, size_t block_bytes, cudaStream_t stream,
+                      const ChainStatus* st, int gate);
 int trsm_dmma_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
-                      size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st, int gate);
+                      cudaStream_t stream, const ChainStatus* st, int gate);
 size_t trsm_workspace_bytes_small(int k);
 
 static int trsm_blocks(int k) { return (k + TB_COLS - 1) / TB_COLS; }
@@ -45,20 +47,35 @@ trsm_pairs_prep_kernel(const z64* __restrict__ R, int64_t ldr, int k, double* fr
                       width, -1.0);
 }
 
-int trsm_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
-                 size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st, int gate) {
-    if (rows == 0 || k == 0) return FB_OK;
-    if (k <= TB_COLS) return trsm_dmma_enqueue(Y, ldy, rows, k, R, ldr, workspace, workspace_bytes, stream, st, gate);
+// What the solves by R need in the workspace: a plan per diagonal block and,
+// past 64 columns, the pairs' fragments. One preparation serves any number of
+// row blocks.
+int trsm_prepare_enqueue(int k, const z64* R, int64_t ldr, void* workspace, size_t workspace_bytes,
+                         cudaStream_t stream, const ChainStatus* st, int gate) {
+    if (k == 0) return FB_OK;
     if (!workspace || workspace_bytes < trsm_workspace_bytes(k)) {
         set_error(FB_ENOMEM, "rdiv_upper!: workspace of %zu bytes, need %zu", workspace_bytes, trsm_workspace_bytes(k));
         return FB_ENOMEM;
     }
+    if (k > TB_COLS) {
+        const int nb = trsm_blocks(k);
+        double* pairs = reinterpret_cast<double*>(static_cast<char*>(workspace) + (size_t)nb * trsm_diag_bytes());
+        trsm_pairs_prep_kernel<<<nb * (nb - 1) / 2, 256, 0, stream>>>(R, ldr, k, pairs,
+                                                                      trsm_pair_bytes() / sizeof(double), st, gate);
+        FB_LAUNCHED("trsm_pairs_prep_kernel");
+    }
+    return trsm_prep_enqueue(R, ldr, k, workspace, trsm_diag_bytes(), stream, st, gate);
+}
+
+// Y <- Y R^-1 from a prepared workspace.
+int trsm_solve_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
+                       cudaStream_t stream, const ChainStatus* st, int gate) {
+    if (rows == 0 || k == 0) return FB_OK;
+    if (k <= TB_COLS) return trsm_dmma_enqueue(Y, ldy, rows, k, R, ldr, workspace, stream, st, gate);
     const int nb = trsm_blocks(k);
     char* ws = static_cast<char*>(workspace);
     double* pairs = reinterpret_cast<double*>(ws + (size_t)nb * trsm_diag_bytes());
     const size_t pair_doubles = trsm_pair_bytes() / sizeof(double);
-    trsm_pairs_prep_kernel<<<nb * (nb - 1) / 2, 256, 0, stream>>>(R, ldr, k, pairs, pair_doubles, st, gate);
-    FB_LAUNCHED("trsm_pairs_prep_kernel");
     for (int b = 0; b < nb; ++b) {
         const int width = k - TB_COLS * b < TB_COLS ? k - TB_COLS * b : TB_COLS;
         z64* Yb = Y + (int64_t)TB_COLS * b * ldy;
@@ -68,9 +85,16 @@ int trsm_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t
                                 nullptr, 0, nullptr, 0, frag, nullptr, zmake(1.0, 0.0), 1, stream, st, gate));
         }
         FB_TRY(trsm_dmma_enqueue(Yb, ldy, rows, width, R + (int64_t)TB_COLS * b * (1 + ldr), ldr,
-                                 ws + (size_t)b * trsm_diag_bytes(), trsm_diag_bytes(), stream, st, gate));
+                                 ws + (size_t)b * trsm_diag_bytes(), stream, st, gate));
     }
     return FB_OK;
+}
+
+int trsm_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
+                 size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st, int gate) {
+    if (rows == 0 || k == 0) return FB_OK;
+    FB_TRY(trsm_prepare_enqueue(k, R, ldr, workspace, workspace_bytes, stream, st, gate));
+    return trsm_solve_enqueue(Y, ldy, rows, k, R, ldr, workspace, stream, st, gate);
 }
 
 }  // namespace fb

@@ -26,6 +26,7 @@
 namespace fb {
 
 constexpr int TR_THREADS = 256;
+constexpr int TR_PREP_THREADS = 512;
 
 // Substitution for rows in [first, rows) step `stride`: the fallback.
 __device__ void trsm_substitute_rows(z64* __restrict__ Y, int64_t ldy, int64_t rows, int k,
@@ -40,32 +41,35 @@ __device__ void trsm_substitute_rows(z64* __restrict__ Y, int64_t ldy, int64_t r
     }
 }
 
-// One CTA: inv(R) in shared memory, the condition numbers, the choice of
-// path, and the chosen path's B fragments in the workspace.
+// One CTA per 64-column diagonal block of R (one in all for k <= 64): inv(R)
+// in shared memory, the condition numbers, the choice of path, and the chosen
+// path's B fragments in the workspace, block b's at b * block_bytes.
 //   inverse:    cond_1(R) <= TR_INV_COND_LIMIT: Y inv(R) as one product
 //               (fragments of inv(R), n-tile t holding k-steps 0..2t+1);
 //   blocked:    otherwise, if every diagonal 8 x 8 block has cond_1 up to
 //               TR_COND_LIMIT (fragments of -R_cb and inv(R_bb));
 //   substitute: otherwise, plain substitution (no fragments).
-// inv(R) is computed by rows from the bottom, every column of a row at once,
-// four threads to a column sharing the dot product.
-__global__ void __launch_bounds__(256, 1)
-trsm_prep_kernel(const z64* __restrict__ R, int64_t ldr, int k, TrsmPlan* plan, double* __restrict__ frag,
+__global__ void __launch_bounds__(TR_PREP_THREADS, 1)
+trsm_prep_kernel(const z64* __restrict__ R, int64_t ldr, int k, char* plans, size_t block_bytes,
                  const ChainStatus* st, int gate) {
     if (gated_off(st, gate)) return;
     constexpr int LD = TR_PREP_LD;
+    TrsmPlan* plan = reinterpret_cast<TrsmPlan*>(plans + blockIdx.x * block_bytes);
+    double* frag = reinterpret_cast<double*>(plans + blockIdx.x * block_bytes + TR_PLAN_BYTES);
+    R += (int64_t)TR_KMAX * blockIdx.x * (1 + ldr);
+    k = k - TR_KMAX * (int)blockIdx.x < TR_KMAX ? k - TR_KMAX * (int)blockIdx.x : TR_KMAX;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     z64* Rs = reinterpret_cast<z64*>(smem_raw);   // KP x KP, padded with the identity
     z64* Xs = Rs + TR_KMAX * LD;                   // inv(R)
     const int tid = threadIdx.x;
     const int KP = (k + TR_NB - 1) / TR_NB * TR_NB;
-    for (int e = tid; e < KP * KP; e += blockDim.x) {
-        const int i = e / KP, j = e - i * KP;
-        z64 v = zmake(i == j ? 1.0 : 0.0, 0.0);
-        if (i < k && j < k && i <= j) v = R[i + (int64_t)j * ldr];
-        Rs[i * LD + j] = v;
-        Xs[i * LD + j] = zmake(0.0, 0.0);
-    }
+    for (int j = tid >> 5; j < KP; j += TR_PREP_THREADS / 32)
+        for (int i = tid & 31; i < KP; i += 32) {
+            z64 v = zmake(i == j ? 1.0 : 0.0, 0.0);
+            if (i < k && j < k && i <= j) v = R[i + (int64_t)j * ldr];
+            Rs[i * LD + j] = v;
+            Xs[i * LD + j] = zmake(0.0, 0.0);
+        }
     __syncthreads();
     solve_plan(Rs, Xs, k, plan, frag);
 }
@@ -342,23 +346,26 @@ size_t trsm_workspace_bytes_small(int k) {
     return k <= TR_KMAX ? (size_t)TR_PLAN_BYTES + (size_t)TR_FRAG_DOUBLES * sizeof(double) : 0;
 }
 
-// Prep, then all three solvers; the plan the prep writes lets exactly one of
-// them work, so the choice of path costs no host round trip.
-int trsm_dmma_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
-                      size_t workspace_bytes, cudaStream_t stream, const ChainStatus* st, int gate) {
-    if (k > TR_KMAX) { set_error(FB_ENOTSUP, "trsm_dmma: k = %d is past %d", k, TR_KMAX); return FB_ENOTSUP; }
-    if (!workspace || workspace_bytes < trsm_workspace_bytes_small(k)) {
-        set_error(FB_ENOMEM, "rdiv_upper!: workspace of %zu bytes, need %zu", workspace_bytes,
-                  trsm_workspace_bytes_small(k));
-        return FB_ENOMEM;
-    }
-    TrsmPlan* plan = static_cast<TrsmPlan*>(workspace);
-    double* frag = reinterpret_cast<double*>(static_cast<char*>(workspace) + TR_PLAN_BYTES);
-    const size_t prep_smem = (size_t)2 * TR_KMAX * (TR_KMAX + 1) * sizeof(z64);
+// The plans of R's 64-column diagonal blocks, block b's at b * block_bytes of
+// the workspace.
+int trsm_prep_enqueue(const z64* R, int64_t ldr, int k, void* workspace, size_t block_bytes, cudaStream_t stream,
+                      const ChainStatus* st, int gate) {
+    const size_t prep_smem = (size_t)2 * TR_KMAX * TR_PREP_LD * sizeof(z64);
     FB_CUDA(cudaFuncSetAttribute(trsm_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem),
             "cudaFuncSetAttribute(trsm_prep_kernel)");
-    trsm_prep_kernel<<<1, 256, prep_smem, stream>>>(R, ldr, k, plan, frag, st, gate);
+    trsm_prep_kernel<<<(k + TR_KMAX - 1) / TR_KMAX, TR_PREP_THREADS, prep_smem, stream>>>(
+        R, ldr, k, static_cast<char*>(workspace), block_bytes, st, gate);
     FB_LAUNCHED("trsm_prep_kernel");
+    return FB_OK;
+}
+
+// All three solvers; the plan in the workspace lets exactly one of them work,
+// so the choice of path costs no host round trip.
+int trsm_dmma_enqueue(z64* Y, int64_t ldy, int64_t rows, int k, const z64* R, int64_t ldr, void* workspace,
+                      cudaStream_t stream, const ChainStatus* st, int gate) {
+    if (k > TR_KMAX) { set_error(FB_ENOTSUP, "trsm_dmma: k = %d is past %d", k, TR_KMAX); return FB_ENOTSUP; }
+    TrsmPlan* plan = static_cast<TrsmPlan*>(workspace);
+    double* frag = reinterpret_cast<double*>(static_cast<char*>(workspace) + TR_PLAN_BYTES);
     int status = FB_OK;
     switch ((k + 3) / 4) {
 #define FB_INV_CASE(n) case n: status = launch_trsm_inv<n>(Y, ldy, rows, k, plan, frag, stream, st, gate); break;
