@@ -104,6 +104,7 @@ SIGNATURES = {
     "fb_zcholqr2_workspace_size": [_i64, _int, _psz],
     "fb_zcholqr2": [_vp, _i64, _i64, _int, _vp, _i64, _pint, _pint, _vp, _sz, _vp],
     "fb_zcholqr2_query": [_vp, _pint, _pint, _pdbl],
+    "fb_zcholqr2_last_shifts": [_pdbl],
     "fb_zcholqr2_staged_blocks": [_i64, _int, _pint],
     "fb_zcholqr2_staged_workspace_size": [_i64, _int, _int, _psz],
     "fb_zcholqr2_staged": [_vp, _int, _vp, _vp, _int, _vp, _i64, _i64, _int, _vp, _i64, ctypes.c_double, _pint,

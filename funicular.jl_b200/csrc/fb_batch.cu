@@ -1098,8 +1098,7 @@ int fb_zcholqr2_batched_persistent(fb_z128* const* Y, const int64_t* ldy, const 
     cudaStream_t stream = stream_of(queue);
     char* ws = static_cast<char*>(workspace);
     FB_CUDA(cudaMemsetAsync(ws, 0, W.scratch, stream), "cudaMemsetAsync");
-    FB_CUDA(cudaFuncSetAttribute(batch_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PB_SMEM),
-            "cudaFuncSetAttribute(batch_chain_kernel)");
+    FB_ALLOW_SMEM(batch_chain_kernel, PB_SMEM);
     // Largest first (work ~ N k^2), so that the long chunks start early and
     // the small instances fill the end of every phase.
     std::vector<int> order(count);

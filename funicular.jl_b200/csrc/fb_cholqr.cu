@@ -46,7 +46,7 @@ int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t l
                   ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u, TrsmPlan* plan,
                   double* frag);
 int compose_r_enqueue(z64* R, int64_t ldr, int k, const z64* U1, int64_t ldu1, const z64* U2, int64_t ldu2,
-                      const z64* U3, int64_t ldu3, const ChainStatus* st, cudaStream_t stream);
+                      const z64* U3, int64_t ldu3, const ChainStatus* st, int two_passes_only, cudaStream_t stream);
 
 // One pass's factor and everything its solves need in trsm_ws: up to 64
 // columns the Cholesky's own launch leaves the solve plan there.
@@ -94,6 +94,34 @@ int fb_zcholqr2_workspace_size(int64_t N, int k, size_t* bytes) {
     return FB_OK;
 }
 
+// The shifts of this thread's last call that waited for its chain.
+static thread_local double t_last_shifts[3];
+
+// What a chain's status says, as fb_zcholqr2_query reports it.
+static int read_status(const ChainStatus& host, int* info, int* passes, double* shifts) {
+    if (host.timeout) {
+        static const char* const sites[] = {"?", "a Gram stage", "a Gram copy slot", "a solve stage",
+                                            "a solve copy slot", "a factor-ready flag", "a chunk-solved flag"};
+        const int site = host.timeout >= 1 && host.timeout <= 6 ? host.timeout : 0;
+        set_error(FB_ECUDA, "cholqr2! batch: a device-side wait of the persistent kernel (on %s) gave up after its "
+                  "2 s limit, so the results are not valid", sites[site]);
+        return FB_ECUDA;
+    }
+    if (info) *info = host.failed;
+    if (passes) *passes = (host.shifted[1] | host.shifted[2]) ? 3 : 2;
+    if (shifts)
+        for (int p = 0; p < 3; ++p) shifts[p] = host.shift[p + 1];
+    if (host.failed) {
+        set_error(FB_ENOTSPD,
+                  "the Gram matrix of pass %d is not positive definite even after a shift of %.17g, so the "
+                  "columns are numerically dependent: a zero column, a duplicated one, or a condition number "
+                  "past 4.5e15. Drop the dependent columns before orthonormalizing",
+                  host.failed, host.shift[host.failed]);
+        return FB_ENOTSPD;
+    }
+    return FB_OK;
+}
+
 // The chain of one instance. status, when given, replaces the workspace's own
 // status block (a batch keeps one status per instance and shares the rest).
 static int cholqr2_chain(fb_z128* Y, int64_t ldy, int64_t N, int k, fb_z128* R, int64_t ldr, int* info,
@@ -129,8 +157,7 @@ static int cholqr2_chain(fb_z128* Y, int64_t ldy, int64_t N, int k, fb_z128* R, 
     z64* Yz = reinterpret_cast<z64*>(Y);
     const z64 one = zmake(1.0, 0.0), zero = zmake(0.0, 0.0);
 
-    FB_CUDA(cudaMemsetAsync(st, 0, sizeof(ChainStatus), stream), "cudaMemsetAsync");
-    for (int pass = 1; pass <= 3; ++pass) {
+    auto enqueue_pass = [&](int pass) -> int {
         const int gate = pass == 3 ? GATE_THIRD : GATE_HEALTHY;
         if (tensor)
             FB_TRY(ozaki_gram_enqueue(G, k, Yz, ldy, N, k, one, zero, gram_ws, gram_bytes, stream, st, gate));
@@ -141,15 +168,34 @@ static int cholqr2_chain(fb_z128* Y, int64_t ldy, int64_t N, int k, fb_z128* R, 
         // the pass as shifted, so the third pass runs and R = R3 R2 R1.
         FB_TRY(factor_enqueue(G, k, N, U[pass - 1], gwork, trsm_ws, trsm_bytes, st, pass, gate, stream,
                               pass == 1 ? forced_u : 0.0));
-        FB_TRY(trsm_solve_enqueue(Yz, ldy, N, k, U[pass - 1], k, trsm_ws, stream, st, gate));
+        return trsm_solve_enqueue(Yz, ldy, N, k, U[pass - 1], k, trsm_ws, stream, st, gate);
+    };
+    auto enqueue_r = [&](int two_passes_only) {
+        return compose_r_enqueue(reinterpret_cast<z64*>(R), ldr, k, U[0], k, U[1], k, U[2], k, st, two_passes_only,
+                                 stream);
+    };
+    FB_CUDA(cudaMemsetAsync(st, 0, sizeof(ChainStatus), stream), "cudaMemsetAsync");
+    FB_TRY(enqueue_pass(1));
+    FB_TRY(enqueue_pass(2));
+    if (!info) {
+        FB_TRY(enqueue_pass(3));
+        return enqueue_r(0);
     }
-    FB_TRY(compose_r_enqueue(reinterpret_cast<z64*>(R), ldr, k, U[0], k, U[1], k, U[2], k, st, stream));
-
-    if (info) {
+    // A caller that waits reads the status after two passes, so a third one is
+    // launched only when it has to run (its seven gated launches take 16 us of
+    // the GPU and as much of the host when it has not).
+    ChainStatus host{};
+    FB_TRY(enqueue_r(1));
+    FB_CUDA(cudaMemcpyAsync(&host, st, sizeof host, cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync");
+    FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+    if (!host.failed && (host.shifted[1] | host.shifted[2])) {
+        FB_TRY(enqueue_pass(3));
+        FB_TRY(enqueue_r(0));
+        FB_CUDA(cudaMemcpyAsync(&host, st, sizeof host, cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync");
         FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-        return fb_zcholqr2_query(st, info, passes, nullptr);
     }
-    return FB_OK;
+    for (int p = 0; p < 3; ++p) t_last_shifts[p] = host.shift[p + 1];
+    return read_status(host, info, passes, nullptr);
 }
 
 // A batch runs on up to 8 (tunable to 1..16) library-owned streams ("lanes") forked
@@ -326,26 +372,12 @@ int fb_zcholqr2_query(const void* workspace, int* info, int* passes, double* shi
     if (!workspace) { set_error(FB_EINVAL, "fb_zcholqr2_query: NULL workspace"); return FB_EINVAL; }
     ChainStatus host{};
     FB_CUDA(cudaMemcpy(&host, workspace, sizeof host, cudaMemcpyDeviceToHost), "cudaMemcpy");
-    if (host.timeout) {
-        static const char* const sites[] = {"?", "a Gram stage", "a Gram copy slot", "a solve stage",
-                                            "a solve copy slot", "a factor-ready flag", "a chunk-solved flag"};
-        const int site = host.timeout >= 1 && host.timeout <= 6 ? host.timeout : 0;
-        set_error(FB_ECUDA, "cholqr2! batch: a device-side wait of the persistent kernel (on %s) gave up after its "
-                  "2 s limit, so the results are not valid", sites[site]);
-        return FB_ECUDA;
-    }
-    if (info) *info = host.failed;
-    if (passes) *passes = (host.shifted[1] | host.shifted[2]) ? 3 : 2;
-    if (shifts)
-        for (int p = 0; p < 3; ++p) shifts[p] = host.shift[p + 1];
-    if (host.failed) {
-        set_error(FB_ENOTSPD,
-                  "the Gram matrix of pass %d is not positive definite even after a shift of %.17g, so the "
-                  "columns are numerically dependent: a zero column, a duplicated one, or a condition number "
-                  "past 4.5e15. Drop the dependent columns before orthonormalizing",
-                  host.failed, host.shift[host.failed]);
-        return FB_ENOTSPD;
-    }
+    return read_status(host, info, passes, shifts);
+}
+
+int fb_zcholqr2_last_shifts(double* shifts) {
+    if (!shifts) { set_error(FB_EINVAL, "fb_zcholqr2_last_shifts: NULL"); return FB_EINVAL; }
+    for (int p = 0; p < 3; ++p) shifts[p] = t_last_shifts[p];
     return FB_OK;
 }
 
@@ -620,7 +652,7 @@ int fb_zcholqr2_staged(void* const* host_panels, int host_type, const int64_t* h
         }
         FB_CUDA(cudaStreamWaitEvent(stream, sent[nb - 1], 0), "cudaStreamWaitEvent");
     }
-    FB_TRY(compose_r_enqueue(reinterpret_cast<z64*>(R), ldr, k, U[0], k, U[1], k, U[2], k, st, stream));
+    FB_TRY(compose_r_enqueue(reinterpret_cast<z64*>(R), ldr, k, U[0], k, U[1], k, U[2], k, st, 0, stream));
     FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     int inf = 0;
     const int status = fb_zcholqr2_query(st, &inf, passes, nullptr);

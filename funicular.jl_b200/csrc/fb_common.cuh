@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <cstdio>
@@ -40,6 +41,25 @@ void count_launch();
     do {                                   \
         ::fb::count_launch();              \
         FB_CUDA(cudaGetLastError(), what); \
+    } while (0)
+
+// What a launch site asks the runtime about its kernel, kept per device: each
+// question costs about a microsecond of host time, as much as a launch, and a
+// small orthonormalization makes some twenty of them.
+struct PerDevice {
+    static constexpr int DEVICES = 64;
+    std::atomic<int> value[DEVICES] = {};
+};
+// Lets `kernel` use at least `bytes` of dynamic shared memory.
+int allow_smem(const void* kernel, size_t bytes, PerDevice& set, const char* what);
+// Blocks of `threads` threads and `bytes` of dynamic shared memory that fit on
+// an SM (at least 1); `kept` is for this kernel and these sizes alone.
+int blocks_per_sm(const void* kernel, int threads, size_t bytes, PerDevice& kept, int* blocks);
+
+#define FB_ALLOW_SMEM(kernel, bytes)                                                              \
+    do {                                                                                          \
+        static ::fb::PerDevice fb_smem_set_;                                                      \
+        FB_TRY(::fb::allow_smem(reinterpret_cast<const void*>(kernel), bytes, fb_smem_set_, #kernel)); \
     } while (0)
 
 inline cudaStream_t stream_of(fb_queue_t q) { return reinterpret_cast<cudaStream_t>(q); }

@@ -520,13 +520,6 @@ static GramLaunch gram_launch(const GramShape& sh, bool diag) {
     return ln;
 }
 
-template <int PPW>
-static int set_gram_attr(size_t smem) {
-    FB_CUDA(cudaFuncSetAttribute(gram_dmma_kernel<PPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-            "cudaFuncSetAttribute(gram_dmma_kernel)");
-    return FB_OK;
-}
-
 // CTAs of the larger launch that fit on one SM at once: the chunk count is
 // chosen from it so that one wave covers the GPU.
 static int gram_ctas_per_sm(int64_t rows, int kA, int kB, bool hermitian) {
@@ -548,7 +541,7 @@ template <int PPW>
 static int launch_gram_dmma(const CUtensorMap& ma, const CUtensorMap& mb, int64_t rows, const GramShape& sh,
                             const GramLaunch& ln, z64* partial, cudaStream_t stream, const ChainStatus* st, int gate,
                             int chunk0, int chunk1, const SplitGate& split) {
-    FB_TRY(set_gram_attr<PPW>(ln.smem));
+    FB_ALLOW_SMEM(gram_dmma_kernel<PPW>, ln.smem);
     dim3 grid(ln.ntiles, chunk1 - chunk0);
     gram_dmma_kernel<PPW><<<grid, (ln.consumers + 1) * 32, ln.smem, stream>>>(ma, mb, rows, sh, ln, partial, st, gate,
                                                                               chunk0, split);
@@ -627,7 +620,8 @@ static int dmma_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_
     if (chunk0 >= chunk1) return FB_OK;
     CUtensorMap ma, mb;
     FB_TRY(encode_panel_map(&ma, A, rows, kA, lda, sh.tw_a));
-    FB_TRY(encode_panel_map(&mb, B, rows, kB, ldb, sh.tw_b));
+    if (hermitian) mb = ma;
+    else FB_TRY(encode_panel_map(&mb, B, rows, kB, ldb, sh.tw_b));
     if (hermitian) sh.sdiag = gram_launch(sh, true).sdiag;
     const bool launches[2] = {hermitian, !hermitian || sh.nt_a > 1};
     for (int d = 0; d < 2; ++d) {

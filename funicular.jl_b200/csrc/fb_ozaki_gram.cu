@@ -717,8 +717,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, int64_t rows, co
                   double* partial, SplitStat* stats, cudaStream_t stream, const ChainStatus* st, int gate, int chunk0,
                   int chunk1) {
     using C = Cfg<FULL>;
-    FB_CUDA(cudaFuncSetAttribute(split_gram_kernel<FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM),
-            "cudaFuncSetAttribute(split_gram_kernel)");
+    FB_ALLOW_SMEM(split_gram_kernel<FULL>, C::SMEM);
     split_gram_kernel<FULL><<<dim3((unsigned)ntiles, (unsigned)(chunk1 - chunk0)), C::THREADS, C::SMEM, stream>>>(
         ma, mb, rows, sh, partial, stats, st, gate, chunk0);
     FB_LAUNCHED("split_gram_kernel");
@@ -766,7 +765,8 @@ int split_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb,
     SplitStat* stats = reinterpret_cast<SplitStat*>(ws + L.stats);
     CUtensorMap ma, mb;
     FB_TRY(encode_panel_map(&ma, A, rows, kA, lda, 64));
-    FB_TRY(encode_panel_map(&mb, B, rows, kB, ldb, 64));
+    if (sh.hermitian) mb = ma;
+    else FB_TRY(encode_panel_map(&mb, B, rows, kB, ldb, 64));
     const int full = sh.hermitian ? sh.ntiles - sh.nt_a : sh.ntiles;
     if (sh.hermitian)
         FB_TRY(split::launch<false>(ma, mb, rows, sh, sh.nt_a, partial, stats, stream, st, gate, chunk0, chunk1));

@@ -76,15 +76,18 @@ potrf_kernel(const z64* __restrict__ G, int64_t ldg, int k, int64_t N,
 // after the last pass instead of inside each pass's one-CTA factor step. A
 // block per column; 32 rows a warp and, where that leaves warps, the sum over
 // the columns of U cut into `parts` interleaved runs, added in order. U3
-// counts only if a third pass ran, U1 may be NULL (R = U2). Latency-bound:
-// eight loads a thread in flight.
+// counts only if a third pass ran, U1 may be NULL (R = U2); two_passes_only
+// leaves R alone when a third pass is still to come. Latency-bound: eight
+// loads a thread in flight.
 constexpr int COMPOSE_THREADS = 512;
 
 __global__ void __launch_bounds__(COMPOSE_THREADS)
 compose_r_kernel(z64* __restrict__ R, int64_t ldr, int k, const z64* __restrict__ U1, int64_t ldu1,
                  const z64* __restrict__ U2, int64_t ldu2, const z64* __restrict__ U3, int64_t ldu3,
-                 const ChainStatus* st) {
+                 const ChainStatus* st, int two_passes_only) {
     if (st->failed) return;
+    const bool shifted = (st->shifted[1] | st->shifted[2]) != 0;
+    if (two_passes_only && shifted) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     z64* t = reinterpret_cast<z64*>(smem_raw);   // the column so far
     z64* red = t + k;                            // COMPOSE_THREADS partial sums
@@ -93,7 +96,7 @@ compose_r_kernel(z64* __restrict__ R, int64_t ldr, int k, const z64* __restrict_
         for (int i = threadIdx.x; i < k; i += blockDim.x) R[i + (int64_t)j * ldr] = U2[i + (int64_t)j * ldu2];
         return;
     }
-    const bool third = U3 != nullptr && (st->shifted[1] | st->shifted[2]) != 0;
+    const bool third = U3 != nullptr && shifted;
     const int span = k < COMPOSE_THREADS ? (k + 31) / 32 * 32 : COMPOSE_THREADS;
     const int parts = COMPOSE_THREADS / span;
     const int part = threadIdx.x / span, lane = threadIdx.x - part * span;
@@ -134,12 +137,11 @@ compose_r_kernel(z64* __restrict__ R, int64_t ldr, int k, const z64* __restrict_
 }
 
 int compose_r_enqueue(z64* R, int64_t ldr, int k, const z64* U1, int64_t ldu1, const z64* U2, int64_t ldu2,
-                      const z64* U3, int64_t ldu3, const ChainStatus* st, cudaStream_t stream) {
+                      const z64* U3, int64_t ldu3, const ChainStatus* st, int two_passes_only, cudaStream_t stream) {
     const size_t smem = (size_t)(k + COMPOSE_THREADS) * sizeof(z64);
-    if (smem > 48 * 1024)
-        FB_CUDA(cudaFuncSetAttribute(compose_r_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                "cudaFuncSetAttribute(compose_r_kernel)");
-    compose_r_kernel<<<k, COMPOSE_THREADS, smem, stream>>>(R, ldr, k, U1, ldu1, U2, ldu2, U3, ldu3, st);
+    FB_ALLOW_SMEM(compose_r_kernel, smem);
+    compose_r_kernel<<<k, COMPOSE_THREADS, smem, stream>>>(R, ldr, k, U1, ldu1, U2, ldu2, U3, ldu3, st,
+                                                            two_passes_only);
     FB_LAUNCHED("compose_r_kernel");
     return FB_OK;
 }
@@ -151,12 +153,11 @@ size_t potrf_gwork_bytes(int k) { return k > POTRF_PACKED_MAX_K ? (size_t)k * k 
 int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t ldu, z64* gwork,
                   ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u, TrsmPlan* plan,
                   double* frag) {
-#define FB_POTRF(store, smem)                                                                                        \
-    do {                                                                                                             \
-        FB_CUDA(cudaFuncSetAttribute(potrf_kernel<store>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem)), \
-                "cudaFuncSetAttribute(potrf_kernel)");                                                               \
-        potrf_kernel<store><<<1, POTRF_THREADS, (smem), stream>>>(G, ldg, k, N, U, ldu, gwork, st, pass, gate,       \
-                                                                  forced_u, plan, frag);                             \
+#define FB_POTRF(store, smem)                                                                                  \
+    do {                                                                                                       \
+        FB_ALLOW_SMEM(potrf_kernel<store>, smem);                                                              \
+        potrf_kernel<store><<<1, POTRF_THREADS, (smem), stream>>>(G, ldg, k, N, U, ldu, gwork, st, pass, gate, \
+                                                                  forced_u, plan, frag);                       \
     } while (0)
     if (k <= TR_KMAX) FB_POTRF(STORE_PLAN, (size_t)2 * TR_KMAX * TR_PREP_LD * sizeof(z64));
     else if (k <= POTRF_PACKED_MAX_K) FB_POTRF(STORE_PACKED, (size_t)k * (k + 1) / 2 * sizeof(z64));
@@ -212,7 +213,7 @@ static int potrf_call(fb_z128* U, int64_t ldu, const fb_z128* G, int64_t ldg, in
                          nullptr, nullptr));
     if (Rout)
         FB_TRY(compose_r_enqueue(reinterpret_cast<z64*>(Rout), ldrout, k, reinterpret_cast<const z64*>(Rin), ldrin, Uz,
-                                 ldu, nullptr, 0, st, stream));
+                                 ldu, nullptr, 0, st, 0, stream));
     ChainStatus host{};
     FB_CUDA(cudaMemcpyAsync(&host, st, sizeof host, cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync");
     FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");

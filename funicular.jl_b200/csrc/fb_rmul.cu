@@ -163,12 +163,10 @@ static int launch_rmul_dmma(z64* D, int64_t ldd, const z64* A1, int64_t lda1, co
                             const z64* Cm = nullptr, int64_t ldcm = 0) {
     const bool lower = NTK == NTN && A1 != nullptr;
     const size_t smem = (size_t)(dense_frag_doubles(NTK, NTN) + (lower ? lower_frag_doubles(NTN) : 0)) * sizeof(double);
-    FB_CUDA(cudaFuncSetAttribute(rmul_dmma_kernel<NTK, NTN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-            "cudaFuncSetAttribute(rmul_dmma_kernel)");
+    FB_ALLOW_SMEM((rmul_dmma_kernel<NTK, NTN>), smem);
+    static PerDevice fit[2];
     int per_sm = 0;
-    FB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rmul_dmma_kernel<NTK, NTN>, RM_THREADS, smem),
-            "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    if (per_sm < 1) per_sm = 1;
+    FB_TRY(blocks_per_sm(reinterpret_cast<const void*>(rmul_dmma_kernel<NTK, NTN>), RM_THREADS, smem, fit[lower], &per_sm));
     const int64_t units = (rows + 7) / 8;
     const int teams_per_cta = RM_THREADS / 32 / rm_split(NTN);
     int64_t need = (units + teams_per_cta - 1) / teams_per_cta;

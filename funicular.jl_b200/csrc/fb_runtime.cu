@@ -48,6 +48,35 @@ int sm_count() {
     return counts[dev];
 }
 
+int allow_smem(const void* kernel, size_t bytes, PerDevice& set, const char* what) {
+    int dev = 0;
+    FB_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
+    const bool kept = dev >= 0 && dev < PerDevice::DEVICES;
+    if (kept && set.value[dev].load(std::memory_order_acquire) >= (int)bytes) return FB_OK;
+    // Only ever raised, by one thread at a time.
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    if (kept && set.value[dev].load(std::memory_order_acquire) >= (int)bytes) return FB_OK;
+    FB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), what);
+    if (kept) set.value[dev].store((int)bytes, std::memory_order_release);
+    return FB_OK;
+}
+
+int blocks_per_sm(const void* kernel, int threads, size_t bytes, PerDevice& kept, int* blocks) {
+    int dev = 0;
+    FB_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
+    const bool keep = dev >= 0 && dev < PerDevice::DEVICES;
+    int n = keep ? kept.value[dev].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        FB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, bytes),
+                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+        if (n < 1) n = 1;
+        if (keep) kept.value[dev].store(n, std::memory_order_relaxed);
+    }
+    *blocks = n;
+    return FB_OK;
+}
+
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     static std::once_flag once;
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;

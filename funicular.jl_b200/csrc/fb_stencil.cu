@@ -181,8 +181,7 @@ int fb_zlaplace7_apply(fb_z128* Y, int64_t ldy, const fb_z128* X, int64_t ldx, i
     if (cols * zchunks <= 65535 && (ny + LT_Y - 1) / LT_Y <= 65535 && nx < (1 << 30)) {
         CUtensorMap tm;
         FB_TRY(encode_grid_map(&tm, X, nx, ny, nz, cols, ldx, LT_ROW, LT_Y + 2));
-        FB_CUDA(cudaFuncSetAttribute(laplace7_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LT_SMEM),
-                "cudaFuncSetAttribute(laplace7_tiled_kernel)");
+        FB_ALLOW_SMEM(laplace7_tiled_kernel, LT_SMEM);
         const dim3 grid((unsigned)((nx + LT_X - 1) / LT_X), (unsigned)((ny + LT_Y - 1) / LT_Y),
                         (unsigned)(cols * zchunks));
         laplace7_tiled_kernel<<<grid, LT_X * LT_Y + 32, LT_SMEM, stream_of(queue)>>>(

@@ -305,12 +305,10 @@ static int launch_trsm_dmma2(z64* Y, int64_t ldy, int64_t rows, int k, const Trs
                              cudaStream_t stream, const ChainStatus* st, int gate) {
     constexpr int NPAIRS = NBLK * (NBLK + 1) / 2;
     const size_t smem = (size_t)NPAIRS * TR_FRAG * sizeof(double) + (TR2_THREADS / 32) * 2 * TR_BUF * sizeof(z64);
-    FB_CUDA(cudaFuncSetAttribute(trsm_dmma2_kernel<NBLK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-            "cudaFuncSetAttribute(trsm_dmma2_kernel)");
+    FB_ALLOW_SMEM(trsm_dmma2_kernel<NBLK>, smem);
+    static PerDevice fit;
     int per_sm = 0;
-    FB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trsm_dmma2_kernel<NBLK>, TR2_THREADS, smem),
-            "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    if (per_sm < 1) per_sm = 1;
+    FB_TRY(blocks_per_sm(reinterpret_cast<const void*>(trsm_dmma2_kernel<NBLK>), TR2_THREADS, smem, fit, &per_sm));
     const int64_t pairs = ((rows + 7) / 8 + 1) / 2;
     int64_t need = (pairs + TR2_THREADS / 32 - 1) / (TR2_THREADS / 32);
     int64_t grid = (int64_t)sm_count() * per_sm;
@@ -325,12 +323,10 @@ template <int NT>
 static int launch_trsm_inv(z64* Y, int64_t ldy, int64_t rows, int k, const TrsmPlan* plan, const double* frag,
                            cudaStream_t stream, const ChainStatus* st, int gate) {
     const size_t smem = (size_t)32 * NT * (NT + 1) * sizeof(double);
-    FB_CUDA(cudaFuncSetAttribute(trsm_inv_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-            "cudaFuncSetAttribute(trsm_inv_kernel)");
+    FB_ALLOW_SMEM(trsm_inv_kernel<NT>, smem);
+    static PerDevice fit;
     int per_sm = 0;
-    FB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trsm_inv_kernel<NT>, TR_THREADS, smem),
-            "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    if (per_sm < 1) per_sm = 1;
+    FB_TRY(blocks_per_sm(reinterpret_cast<const void*>(trsm_inv_kernel<NT>), TR_THREADS, smem, fit, &per_sm));
     const int64_t units = (rows + 7) / 8;
     int64_t need = (units + TR_THREADS / 32 - 1) / (TR_THREADS / 32);
     int64_t grid = (int64_t)sm_count() * per_sm;
@@ -351,8 +347,7 @@ size_t trsm_workspace_bytes_small(int k) {
 int trsm_prep_enqueue(const z64* R, int64_t ldr, int k, void* workspace, size_t block_bytes, cudaStream_t stream,
                       const ChainStatus* st, int gate) {
     const size_t prep_smem = (size_t)2 * TR_KMAX * TR_PREP_LD * sizeof(z64);
-    FB_CUDA(cudaFuncSetAttribute(trsm_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem),
-            "cudaFuncSetAttribute(trsm_prep_kernel)");
+    FB_ALLOW_SMEM(trsm_prep_kernel, prep_smem);
     trsm_prep_kernel<<<(k + TR_KMAX - 1) / TR_KMAX, TR_PREP_THREADS, prep_smem, stream>>>(
         R, ldr, k, static_cast<char*>(workspace), block_bytes, st, gate);
     FB_LAUNCHED("trsm_prep_kernel");

@@ -210,7 +210,7 @@ def cholqr2_resident(backend, Y: DeviceMatrix, R: DeviceMatrix, wait: bool = Tru
         return None
     shifts = (ctypes.c_double * 3)()
     if status == _lib.FB_OK:
-        status = lib.fb_zcholqr2_query(_vp(ws), None, None, shifts)
+        status = lib.fb_zcholqr2_last_shifts(shifts)
     if status == _lib.FB_ENOTSPD:
         raise NotPositiveDefinite(_lib.last_error())
     _lib.check(status, "cholqr2!")

@@ -209,8 +209,9 @@ int fb_zpotrf_shifted(fb_z128* U, int64_t ldu, const fb_z128* G, int64_t ldg,
  * shifted, R = R3 R2 R1 written to R (k x k, zeros below the diagonal).
  * Every step runs on `queue`; the branch to the third pass and the stop after
  * a failed factorization are taken on the device, so the call enqueues a
- * fixed sequence of launches. With info != NULL the call synchronizes and
- * sets *info = 0, or the 1-based pass whose Gram was not positive definite
+ * fixed sequence of launches. With info != NULL the call synchronizes (once
+ * after two passes, and once more when a third has to run) and sets
+ * *info = 0, or the 1-based pass whose Gram was not positive definite
  * (returning FB_ENOTSPD); *passes = 2 or 3 if non-NULL. With info == NULL it
  * returns at once and fb_zcholqr2_query reads the outcome after the queue
  * has drained. workspace: fb_zcholqr2_workspace_size bytes, 256-byte
@@ -221,6 +222,10 @@ int fb_zcholqr2(fb_z128* Y, int64_t ldy, int64_t N, int k,
                 void* workspace, size_t workspace_bytes, fb_queue_t queue);
 int fb_zcholqr2_query(const void* workspace, int* info, int* passes,
                       double* shifts /* 3 entries, or NULL */);
+/* The shifts (3 entries) of this host thread's last fb_zcholqr2,
+ * fb_zcholqr2_tc or fb_zcholqr3_shifted call with info != NULL, which has read
+ * them already: no device access. */
+int fb_zcholqr2_last_shifts(double* shifts);
 
 /* cholqr2!(Y) (src/panelblas.jl:130-146) end to end for a matrix held in
  * page-locked host panels (the resident path of a PanelMatrix whose panels
