@@ -1,7 +1,11 @@
 // gram_accumulate! (src/kernels.jl:22-55): C <- alpha A^H B + beta C for tall
-// skinny A (rows x kA) and B (rows x kB), ComplexF64, FP64 throughout.
+// skinny A (rows x kA) and B (rows x kB), ComplexF64. Wide and tall products
+// run in the split form of fb_ozaki_gram.cu (gram_takes_split draws the line),
+// with the FP64 kernels of this file behind its verdict; all others run here,
+// the folded ones of narrow panels in gram_narrow_kernel and the rest in
+// gram_dmma_kernel.
 //
-// Layout of the work. C is cut into tiles of at most 64 x 64 columns. A CTA
+// Layout of the work (gram_dmma_kernel). C is cut into tiles of at most 64 x 64 columns. A CTA
 // owns one tile and one chunk of rows, which it streams through shared memory
 // in stages of 32 rows: one producer warp issues TMA loads (boxes of 8 rows x
 // the tile's columns, 128-byte swizzled, zero-filled past the last row and
@@ -320,6 +324,153 @@ gram_dmma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
 }
 
+// The folded Gram of a narrow panel (at most G_NARROW_STRIPS strips of eight
+// columns, one tile). Dealt out to warps, so few blocks leave the
+// sub-partitions uneven (k = 32: ten blocks, five warps, so one sub-partition
+// of four gets two of them and the FP64 pipe runs at 5/8; k = 8: one warp).
+// Here every warp computes ALL of the folded blocks on its own rows instead:
+// warp w of the CTA takes the 8-row boxes w, w + GN_WARPS, ... of the chunk
+// through a ring of its own, which its lane 0 refills, so no warp waits for
+// another until the end, when the CTA adds its warps' blocks in order. The A
+// and B fragments of a strip are the same registers: two 8-byte loads a lane
+// feed its block row and its block column.
+// Bounds at 2^20 rows, us: the FP64 tensor pipe 29 (k = 16, both parts of the
+// diagonal blocks 44), 117 (k = 32), 183 (k = 40); memory 41, 82, 103.
+// Measured, blocks dealt to warps / this: k = 8 80 / 37, k = 16 119 / 68,
+// k = 24 148 / 114, k = 32 215 / 153, k = 40 382 / 222; 1e5 rows: k = 8
+// 28 / 12, k = 32 32 / 25, k = 48 51 / 41. At k = 32 that is 0.77 of the FP64
+// pipe. More strips do not fit a warp's registers (six take 206).
+constexpr int G_NARROW_STRIPS = 6;      // 8-column strips, at most (k <= 48)
+constexpr int GN_WARPS = 8;
+
+__host__ __device__ constexpr int gn_slots(int strips) {
+    const int fit = (200 * 1024) / (GN_WARPS * strips * 1024);
+    return fit < 8 ? fit : 8;
+}
+
+template <int S, bool SDIAG>
+__global__ void __launch_bounds__(GN_WARPS * 32, 1)
+gram_narrow_kernel(const __grid_constant__ CUtensorMap tmA, int64_t rows, GramShape sh, z64* __restrict__ partial,
+                   const ChainStatus* st, int gate, int chunk0, SplitGate split) {
+    if (gated_off(st, gate) || split.accepted()) return;
+    constexpr int SLOTS = gn_slots(S);
+    constexpr int BOX = S * 1024;                     // 8 rows x 8 S columns
+    constexpr int NDIAG = SDIAG ? 2 : 4;              // doubles a lane holds of a diagonal block
+    constexpr int NACC = S * NDIAG + S * (S - 1) / 2 * 4;
+    static_assert(NACC * 256 <= SLOTS * BOX, "a warp's blocks fit its ring");
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GN_WARPS * SLOTS * BOX);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* ring = smem + warp * SLOTS * BOX;
+    uint64_t* full = bars + warp * SLOTS;
+    if (lane == 0) {
+        for (int b = 0; b < SLOTS; ++b) mbar_init(&full[b], 1);
+        mbar_fence_init();
+    }
+    __syncwarp();
+
+    const int chunk = chunk0 + (int)blockIdx.x;
+    const int64_t row0 = (int64_t)chunk * sh.chunk_rows;
+    const int64_t row_end = min(rows, row0 + sh.chunk_rows);
+    const int nboxes = (int)((row_end - row0 + GS_BOX_ROWS - 1) / GS_BOX_ROWS);
+    const int mine = nboxes > warp ? (nboxes - warp + GN_WARPS - 1) / GN_WARPS : 0;
+    auto fetch = [&](int j, int b) {
+        mbar_arrive_expect_tx(&full[b], BOX);
+        tma_load_2d(ring + b * BOX, &tmA, (int)(2 * (row0 + (int64_t)(warp + j * GN_WARPS) * GS_BOX_ROWS)), 0, &full[b]);
+    };
+    if (lane == 0)
+        for (int j = 0; j < mine && j < SLOTS; ++j) fetch(j, j);
+
+    const int col8 = lane >> 2, t = (lane >> 1) & 1, part = lane & 1;
+    const int own = col8 * 128 + part * 8, oth = col8 * 128 + (part ^ 1) * 8;
+    int swz[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) swz[q] = ((q + 4 * t) ^ col8) << 4;
+    const unsigned long long flip = part ? 0ull : 0x8000000000000000ull;
+
+    double acc[NACC];
+#pragma unroll
+    for (int i = 0; i < NACC; ++i) acc[i] = 0.0;
+    bool ok = true;
+    int b = 0;
+    uint32_t phase = 0;
+    int todo = mine;
+    for (int j = 0; j < todo; ++j) {
+        // After a wait that ran out, only the boxes already asked for are
+        // waited for.
+        if (!mbar_wait_warp(&full[b], phase) && ok) { ok = false; todo = min(mine, j + SLOTS); }
+        const unsigned char* box = ring + b * BOX;
+        double w[S], o[S];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+                w[i] = *reinterpret_cast<const double*>(box + i * 1024 + own + swz[q]);
+                o[i] = *reinterpret_cast<const double*>(box + i * 1024 + oth + swz[q]);
+            }
+            if (q == 3) {
+#pragma unroll
+                for (int i = 0; i < S; ++i) { hold_loaded(w[i]); hold_loaded(o[i]); }
+                __syncwarp();
+                if (lane == 0 && ok && j + SLOTS < mine) fetch(j + SLOTS, b);
+            }
+            int a = 0;
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+                o[i] = __longlong_as_double(__double_as_longlong(o[i]) ^ flip);
+                if constexpr (SDIAG) {
+                    dmma_884(acc[a], acc[a + 1], w[i] + o[i], w[i]);
+                } else {
+                    dmma_884(acc[a], acc[a + 1], w[i], w[i]);
+                    dmma_884(acc[a + 2], acc[a + 3], o[i], w[i]);
+                }
+                a += NDIAG;
+#pragma unroll
+                for (int l = i + 1; l < S; ++l, a += 4) {
+                    dmma_884(acc[a], acc[a + 1], w[i], w[l]);
+                    dmma_884(acc[a + 2], acc[a + 3], o[i], w[l]);
+                }
+            }
+        }
+        if (++b == SLOTS) { b = 0; phase ^= 1u; }
+    }
+    // A box that never arrived poisons this CTA's share of the result.
+    if (!ok)
+#pragma unroll
+        for (int i = 0; i < NACC; ++i) acc[i] = __longlong_as_double(0x7ff8000000000000ll);
+
+    // Every copy into the ring has been waited for, and read by this warp.
+    __syncwarp();
+    double* mineacc = reinterpret_cast<double*>(ring);
+#pragma unroll
+    for (int i = 0; i < NACC; ++i) mineacc[i * 32 + lane] = acc[i];
+    __syncthreads();
+    z64* out = partial + (size_t)chunk * (size_t)(sh.tw_a * sh.tw_b);
+    const double* all = reinterpret_cast<const double*>(smem);
+    auto sum = [&](int a, int l) {
+        double s = 0.0;
+#pragma unroll
+        for (int v = 0; v < GN_WARPS; ++v) s += all[v * (SLOTS * BOX / 8) + a * 32 + l];
+        return s;
+    };
+    // Block q in the order of the accumulators, split over the warps.
+    int q = 0, a = 0;
+#pragma unroll
+    for (int i = 0; i < S; ++i)
+#pragma unroll
+        for (int l = i; l < S; ++l, ++q) {
+            const bool im = l > i || !SDIAG;
+            if (q % GN_WARPS == warp) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    out[(l * 8 + 2 * (lane & 3) + c) * sh.tw_a + i * 8 + (lane >> 2)] =
+                        zmake(sum(a + c, lane), im ? sum(a + 2 + c, lane) : 0.0);
+            }
+            a += im ? 4 : 2;
+        }
+}
+
 // Entry (li, lj) of a tile summed over the chunks by one warp: lane l adds
 // chunks l, l+32, ... in order, then a fixed shuffle tree adds the lanes (the
 // sum is lane 0's).
@@ -445,31 +596,21 @@ static GramShape gram_shape(int64_t rows, int kA, int kB, int hermitian, int cta
 }
 
 // The consumer slots' blocks. Full tiles: row-major. Folded diagonal tiles
-// with at least as many warps as block rows: warp w < nb takes the diagonal
+// (seven or eight block rows, at least as many warps): warp w < nb takes the diagonal
 // block (w, w) in slot 0 (one MMA a k-step, S-coded) and then blocks of its
 // own block row (sharing the A fragment); the rest fill the free slots in
 // order. At k = 64 (eight block rows, three blocks a warp, twelve warps) this
 // gives warps 0-7 one diagonal and two off-diagonal blocks and warps 8-11
 // three off-diagonal ones, so each sub-partition (warps w, w + 4, w + 8)
-// issues 5 + 5 + 6 = 16 MMAs a k-step. Smaller tiles without that many warps
-// compute their diagonal blocks like any other.
+// issues 5 + 5 + 6 = 16 MMAs a k-step.
 static void build_pair_table(GramLaunch& ln) {
     for (int i = 0; i < 64; ++i) ln.pi[i] = ln.pj[i] = -1;
-    ln.sdiag = 0;
-    std::vector<std::pair<int, int>> order;
+    ln.sdiag = ln.diag;
     if (ln.diag) {
-        for (int I = 0; I < ln.nb_a; ++I)
-            for (int J = I; J < ln.nb_a; ++J) order.push_back({I, J});
-    } else {
-        for (int I = 0; I < ln.nb_a; ++I)
-            for (int J = 0; J < ln.nb_b; ++J) order.push_back({I, J});
-    }
-    if (ln.diag && ln.consumers >= ln.nb_a) {
-        ln.sdiag = 1;
         std::vector<std::vector<std::pair<int, int>>> warps(ln.consumers);
         std::vector<std::pair<int, int>> off;
-        for (auto& p : order)
-            if (p.first != p.second) off.push_back(p);
+        for (int I = 0; I < ln.nb_a; ++I)
+            for (int J = I + 1; J < ln.nb_a; ++J) off.push_back({I, J});
         std::vector<bool> used(off.size(), false);
         for (int w = 0; w < ln.nb_a; ++w) {
             warps[w].push_back({w, w});
@@ -486,9 +627,9 @@ static void build_pair_table(GramLaunch& ln) {
             }
         return;
     }
-    for (size_t q = 0; q < order.size() && q < 64; ++q) {
-        ln.pi[q] = (signed char)order[q].first;
-        ln.pj[q] = (signed char)order[q].second;
+    for (int q = 0; q < ln.npairs; ++q) {
+        ln.pi[q] = (signed char)(q / ln.nb_b);
+        ln.pj[q] = (signed char)(q % ln.nb_b);
     }
 }
 
@@ -520,9 +661,20 @@ static GramLaunch gram_launch(const GramShape& sh, bool diag) {
     return ln;
 }
 
+// Two and three strips compute both parts of their diagonal blocks: they are
+// bound by memory either way.
+__host__ __device__ constexpr bool narrow_sdiag(int strips) { return strips != 2 && strips != 3; }
+
+// Whether the narrow kernel takes the folded Gram of this many columns.
+static bool gram_is_narrow(int k, bool hermitian) { return hermitian && k <= 8 * G_NARROW_STRIPS; }
+
+// Whether the diagonal blocks of a folded Gram's partial tiles hold S.
+static int folded_sdiag(const GramShape& sh, int k) { return gram_is_narrow(k, true) ? narrow_sdiag(sh.tw_a / 8) : 1; }
+
 // CTAs of the larger launch that fit on one SM at once: the chunk count is
 // chosen from it so that one wave covers the GPU.
 static int gram_ctas_per_sm(int64_t rows, int kA, int kB, bool hermitian) {
+    if (gram_is_narrow(kA, hermitian)) return 1;
     GramShape sh = gram_shape(rows, kA, kB, hermitian ? 1 : 0, 1);
     // The larger of the two launches sets the pace: the diagonal tile when
     // there is only one, the off-diagonal tiles otherwise.
@@ -546,6 +698,18 @@ static int launch_gram_dmma(const CUtensorMap& ma, const CUtensorMap& mb, int64_
     gram_dmma_kernel<PPW><<<grid, (ln.consumers + 1) * 32, ln.smem, stream>>>(ma, mb, rows, sh, ln, partial, st, gate,
                                                                               chunk0, split);
     FB_LAUNCHED("gram_dmma_kernel");
+    return FB_OK;
+}
+
+template <int S, bool SDIAG>
+static int launch_gram_narrow(const CUtensorMap& ma, int64_t rows, const GramShape& sh, z64* partial,
+                              cudaStream_t stream, const ChainStatus* st, int gate, int chunk0, int chunk1,
+                              const SplitGate& split) {
+    constexpr size_t smem = (size_t)GN_WARPS * gn_slots(S) * (S * 1024 + sizeof(uint64_t)) + 1024;
+    FB_ALLOW_SMEM((gram_narrow_kernel<S, SDIAG>), smem);
+    gram_narrow_kernel<S, SDIAG><<<chunk1 - chunk0, GN_WARPS * 32, smem, stream>>>(ma, rows, sh, partial, st, gate,
+                                                                                 chunk0, split);
+    FB_LAUNCHED("gram_narrow_kernel");
     return FB_OK;
 }
 
@@ -622,7 +786,19 @@ static int dmma_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_
     FB_TRY(encode_panel_map(&ma, A, rows, kA, lda, sh.tw_a));
     if (hermitian) mb = ma;
     else FB_TRY(encode_panel_map(&mb, B, rows, kB, ldb, sh.tw_b));
-    if (hermitian) sh.sdiag = gram_launch(sh, true).sdiag;
+    if (gram_is_narrow(kA, hermitian)) {
+        switch (sh.tw_a / 8) {
+#define FB_NARROW_CASE(s) launch_gram_narrow<s, narrow_sdiag(s)>(ma, rows, sh, partial, stream, st, gate, chunk0, chunk1, split)
+            case 1: return FB_NARROW_CASE(1);
+            case 2: return FB_NARROW_CASE(2);
+            case 3: return FB_NARROW_CASE(3);
+            case 4: return FB_NARROW_CASE(4);
+            case 5: return FB_NARROW_CASE(5);
+            default: return FB_NARROW_CASE(6);
+#undef FB_NARROW_CASE
+        }
+    }
+    sh.sdiag = hermitian;
     const bool launches[2] = {hermitian, !hermitian || sh.nt_a > 1};
     for (int d = 0; d < 2; ++d) {
         if (!launches[d]) continue;
@@ -677,7 +853,7 @@ int gram_reduce_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z6
                         int kB, bool hermitian, z64 alpha, z64 beta, void* workspace, cudaStream_t stream,
                         const ChainStatus* st, int gate) {
     GramShape sh = gram_plan(rows, kA, kB, hermitian);
-    if (hermitian && sh.nchunks > 0) sh.sdiag = gram_launch(sh, true).sdiag;
+    if (hermitian && sh.nchunks > 0) sh.sdiag = folded_sdiag(sh, kA);
     z64* partial = static_cast<z64*>(workspace);
     SplitGate split{};
     if (gram_takes_split(rows, kA, kB, hermitian)) {
