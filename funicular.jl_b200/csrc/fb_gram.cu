@@ -722,20 +722,32 @@ static GramShape gram_plan(int64_t rows, int kA, int kB, bool hermitian) {
 }
 
 // Whether the Gram of this shape runs in the split form (fb_ozaki_gram.cu).
-// It costs whole 64 x 64 tiles whatever the columns, and some 20 us more in
-// fixed work than the FP64 kernels (scales, drains, verdict, two more
-// launches), so narrow and short products stay in FP64. Microseconds, FP64 /
-// split, on both sides of the lines drawn here:
-//   folded, 1e6 rows: k = 32 207 / 320, k = 40 367 / 320, k = 64 535 / 326;
-//   folded, k = 64: 1e5 rows 70 / 73, 2e5 rows 122 / 103;
-//   folded, k = 128: 5e4 rows 141 / 136, 1e5 rows 243 / 189;
-//   cross, 1e6 rows: 32 x 32 282 / 511, 40 x 40 507 / 526, 48 x 48 568 / 517,
-//   64 x 64 933 / 563; 64 x 64: 5e4 rows 65 / 64, 1e5 rows 113 / 89.
+// Two things draw the lines.
+// Accuracy: the slices' error relative to ||a_i|| ||b_j|| falls with the rows
+// (entries are cut at 2^-51 of their column's scale), that of the FP64 kernels
+// does not; the split form is taken where its is no larger. Gaussian entries,
+// against 64-bit-mantissa sums, rms off the diagonal in 1e-18 (FP64 / split),
+// in brackets the largest error of any entry in 1e-16:
+//   folded, k = 64: 1.5e5 rows 3.7 / 6.0 (2.4 / 2.7), 2.5e5 rows 3.9 / 4.2
+//   (3.7 / 2.5), 3e5 rows 3.7 / 3.5 (3.7 / 2.1), 5e5 rows 3.9 / 3.3 (2.8 / 0.9);
+//   k = 100: 2.5e5 rows 3.7 / 4.2, 3e5 rows 3.8 / 3.3;
+//   cross, 64 x 64: 1.5e5 rows 3.8 / 4.6, 2.5e5 rows 3.9 / 3.6, 5e5 rows 4.0 / 2.6.
+// Time: the split form costs whole 64 x 64 tiles whatever the columns, and
+// some 20 us more in fixed work than the FP64 kernels (scales, drains,
+// verdict, two more launches). Microseconds, FP64 / split:
+//   folded, k = 40: 1e6 rows 213 / 273;
+//   k = 48: 3e5 rows 98 / 105, 5e5 rows 153 / 154, 1e6 rows 289 / 273;
+//   k = 64: 2e5 rows 122 / 82, 1e6 rows 535 / 300;
+//   cross, 32 blocks of 8 x 8 a tile: 64 x 32, 1e6 rows 506 / 521;
+//   36 blocks: 48 x 48, 1e5 rows 72 / 82, 4.1e5 rows 242 / 234;
+//   40 blocks (where the FP64 kernel has eight a warp) and more: 64 x 36, 6e4
+//   rows 82 / 61; 64 x 64, 1e5 rows 113 / 82.
 static bool gram_takes_split(int64_t rows, int kA, int kB, bool hermitian) {
     if (rows > ((int64_t)1 << 30)) return false;   // the tile loads' 32-bit coordinates
+    if (hermitian) return kA > 40 && rows >= (kA > 48 ? 300000 : 500000);
     const int a = kA < G_TILE ? kA : G_TILE, b = kB < G_TILE ? kB : G_TILE;
-    if (hermitian) return kA > G_TILE ? rows >= 60000 : (kA > 40 && rows >= 150000);
-    return a * b >= 48 * 48 && rows >= 60000;
+    const int blocks = ((a + 7) / 8) * ((b + 7) / 8);
+    return blocks >= 36 && rows >= (blocks >= 40 ? 250000 : 400000);
 }
 
 // The workspace of a split Gram: the split's own layout, whose partial tiles

@@ -30,7 +30,7 @@ def norms(A):
     return np.linalg.norm(A, axis=0)
 
 
-@pytest.mark.parametrize("N", [149_999, 150_000, 150_001, 150_015])
+@pytest.mark.parametrize("N", [299_999, 300_000, 300_001, 300_015])
 @pytest.mark.parametrize("k", [40, 41, 64, 65, 128, 130])
 def test_folded(fb, backend, N, k):
     rng = np.random.default_rng(N + k)
@@ -46,8 +46,8 @@ def test_folded(fb, backend, N, k):
     assert np.max(np.abs(H - want) / (3 * scale + 2)) <= 4 * EPS * np.sqrt(N)
 
 
-@pytest.mark.parametrize("N,kA,kB", [(59_999, 64, 64), (60_000, 64, 64), (60_017, 48, 48), (60_001, 64, 36),
-                                     (70_003, 100, 70), (60_002, 129, 64)])
+@pytest.mark.parametrize("N,kA,kB", [(249_999, 64, 64), (250_000, 64, 64), (400_017, 48, 48), (250_001, 64, 36),
+                                     (250_003, 100, 70), (250_002, 129, 64)])
 def test_cross(fb, backend, N, kA, kB):
     rng = np.random.default_rng(N + kA + kB)
     A, B = randmatrix(rng, N, kA), randmatrix(rng, N, kB)
@@ -58,10 +58,10 @@ def test_cross(fb, backend, N, kA, kB):
 def test_zero_columns_and_rows_that_grow(fb, backend):
     # Scales adapt as the rows grow by 2^40; zero columns stay exactly zero.
     rng = np.random.default_rng(3)
-    N, k = 200_000, 64
+    N, k = 300_000, 64
     A = randmatrix(rng, N, k) * (2.0 ** (40 * np.arange(N) / N))[:, None]
     A[:, 5] = 0
-    A[:150_000, 9] = 0
+    A[:200_000, 9] = 0
     G = gram(fb, backend, A)
     n = norms(A)
     n[5] = 1.0
@@ -72,11 +72,10 @@ def test_zero_columns_and_rows_that_grow(fb, backend):
 @pytest.mark.parametrize("same", [True, False])
 def test_a_spike_is_summed_in_fp64(fb, backend, same):
     # One entry of 2^40 in a column of unit entries. Against the exact product
-    # the FP64 sums are off by at most (rows of a chunk) eps 2^40, about 0.3;
-    # slices scaled for the spike would lose about 2^-9 of every other entry
-    # of the column, some 0.6 in each sum.
+    # the FP64 sums are off by at most (rows of a chunk) eps 2^40; slices scaled
+    # for the spike would round every other entry of the column to 2^-11.
     rng = np.random.default_rng(4)
-    N, k = 200_000, 64
+    N, k = 300_000, 64
     A = (rng.standard_normal((N, k)) + 1j * rng.standard_normal((N, k))) / np.sqrt(2)
     A[77, 3] = 2.0 ** 40
     B = A if same else (rng.standard_normal((N, k)) + 1j * rng.standard_normal((N, k))) / np.sqrt(2)
@@ -95,7 +94,7 @@ def test_what_slices_cannot_hold_is_summed_in_fp64(fb, backend, value, same):
     # A NaN, an infinity or a magnitude whose products leave the slices' range
     # reaches only the rows and columns it belongs to.
     rng = np.random.default_rng(5)
-    N, k = 160_001, 56
+    N, k = 300_001, 56
     A = randmatrix(rng, N, k)
     B = A if same else randmatrix(rng, N, k)
     ref = A.conj().T @ B
