@@ -569,10 +569,11 @@ __device__ void pb_solve_inverse(GramCtx& c, uint32_t& full_par, z64* Y, int64_t
                 a[s] = (got && col < k) ? *reinterpret_cast<const double*>(base + col * c.col_bytes) : 0.0;
             }
             if (u + NSW >= end) {
+                uint32_t seen = 0;
 #pragma unroll
-                for (int s = 0; s < NS; ++s) hold_loaded(a[s]);
+                for (int s = 0; s < NS; ++s) mark_loaded(seen, a[s]);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&c.empty[slot]);
+                if (lane == 0) mbar_arrive(&c.empty[slot + (seen & zero)]);
             }
             const int64_t row = c.row0 + u * 8 + rr;
             const bool live = row < rows;

@@ -351,7 +351,7 @@ __host__ __device__ constexpr int gn_slots(int strips) {
 template <int S, bool SDIAG>
 __global__ void __launch_bounds__(GN_WARPS * 32, 1)
 gram_narrow_kernel(const __grid_constant__ CUtensorMap tmA, int64_t rows, GramShape sh, z64* __restrict__ partial,
-                   const ChainStatus* st, int gate, int chunk0, SplitGate split) {
+                   const ChainStatus* st, int gate, int chunk0, SplitGate split, int zero) {
     if (gated_off(st, gate) || split.accepted()) return;
     constexpr int SLOTS = gn_slots(S);
     constexpr int BOX = S * 1024;                     // 8 rows x 8 S columns
@@ -410,10 +410,11 @@ gram_narrow_kernel(const __grid_constant__ CUtensorMap tmA, int64_t rows, GramSh
                 o[i] = *reinterpret_cast<const double*>(box + i * 1024 + oth + swz[q]);
             }
             if (q == 3) {
+                uint32_t seen = 0;
 #pragma unroll
-                for (int i = 0; i < S; ++i) { hold_loaded(w[i]); hold_loaded(o[i]); }
+                for (int i = 0; i < S; ++i) { mark_loaded(seen, w[i]); mark_loaded(seen, o[i]); }
                 __syncwarp();
-                if (lane == 0 && ok && j + SLOTS < mine) fetch(j + SLOTS, b);
+                if (lane == 0 && ok && j + SLOTS < mine) fetch(j + SLOTS, b + (int)(seen & zero));
             }
             int a = 0;
 #pragma unroll
@@ -708,7 +709,7 @@ static int launch_gram_narrow(const CUtensorMap& ma, int64_t rows, const GramSha
     constexpr size_t smem = (size_t)GN_WARPS * gn_slots(S) * (S * 1024 + sizeof(uint64_t)) + 1024;
     FB_ALLOW_SMEM((gram_narrow_kernel<S, SDIAG>), smem);
     gram_narrow_kernel<S, SDIAG><<<chunk1 - chunk0, GN_WARPS * 32, smem, stream>>>(ma, rows, sh, partial, st, gate,
-                                                                                 chunk0, split);
+                                                                                 chunk0, split, 0);
     FB_LAUNCHED("gram_narrow_kernel");
     return FB_OK;
 }

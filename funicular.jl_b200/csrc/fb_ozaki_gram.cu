@@ -230,7 +230,7 @@ template <bool FULL>
 __global__ void __launch_bounds__(Cfg<FULL>::THREADS, 1)
 split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int64_t rows,
                   SplitShape sh, double* __restrict__ partial, SplitStat* __restrict__ stats, const ChainStatus* st,
-                  int gate, int chunk0) {
+                  int gate, int chunk0, int zero) {
     if (gated_off(st, gate)) return;
     using C = Cfg<FULL>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -438,16 +438,17 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 // A new epoch: the MMAs of the one before it all precede this
                 // stage's, which wait for this group. (The rows are read
                 // again, so that no register holds them across the drain.)
+                uint32_t seen = 0;
                 if (TO_A && fresh && s > 0) {
                     if (!drain(s - 1, stage.Eold, stage.Eold + (FULL ? 64 : 0), stage.epoch > 1) || !load(s))
                         return false;
 #pragma unroll
                     for (int n = 0; n < NC; ++n)
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) hold_loaded(v[n][e]);
+                        for (int e = 0; e < 8; ++e) mark_loaded(seen, v[n][e]);
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&fp_empty[s % C::SLOTS]);
+                if (lane == 0) mbar_arrive(&fp_empty[s % C::SLOTS + (seen & zero)]);
                 double sc[NC];
 #pragma unroll
                 for (int n = 0; n < NC; ++n) {
@@ -726,7 +727,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, int64_t rows, co
     using C = Cfg<FULL>;
     FB_ALLOW_SMEM(split_gram_kernel<FULL>, C::SMEM);
     split_gram_kernel<FULL><<<dim3((unsigned)ntiles, (unsigned)(chunk1 - chunk0)), C::THREADS, C::SMEM, stream>>>(
-        ma, mb, rows, sh, partial, stats, st, gate, chunk0);
+        ma, mb, rows, sh, partial, stats, st, gate, chunk0, 0);
     FB_LAUNCHED("split_gram_kernel");
     return FB_OK;
 }

@@ -67,7 +67,7 @@ constexpr size_t LT_SMEM = (size_t)LT_SLOTS * LT_PLANE + 2 * LT_SLOTS * sizeof(u
 
 __global__ void __launch_bounds__(LT_X * LT_Y + 32, 2)
 laplace7_tiled_kernel(const __grid_constant__ CUtensorMap tm, z64* __restrict__ Y, int64_t ldy, int nx, int ny, int nz,
-                      z64 shift, int zchunks) {
+                      z64 shift, int zchunks, int zero) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)LT_SLOTS * LT_PLANE);
@@ -116,9 +116,10 @@ laplace7_tiled_kernel(const __grid_constant__ CUtensorMap tm, z64* __restrict__ 
     bool ok = mbar_wait_warp(&full[0], 0) && mbar_wait_warp(&full[1], 0);
     below = point(0, 0);
     cur = point(1, 0);
-    hold_loaded(below.x);
+    uint32_t seen = 0;
+    mark_loaded(seen, below.x);
     __syncwarp();
-    if (tx == 0) mbar_arrive(&empty[0]);
+    if (tx == 0) mbar_arrive(&empty[seen & zero]);
     int b = 1, nb = 2;
     uint32_t ph = 0;
     for (int z = z0; z < z1; ++z) {
@@ -127,10 +128,12 @@ laplace7_tiled_kernel(const __grid_constant__ CUtensorMap tm, z64* __restrict__ 
         const z64 l = point(b, -1), r = point(b, 1), d = point(b, -LT_ROW), u = point(b, LT_ROW);
         double sx = l.x + r.x + d.x + u.x + below.x + above.x;
         double sy = l.y + r.y + d.y + u.y + below.y + above.y;
-        hold_loaded(sx);
-        hold_loaded(sy);
+        mark_loaded(seen, l.x);
+        mark_loaded(seen, r.x);
+        mark_loaded(seen, d.x);
+        mark_loaded(seen, u.x);
         __syncwarp();
-        if (tx == 0) mbar_arrive(&empty[b]);
+        if (tx == 0) mbar_arrive(&empty[b + (seen & zero)]);
         if (!ok) sx = __longlong_as_double(0x7ff8000000000000ll);   // a plane never came: no silent wrong answer
         if (inside) *y = zmake(dr * cur.x - di * cur.y - sx, dr * cur.y + di * cur.x - sy);
         y += plane;
@@ -185,7 +188,7 @@ int fb_zlaplace7_apply(fb_z128* Y, int64_t ldy, const fb_z128* X, int64_t ldx, i
         const dim3 grid((unsigned)((nx + LT_X - 1) / LT_X), (unsigned)((ny + LT_Y - 1) / LT_Y),
                         (unsigned)(cols * zchunks));
         laplace7_tiled_kernel<<<grid, LT_X * LT_Y + 32, LT_SMEM, stream_of(queue)>>>(
-            tm, reinterpret_cast<z64*>(Y), ldy, nx, ny, nz, zmake(shift.re, shift.im), (int)zchunks);
+            tm, reinterpret_cast<z64*>(Y), ldy, nx, ny, nz, zmake(shift.re, shift.im), (int)zchunks, 0);
         FB_LAUNCHED("laplace7_tiled_kernel");
         return FB_OK;
     }

@@ -68,11 +68,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return true;
 }
 
-// A value that comes from shared memory is in its register before anything
-// after this point in program order runs. A warp that gives a buffer back with
-// mbar_arrive needs it: the arrival and a load still on its way take different
-// paths, and a copy into the buffer could otherwise overtake the load.
-__device__ __forceinline__ void hold_loaded(double& v) { asm volatile("" : "+d"(v)::"memory"); }
+// Values read from shared memory, marked as arrived. A load and what gives its
+// buffer back (an mbarrier arrival, the next copy into it) take different
+// paths, and the later one can overtake the load. So what gives the buffer back
+// takes an address that depends on every value read: bar + (seen & zero), with
+// `zero` a kernel argument that is always 0, which the compiler cannot see.
+__device__ __forceinline__ void mark_loaded(uint32_t& seen, double v) { seen |= (uint32_t)__double2hiint(v); }
 
 // mbar_wait by a whole converged warp, every lane polling and the warp
 // deciding together. The branch is then uniform: lanes that left a polling
