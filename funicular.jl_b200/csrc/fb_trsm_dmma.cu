@@ -5,10 +5,11 @@
 // so every flop is in 8 x 8 complex products (DMMA m8n8k4 on the real form
 // of the complex product), the diagonal blocks entering through their
 // inverses. That costs 14 % more flops than substitution and makes the error
-// of block b grow with cond(R_bb) instead of staying at a few eps; each CTA
-// therefore estimates cond_1(R_bb) of every diagonal block while it builds
-// the inverses, and if one exceeds TR_COND_LIMIT the whole CTA solves its rows
-// by plain substitution instead (the reference's ztrsm arithmetic).
+// of block b grow with cond(R_bb) instead of staying at a few eps; the plan
+// therefore estimates cond_1(R_bb) of every diagonal block with the inverses,
+// and if one exceeds TR_COND_LIMIT all rows are solved by plain substitution
+// instead (the reference's ztrsm arithmetic). A well-conditioned R is solved
+// as one product by inv(R).
 //
 // A warp owns rows for the whole solve (16 in the blocked path: two 8-row
 // units sharing every B fragment; 8 in the product by the inverse), so warps
@@ -16,10 +17,13 @@
 // registers, already in the MMA A-operand layout; results leave the
 // accumulators (C layout) through a small per-warp shared buffer that
 // transposes them into that layout.
-// Every CTA first expands R into "fragment order" in shared memory: for each
-// pair of column blocks (c <= b), the 16 x 16 real matrix of the product
-// with -R_cb (c < b) or inv(R_bb) (c = b), laid out so that each lane's MMA B
-// operand is one consecutive 8-byte load.
+// The plan (the Cholesky's launch or trsm_prep_kernel) holds R in "fragment
+// order", which every CTA copies to shared memory: for each pair of column
+// blocks (c <= b), the 16 x 16 real matrix of the product with -R_cb (c < b) or
+// inv(R_bb) (c = b), laid out so that each lane's MMA B operand is one
+// consecutive 8-byte load.
+#include <algorithm>
+
 #include "fb_factor.cuh"
 #include "fb_tma.cuh"
 
@@ -91,34 +95,84 @@ __device__ __forceinline__ void copy_frags(double* dst, const double* __restrict
     __syncthreads();
 }
 
-// Y R^-1 as one product by inv(R) (path inverse): a warp owns 8 rows, loads
-// them once in the MMA A layout and writes each 4-column n-tile of the result
-// straight from the accumulators; n-tile t needs k-steps 0..2t+1 only.
+// Y R^-1 as one product by inv(R) (path inverse): a warp owns 8 rows at a time,
+// holds them in the MMA A layout and writes each 4-column n-tile of the result
+// straight from the accumulators; n-tile t needs k-steps 0..2t+1 only. The rows
+// come by TMA through a ring of the warp's own, which its lane 0 refills: with
+// loads straight to registers every warp waited out the memory latency once a
+// unit. One unit of 64 columns is in flight while its predecessor is
+// multiplied, more of narrower ones; the fragments take 70 KB at k = 64.
+// Bounds at 2^20 rows, us: the FP64 tensor pipe 122 (k = 32: 72 MMAs a unit),
+// 490 (k = 64: 272); memory 164, 328. Measured, loads to registers / this:
+// k = 16 142 / 120, k = 32 295 / 215, k = 48 450 / 370, k = 64 708 / 607; 4096
+// rows: k = 16 21 / 16, k = 64 82 / 38 (a short panel spreads over the SMs).
+constexpr int TRI_WARPS = 16;                 // warps of a CTA, one CTA an SM
+constexpr size_t TRI_SMEM = 220 * 1024;       // fragments and rings
+
+__host__ __device__ constexpr int tri_frag_bytes(int nt) { return 32 * nt * (nt + 1) * 8; }
+__host__ __device__ constexpr int tri_box_bytes(int nt) { return 4 * nt * 128; }   // 8 rows x 4 nt columns
+// The swizzle goes by address: a slot starts at a multiple of its 1024 bytes.
+__host__ __device__ constexpr int tri_slot_bytes(int nt) { return (tri_box_bytes(nt) + 1023) / 1024 * 1024; }
+__host__ __device__ constexpr int tri_slots(int nt) {
+    const int fit = (int)((TRI_SMEM - tri_frag_bytes(nt)) / (TRI_WARPS * tri_slot_bytes(nt)));
+    return fit < 4 ? fit : 4;
+}
+
 template <int NT>
-__global__ void __launch_bounds__(TR_THREADS, 2)
-trsm_inv_kernel(z64* __restrict__ Y, int64_t ldy, int64_t rows, int k, const TrsmPlan* plan,
-                const double* __restrict__ gfrag, const ChainStatus* st, int gate, int zero) {
+__global__ void __launch_bounds__(32 * TRI_WARPS, 1)
+trsm_inv_kernel(const __grid_constant__ CUtensorMap tmY, z64* __restrict__ Y, int64_t ldy, int64_t rows, int k,
+                const TrsmPlan* plan, const double* __restrict__ gfrag, const ChainStatus* st, int gate, int zero) {
     if (gated_off(st, gate) || plan->path != PATH_INVERSE) return;
     constexpr int KP = 4 * NT;
     constexpr int NS = KP / 2;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double* frag = reinterpret_cast<double*>(smem_raw);
+    constexpr int SLOTS = tri_slots(NT), SLOT = tri_slot_bytes(NT);
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    unsigned char* ring = smem + warp * SLOTS * SLOT;
+    double* frag = reinterpret_cast<double*>(smem + warps * SLOTS * SLOT);
+    uint64_t* full = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(frag) + tri_frag_bytes(NT)) + warp * SLOTS;
+
+    const int units = (int)((rows + 7) / 8);
+    const int stride = (int)gridDim.x * warps;
+    const int first = (int)blockIdx.x * warps + warp;
+    auto fetch = [&](int u, int b) {
+        mbar_arrive_expect_tx(&full[b], tri_box_bytes(NT));
+        tma_load_2d(ring + b * SLOT, &tmY, u * 16, 0, &full[b]);
+    };
+    if (lane == 0) {
+        for (int b = 0; b < SLOTS; ++b) mbar_init(&full[b], 1);
+        mbar_fence_init();
+        for (int b = 0; b < SLOTS && first + b * stride < units; ++b) fetch(first + b * stride, b);
+    }
     copy_frags(frag, gfrag, 32 * NT * (NT + 1));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cq = lane & 3, acol = cq >> 1, apart = lane & 1, rr = lane >> 2;
-    const int64_t units = (rows + 7) / 8;
-    const int64_t warps_total = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp; u < units; u += warps_total) {
-        const int64_t row = u * 8 + rr;
-        const bool live = row < rows;
-        z64* yrow = Y + (live ? row : 0);
+    // Swizzled offsets of row rr in columns 2 s + acol, s = 0..3 (and the same
+    // eight columns further on).
+    int off[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) off[s] = (2 * s + acol) * 128 + ((rr ^ (2 * s + acol)) << 4) + apart * 8;
+    bool ok = true;
+    int b = 0;
+    uint32_t phase = 0;
+    for (int u = first; u < units; u += stride) {
+        ok = ok && mbar_wait_warp(&full[b], phase);
+        const unsigned char* box = ring + b * SLOT;
         double a[NS];
 #pragma unroll
-        for (int s = 0; s < NS; ++s) {
-            const int col = 2 * s + acol;
-            a[s] = (live && col < k) ? reinterpret_cast<const double*>(yrow + (int64_t)col * ldy)[apart] : 0.0;
-        }
+        for (int s = 0; s < NS; ++s) a[s] = *reinterpret_cast<const double*>(box + (s >> 2) * 1024 + off[s & 3]);
+        uint32_t seen = 0;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) mark_loaded(seen, a[s]);
+        __syncwarp();
+        if (lane == 0 && ok && u + SLOTS * stride < units) fetch(u + SLOTS * stride, b + (int)(seen & zero));
+        if (++b == SLOTS) { b = 0; phase ^= 1u; }
+        // Rows that never arrived come out as NaN.
+        if (!ok) a[0] = __longlong_as_double(0x7ff8000000000000ll);
+        const int64_t row = (int64_t)u * 8 + rr;
+        const bool live = row < rows;
+        z64* yrow = Y + row;
         // The loads of n-tile t wait for the result of n-tile t - 2 and,
         // inside a tile, each group of eight for the group before: two tiles
         // in flight, and no more fragments in registers than that needs.
@@ -322,21 +376,27 @@ static int launch_trsm_dmma2(z64* Y, int64_t ldy, int64_t rows, int k, const Trs
 template <int NT>
 static int launch_trsm_inv(z64* Y, int64_t ldy, int64_t rows, int k, const TrsmPlan* plan, const double* frag,
                            cudaStream_t stream, const ChainStatus* st, int gate) {
-    const size_t smem = (size_t)32 * NT * (NT + 1) * sizeof(double);
-    FB_ALLOW_SMEM(trsm_inv_kernel<NT>, smem);
-    static PerDevice fit;
-    int per_sm = 0;
-    FB_TRY(blocks_per_sm(reinterpret_cast<const void*>(trsm_inv_kernel<NT>), TR_THREADS, smem, fit, &per_sm));
-    const int64_t units = (rows + 7) / 8;
-    int64_t need = (units + TR_THREADS / 32 - 1) / (TR_THREADS / 32);
-    int64_t grid = (int64_t)sm_count() * per_sm;
-    if (grid > need) grid = need;
-    if (grid < 1) grid = 1;
-    trsm_inv_kernel<NT><<<(unsigned)grid, TR_THREADS, smem, stream>>>(Y, ldy, rows, k, plan, frag, st, gate, 0);
-    FB_LAUNCHED("trsm_inv_kernel");
+    constexpr int bars = tri_slots(NT) * (int)sizeof(uint64_t);
+    auto smem = [&](int warps) {
+        return (size_t)tri_frag_bytes(NT) + (size_t)warps * (tri_slots(NT) * tri_slot_bytes(NT) + bars) + 1024;
+    };
+    FB_ALLOW_SMEM(trsm_inv_kernel<NT>, smem(TRI_WARPS));
+    // The loads' coordinates are 32-bit: more rows than 2^30 go in slices.
+    constexpr int64_t SLICE = (int64_t)1 << 30;
+    for (int64_t r = 0; r < rows; r += SLICE) {
+        const int64_t n = rows - r < SLICE ? rows - r : SLICE;
+        CUtensorMap map;
+        FB_TRY(encode_panel_map(&map, Y + r, n, k, ldy, 4 * NT));
+        // A short panel spreads over the SMs before it fills them.
+        const int64_t units = (n + 7) / 8, sms = sm_count();
+        const int warps = (int)std::min<int64_t>((units + sms - 1) / sms, TRI_WARPS);
+        const int64_t grid = std::min<int64_t>((units + warps - 1) / warps, sms);
+        trsm_inv_kernel<NT><<<(unsigned)grid, 32 * warps, smem(warps), stream>>>(map, Y + r, ldy, n, k, plan, frag, st,
+                                                                               gate, 0);
+        FB_LAUNCHED("trsm_inv_kernel");
+    }
     return FB_OK;
 }
-
 
 size_t trsm_workspace_bytes_small(int k) {
     return k <= TR_KMAX ? (size_t)TR_PLAN_BYTES + (size_t)TR_FRAG_DOUBLES * sizeof(double) : 0;
