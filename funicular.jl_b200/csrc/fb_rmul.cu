@@ -1,6 +1,7 @@
-// The tensor-core right product D <- beta D + A1 L + A2 C (fb_rmul.cuh).
+// The tensor-core right products (fb_rmul.cuh): D <- beta D + A1 L + A2 C and
+// D <- beta D + A C in rmul_dmma_kernel, tall D <- A C in rmul_pair_kernel.
 //
-// A team of one or two warps owns 8 rows at a time, each warp a contiguous
+// rmul_dmma_kernel: a team of one or two warps owns 8 rows at a time, each warp a contiguous
 // share of the output n-tiles. A warp streams the rows' entries one k-step
 // (two complex columns) at a time, loading each entry of A1 and A2 once (the
 // second warp of a team finds them in L1), and keeps its n-tiles in its
@@ -8,6 +9,8 @@
 // groups of four k-steps ahead of the products; the group after that waits for
 // the products of the current one, which bounds the registers the prefetch
 // holds.
+#include <algorithm>
+
 #include "fb_rmul.cuh"
 #include "fb_tma.cuh"
 
@@ -136,6 +139,125 @@ rmul_dmma_kernel(z64* D, int64_t ldd, const z64* A1, int64_t lda1, const z64* A2
     }
 }
 
+// The tall product by a dense factor alone, D <- A C. A warp owns two 8-row
+// units at a time and all n-tiles, so a fragment read from shared memory feeds
+// two MMAs (with one unit a warp the fragment reads took half of the shared
+// memory pipe), and keeps 4 NTN accumulators a lane. The rows come by TMA, 16
+// columns of both units a stage, through a ring of the warp's own that its
+// lane 0 refills across units. Each accumulator adds the k-steps in order, as
+// in rmul_dmma_kernel: the bits are the same.
+// Bound at 2500003 x 64 by 64 x 64: the FP64 tensor pipe, 2.23 ms (memory
+// 0.78). Measured there, rmul_dmma_kernel / this: 2.74 / 2.42 ms; 64 x 40
+// 2.26 / 1.71, 48 x 48 1.92 / 1.44, 32 x 32 1.12 / 0.68, 20 x 50 2.20 / 0.78
+// (K runs in steps of two columns here, there in the template's).
+// Narrow results leave the registers for twice the warps.
+__host__ __device__ constexpr int rp_warps(int ntn) { return ntn <= 4 ? 16 : 8; }
+constexpr int RP_STAGE = 4096;                       // 2 units x 8 rows x 16 columns
+constexpr size_t RP_SMEM = 227 * 1024 - 2048;        // fragments and rings
+
+template <int NTN>
+__global__ void __launch_bounds__(32 * rp_warps(NTN), 1)
+rmul_pair_kernel(const __grid_constant__ CUtensorMap tmA, z64* D, int64_t ldd, int64_t rows, int K, int n,
+                 const double* __restrict__ gdense, const z64* __restrict__ Cm, int64_t ldcm, int slots, int cwarps,
+                 int zero, const ChainStatus* st, int gate) {
+    if (gated_off(st, gate)) return;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int WARPS = rp_warps(NTN);
+    const int ngroups = (K + 15) / 16;               // stages a unit pair
+    const int ksteps = (K + 1) / 2;
+    unsigned char* ring = smem + warp * slots * RP_STAGE;
+    double* fd = reinterpret_cast<double*>(smem + WARPS * slots * RP_STAGE);
+    uint64_t* full = reinterpret_cast<uint64_t*>(fd + ksteps * NTN * 32) + warp * slots;
+
+    const int pairs = (int)((rows + 15) / 16);
+    const int stride = (int)gridDim.x * cwarps;
+    const int first = warp < cwarps ? (int)blockIdx.x * cwarps + warp : pairs;
+    int fu = first, fg = 0;                          // the next stage to ask for
+    auto fetch = [&](int b) {
+        mbar_arrive_expect_tx(&full[b], RP_STAGE);
+        tma_load_2d(ring + b * RP_STAGE, &tmA, fu * 32, fg * 16, &full[b]);
+        tma_load_2d(ring + b * RP_STAGE + RP_STAGE / 2, &tmA, fu * 32 + 16, fg * 16, &full[b]);
+        if (++fg == ngroups) { fg = 0; fu += stride; }
+    };
+    if (lane == 0) {
+        for (int b = 0; b < slots; ++b) mbar_init(&full[b], 1);
+        mbar_fence_init();
+        for (int b = 0; b < slots && fu < pairs; ++b) fetch(b);
+    }
+    // The factor's fragments, zero past K and n, 16 loads in flight a thread.
+    const int entries = ksteps * NTN * 32;
+    for (int e0 = threadIdx.x; e0 < entries; e0 += 16 * 32 * WARPS) {
+        double v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int e = e0 + i * 32 * WARPS;
+            const int q = e >> 5, s = q / NTN;
+            v[i] = e >= entries ? 0.0 : gdense ? gdense[e] : frag_entry(Cm, ldcm, K, n, s, q - s * NTN, lane, 1.0);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (e0 + i * 32 * WARPS < entries) fd[e0 + i * 32 * WARPS] = v[i];
+    }
+    __syncthreads();
+
+    const int rr = lane >> 2, cq = lane & 3, acol = cq >> 1, apart = lane & 1;
+    // Swizzled offsets of row rr in columns 2 s + acol of a box, s = 0..3 (and
+    // the same eight columns further on).
+    int off[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) off[s] = (2 * s + acol) * 128 + ((rr ^ (2 * s + acol)) << 4) + apart * 8;
+    bool ok = true;
+    int b = 0;
+    uint32_t phase = 0;
+    for (int u = first; u < pairs; u += stride) {
+        const int64_t row = (int64_t)u * 16 + rr;
+        const bool live0 = row < rows, live1 = row + 8 < rows;
+        double acc[2][NTN][2] = {};
+        const double* fp = fd + lane;
+        for (int g = 0; g < ngroups; ++g) {
+            ok = ok && mbar_wait_warp(&full[b], phase);
+            const unsigned char* box = ring + b * RP_STAGE;
+            double a[2][8];
+            uint32_t seen = 0;
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                a[0][s] = *reinterpret_cast<const double*>(box + (s >> 2) * 1024 + off[s & 3]);
+                a[1][s] = *reinterpret_cast<const double*>(box + RP_STAGE / 2 + (s >> 2) * 1024 + off[s & 3]);
+            }
+#pragma unroll
+            for (int s = 0; s < 8; ++s) { mark_loaded(seen, a[0][s]); mark_loaded(seen, a[1][s]); }
+            __syncwarp();
+            if (lane == 0 && ok && fu < pairs) fetch(b + (int)(seen & zero));
+            if (++b == slots) { b = 0; phase ^= 1u; }
+            // Rows that never arrived come out as NaN.
+            if (!ok) a[0][0] = a[1][0] = __longlong_as_double(0x7ff8000000000000ll);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                if (8 * g + s >= ksteps) break;
+                // A step's fragments are read once the previous step's first
+                // product is done, not hoisted further ahead.
+                fp = hold(fp, acc[0][0][0], zero);
+#pragma unroll
+                for (int t = 0; t < NTN; ++t) {
+                    const double bv = fp[t * 32];
+                    dmma_884(acc[0][t][0], acc[0][t][1], a[0][s], bv);
+                    dmma_884(acc[1][t][0], acc[1][t][1], a[1][s], bv);
+                }
+                fp += NTN * 32;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < NTN; ++t) {
+            const int col = 4 * t + cq;
+            if (col >= n) continue;
+            if (live0) D[row + (int64_t)col * ldd] = zmake(acc[0][t][0], acc[0][t][1]);
+            if (live1) D[row + 8 + (int64_t)col * ldd] = zmake(acc[1][t][0], acc[1][t][1]);
+        }
+    }
+}
+
 // The same product on the FP64 pipes, for factors past 64: a thread per row,
 // output columns in order, so D may be the same matrix as A1 (column j of the
 // result reads columns l >= j of A1 only) but must not overlap A2.
@@ -181,6 +303,60 @@ static int launch_rmul_dmma(z64* D, int64_t ldd, const z64* A1, int64_t lda1, co
     return FB_OK;
 }
 
+template <int NTN>
+static int launch_rmul_pair(z64* D, int64_t ldd, const z64* A, int64_t lda, int64_t rows, int K, int n,
+                            const double* fdense, cudaStream_t stream, const ChainStatus* st, int gate, const z64* Cm,
+                            int64_t ldcm) {
+    constexpr int WARPS = rp_warps(NTN);
+    const size_t frags = (size_t)(K + 1) / 2 * NTN * 32 * sizeof(double);
+    const int slots = (int)std::min<size_t>((RP_SMEM - frags) / (WARPS * RP_STAGE), 4);
+    const size_t smem = frags + (size_t)WARPS * slots * (RP_STAGE + sizeof(uint64_t)) + 1024;
+    FB_ALLOW_SMEM(rmul_pair_kernel<NTN>, RP_SMEM + 2048);
+    // The loads' coordinates are 32-bit: more rows than 2^30 go in slices.
+    constexpr int64_t SLICE = (int64_t)1 << 30;
+    for (int64_t r = 0; r < rows; r += SLICE) {
+        const int64_t m = rows - r < SLICE ? rows - r : SLICE;
+        CUtensorMap map;
+        FB_TRY(encode_panel_map(&map, A + r, m, K, lda, 16));
+        // A short panel spreads over the SMs before it fills them.
+        const int64_t pairs = (m + 15) / 16, sms = sm_count();
+        const int warps = (int)std::min<int64_t>((pairs + sms - 1) / sms, WARPS);
+        const int64_t grid = std::min<int64_t>((pairs + warps - 1) / warps, sms);
+        rmul_pair_kernel<NTN><<<(unsigned)grid, 32 * WARPS, smem, stream>>>(
+            map, D + r, ldd, m, K, n, fdense, Cm, ldcm, slots, warps, 0, st, gate);
+        FB_LAUNCHED("rmul_pair_kernel");
+    }
+    return FB_OK;
+}
+
+// D <- A C with the factor as fragments or as a matrix.
+static int rmul_pair_enqueue(z64* D, int64_t ldd, const z64* A, int64_t lda, int64_t rows, int K, int n,
+                             const double* fdense, cudaStream_t stream, const ChainStatus* st, int gate, const z64* Cm,
+                             int64_t ldcm) {
+    switch ((n + 3) / 4) {
+#define FB_RP_CASE(t) \
+    case t: return launch_rmul_pair<t>(D, ldd, A, lda, rows, K, n, fdense, stream, st, gate, Cm, ldcm);
+        FB_RP_CASE(1) FB_RP_CASE(2) FB_RP_CASE(3) FB_RP_CASE(4) FB_RP_CASE(5) FB_RP_CASE(6) FB_RP_CASE(7) FB_RP_CASE(8)
+        FB_RP_CASE(9) FB_RP_CASE(10) FB_RP_CASE(11) FB_RP_CASE(12) FB_RP_CASE(13) FB_RP_CASE(14) FB_RP_CASE(15)
+        FB_RP_CASE(16)
+#undef FB_RP_CASE
+    }
+    set_error(FB_EINVAL, "rmul: no template for a %d x %d factor", K, n);
+    return FB_EINVAL;
+}
+
+// Whether the product by a dense factor runs in rmul_pair_kernel. Its units
+// are twice as long and leave the last wave emptier, so short panels stay in
+// rmul_dmma_kernel, and so do the narrowest, whose stages would be mostly
+// padding, and those that add to D, whose loads only more warps can hide.
+// Microseconds, rmul_dmma_kernel / rmul_pair_kernel: 64 x 64: 5000 rows 23 / 31,
+// 1e5 rows 132 / 140, 2.6e5 rows 308 / 290; 8 x 20: 2.6e5 rows 46 / 31; 4 x 4:
+// 2.6e5 rows 8 / 12, 2.5e6 rows 65 / 64; adding to D, 2^20 x 64 by 64 x 64: the
+// whole adjoint it is part of 10.6 / 11.3 ms.
+static bool rmul_takes_pairs(int64_t rows, int K, int use_beta) {
+    return rows >= (int64_t)1 << 18 && K >= 8 && !use_beta;
+}
+
 // D <- beta D (when use_beta) + A C for a K x n factor C given as a matrix,
 // K, n <= 64, on the tensor cores. The template is the smallest one that
 // holds the factor: square when K and n take the same number of 4-column
@@ -192,6 +368,8 @@ int rmul_matrix_enqueue(z64* D, int64_t ldd, const z64* A, int64_t lda, int64_t 
         set_error(FB_EINVAL, "rmul: a %d x %d factor is past the 64 x 64 the tensor-core product takes", K, n);
         return FB_EINVAL;
     }
+    if (rmul_takes_pairs(rows, K, use_beta))
+        return rmul_pair_enqueue(D, ldd, A, lda, rows, K, n, nullptr, stream, nullptr, GATE_ALWAYS, C, ldc);
     const int ntk = (K + 3) / 4, ntn = (n + 3) / 4;
     if (ntk <= ntn) {
         switch (ntn) {
@@ -223,6 +401,8 @@ int rmul_enqueue(z64* D, int64_t ldd, const z64* A1, int64_t lda1, const z64* A2
     if (A1 && K != n) { set_error(FB_EINVAL, "rmul: a lower triangular factor is square, got %d x %d", K, n); return FB_EINVAL; }
     const int ntk = (K + 3) / 4, ntn = (n + 3) / 4;
     if (K <= RM_KMAX && n <= RM_KMAX && (ntk == ntn || ntk == RM_KMAX / 4)) {
+        if (A1 == nullptr && rmul_takes_pairs(rows, K, use_beta))
+            return rmul_pair_enqueue(D, ldd, A2, lda2, rows, K, n, fdense, stream, st, gate, nullptr, 0);
         if (ntk == ntn) {
             switch (ntn) {
 #define FB_RM_SQ(t) \
