@@ -353,8 +353,9 @@ static int rmul_pair_enqueue(z64* D, int64_t ldd, const z64* A, int64_t lda, int
 // 1e5 rows 132 / 140, 2.6e5 rows 308 / 290; 8 x 20: 2.6e5 rows 46 / 31; 4 x 4:
 // 2.6e5 rows 8 / 12, 2.5e6 rows 65 / 64; adding to D, 2^20 x 64 by 64 x 64: the
 // whole adjoint it is part of 10.6 / 11.3 ms.
-static bool rmul_takes_pairs(int64_t rows, int K, int use_beta) {
-    return rows >= (int64_t)1 << 18 && K >= 8 && !use_beta;
+// TMA wants A on a 16-byte boundary.
+static bool rmul_takes_pairs(const z64* A, int64_t rows, int K, int use_beta) {
+    return rows >= (int64_t)1 << 18 && K >= 8 && !use_beta && ((uintptr_t)A & 15) == 0;
 }
 
 // D <- beta D (when use_beta) + A C for a K x n factor C given as a matrix,
@@ -368,7 +369,7 @@ int rmul_matrix_enqueue(z64* D, int64_t ldd, const z64* A, int64_t lda, int64_t 
         set_error(FB_EINVAL, "rmul: a %d x %d factor is past the 64 x 64 the tensor-core product takes", K, n);
         return FB_EINVAL;
     }
-    if (rmul_takes_pairs(rows, K, use_beta))
+    if (rmul_takes_pairs(A, rows, K, use_beta))
         return rmul_pair_enqueue(D, ldd, A, lda, rows, K, n, nullptr, stream, nullptr, GATE_ALWAYS, C, ldc);
     const int ntk = (K + 3) / 4, ntn = (n + 3) / 4;
     if (ntk <= ntn) {
@@ -401,7 +402,7 @@ int rmul_enqueue(z64* D, int64_t ldd, const z64* A1, int64_t lda1, const z64* A2
     if (A1 && K != n) { set_error(FB_EINVAL, "rmul: a lower triangular factor is square, got %d x %d", K, n); return FB_EINVAL; }
     const int ntk = (K + 3) / 4, ntn = (n + 3) / 4;
     if (K <= RM_KMAX && n <= RM_KMAX && (ntk == ntn || ntk == RM_KMAX / 4)) {
-        if (A1 == nullptr && rmul_takes_pairs(rows, K, use_beta))
+        if (A1 == nullptr && rmul_takes_pairs(A2, rows, K, use_beta))
             return rmul_pair_enqueue(D, ldd, A2, lda2, rows, K, n, fdense, stream, st, gate, nullptr, 0);
         if (ntk == ntn) {
             switch (ntn) {
