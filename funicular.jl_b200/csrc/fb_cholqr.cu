@@ -9,7 +9,8 @@
 // a status block in the workspace: a pass whose Cholesky fails stops every
 // later kernel (Y keeps what the finished passes made of it, as when the
 // reference throws before its rdiv_rows!), and the third pass runs only if a
-// shift fired in pass 1 or 2.
+// shift fired in pass 1 or 2. A call that waits for its result reads the status
+// after two passes instead and launches a third one only when it has to run.
 #include <algorithm>
 #include <atomic>
 #include <mutex>
