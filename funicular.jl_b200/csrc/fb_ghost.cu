@@ -65,17 +65,25 @@ __device__ __forceinline__ void philox4x32_10(uint32_t c[4], const RoundKeys& rk
 constexpr int LN_DOUBLES = 2 * FB_GHOST_LN_ENTRIES;
 constexpr int TRIG_DOUBLES = 2 * 256;
 
-// ln u for u = n 2^-53, 1 <= n <= 2^53, read straight from the integer (the
-// exponent and fraction bits u has as a double, without converting):
-// u = 2^e m with m in (sqrt(1/2), sqrt(2)].
+// The integers become doubles by placing their bits under a power of two and
+// subtracting it, which is exact for these ranges: two additions instead of a
+// count of leading zeros, 64-bit shifts and conversions, all on slow pipes. The
+// fill is bound by instruction issue: 880 -> 854 us for 40001688 x 3.
+
+// ln u for u = n 2^-53, 1 <= n <= 2^53: u = 2^e m with m in (sqrt(1/2), sqrt(2)].
 __device__ __forceinline__ double ln_u53(uint64_t n, const double* __restrict__ lnt) {
-    const int lz = __clzll((long long)n);
-    int e = 10 - lz;                                          // 63 - lz - 53
-    const uint64_t frac = ((n << lz) >> 11) & 0x000fffffffffffffull;
-    double m = __longlong_as_double((long long)(frac | 0x3ff0000000000000ull));
-    if (m > 1.4142135623730951) { m = m * 0.5; e += 1; }
-    const int j = (int)((__double_as_longlong(m) >> 44) & 0xff);
-    const int idx = m >= 1.0 ? j : FB_GHOST_LN_UPPER_BINS + (j - FB_GHOST_LN_LOWER_FIRST);
+    // n = (2^84 + hi 2^32 - (2^84 + 2^52)) + (2^52 + lo).
+    const double d = (__hiloint2double(0x45300000, (int)(n >> 32)) - 0x1.00000001p84) +
+                     __hiloint2double(0x43300000, (int)(uint32_t)n);
+    const int dh = __double2hiint(d);
+    int mh = (dh & 0xfffff) | 0x3ff00000;
+    int eb = dh >> 20;                                        // e + 1023 + 53
+    const bool upper = __hiloint2double(mh, __double2loint(d)) > 1.4142135623730951;
+    if (upper) { mh -= 0x100000; eb += 1; }                   // m / 2
+    const double m = __hiloint2double(mh, __double2loint(d));
+    const int j = (mh >> 12) & 0xff;
+    const int idx = upper ? FB_GHOST_LN_UPPER_BINS + (j - FB_GHOST_LN_LOWER_FIRST) : j;
+    const double e = __hiloint2double(0x43300000, eb) - (0x1p52 + 1076.0);
     const double inv = lnt[2 * idx], lninv = lnt[2 * idx + 1];
     const double r = fma(m, inv, -1.0);
     double p = -1.0 / 8.0;
@@ -86,8 +94,8 @@ __device__ __forceinline__ double ln_u53(uint64_t n, const double* __restrict__ 
     p = fma(p, r, 1.0 / 3.0);
     p = fma(p, r, -0.5);
     const double l1p = fma(r * r, p, r);
-    const double hi = fma((double)e, FB_GHOST_LN2_HI, lninv);
-    const double lo = fma((double)e, FB_GHOST_LN2_LO, l1p);
+    const double hi = fma(e, FB_GHOST_LN2_HI, lninv);
+    const double lo = fma(e, FB_GHOST_LN2_LO, l1p);
     return hi + lo;
 }
 
@@ -96,8 +104,9 @@ __device__ __forceinline__ double ln_u53(uint64_t n, const double* __restrict__ 
 // 2 pi 2^-9).
 __device__ __forceinline__ void cos_sin_2pi(uint64_t b, const double* __restrict__ trig, double& c, double& s) {
     const int j = (int)(b >> 45);
-    const long long f = (long long)(b & ((1ull << 45) - 1)) - (1ll << 44);
-    const double a = ((double)f * 0x1.0p-53) * FB_GHOST_TWO_PI;
+    // The low 45 bits of b less 2^44.
+    const double f = __hiloint2double(0x43300000 | ((int)(b >> 32) & 0x1fff), (int)(uint32_t)b) - 0x1.01p52;
+    const double a = f * (0x1.0p-53 * FB_GHOST_TWO_PI);       // scaling by 2^-53 rounds nothing
     const double a2 = a * a;
     double ps = fma(a2, -1.0 / 5040.0, 1.0 / 120.0);
     ps = fma(ps, a2, -1.0 / 6.0);
