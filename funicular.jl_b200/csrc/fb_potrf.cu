@@ -30,7 +30,8 @@ template <FactorStore S>
 __global__ void __launch_bounds__(POTRF_THREADS, 1)
 potrf_kernel(const z64* __restrict__ G, int64_t ldg, int k, int64_t N,
              z64* __restrict__ U, int64_t ldu, z64* __restrict__ gwork,
-             ChainStatus* st, int pass, int gate, double forced_u, TrsmPlan* plan, double* __restrict__ frag) {
+             ChainStatus* st, int pass, int gate, double forced_u, TrsmPlan* plan, double* __restrict__ frag,
+             const z64* Rin, int64_t ldrin, z64* Rout, int64_t ldrout) {
     if (gated_off(st, gate)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red_scratch[33];
@@ -58,6 +59,19 @@ potrf_kernel(const z64* __restrict__ G, int64_t ldg, int k, int64_t N,
 
     for (int j = warp; j < k; j += nwarps)
         for (int i = lane; i < k; i += 32) U[i + (int64_t)j * ldu] = (i <= j) ? at(i, j) : zmake(0.0, 0.0);
+    if (Rout) {
+        // R = U Rin (U without Rin) over the caller's U, from the factor held
+        // here: what the stores above left there is not read again.
+        __syncthreads();
+        for (int j = warp; j < k; j += nwarps)
+            for (int i = lane; i < k; i += 32) {
+                z64 acc = zmake(0.0, 0.0);
+                if (!Rin && i <= j) acc = at(i, j);
+                if (Rin)
+                    for (int m = i; m <= j; ++m) zmac(acc, at(i, m), Rin[m + (int64_t)j * ldrin]);
+                Rout[i + (int64_t)j * ldrout] = acc;
+            }
+    }
     if (S == STORE_PLAN && plan) {
         __syncthreads();
         z64* Xs = W + TR_KMAX * LD;
@@ -149,15 +163,17 @@ int compose_r_enqueue(z64* R, int64_t ldr, int k, const z64* U1, int64_t ldu1, c
 size_t potrf_gwork_bytes(int k) { return k > POTRF_PACKED_MAX_K ? (size_t)k * k * sizeof(z64) : 0; }
 
 // plan and frag, when given (k <= 64 only), also receive the solve plan of U:
-// what trsm_prepare_enqueue would make of it.
-int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t ldu, z64* gwork,
-                  ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u, TrsmPlan* plan,
-                  double* frag) {
+// what trsm_prepare_enqueue would make of it. Rout, when given, receives U Rin
+// (U without Rin) from the same launch.
+static int potrf_launch(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t ldu, z64* gwork,
+                        ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u, TrsmPlan* plan,
+                        double* frag, const z64* Rin, int64_t ldrin, z64* Rout, int64_t ldrout) {
 #define FB_POTRF(store, smem)                                                                                  \
     do {                                                                                                       \
         FB_ALLOW_SMEM(potrf_kernel<store>, smem);                                                              \
         potrf_kernel<store><<<1, POTRF_THREADS, (smem), stream>>>(G, ldg, k, N, U, ldu, gwork, st, pass, gate, \
-                                                                  forced_u, plan, frag);                       \
+                                                                  forced_u, plan, frag, Rin, ldrin, Rout,      \
+                                                                  ldrout);                                     \
     } while (0)
     if (k <= TR_KMAX) FB_POTRF(STORE_PLAN, (size_t)2 * TR_KMAX * TR_PREP_LD * sizeof(z64));
     else if (k <= POTRF_PACKED_MAX_K) FB_POTRF(STORE_PACKED, (size_t)k * (k + 1) / 2 * sizeof(z64));
@@ -165,6 +181,13 @@ int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t l
 #undef FB_POTRF
     FB_LAUNCHED("potrf_kernel");
     return FB_OK;
+}
+
+int potrf_enqueue(const z64* G, int64_t ldg, int k, int64_t N, z64* U, int64_t ldu, z64* gwork,
+                  ChainStatus* st, int pass, int gate, cudaStream_t stream, double forced_u, TrsmPlan* plan,
+                  double* frag) {
+    return potrf_launch(G, ldg, k, N, U, ldu, gwork, st, pass, gate, stream, forced_u, plan, frag, nullptr, 0, nullptr,
+                        0);
 }
 
 }  // namespace fb
@@ -209,11 +232,14 @@ static int potrf_call(fb_z128* U, int64_t ldu, const fb_z128* G, int64_t ldg, in
     z64* gwork = reinterpret_cast<z64*>(static_cast<char*>(workspace) + align_up(sizeof(ChainStatus), 256));
     FB_CUDA(cudaMemsetAsync(st, 0, sizeof(ChainStatus), stream), "cudaMemsetAsync");
     z64* Uz = reinterpret_cast<z64*>(U);
-    FB_TRY(potrf_enqueue(reinterpret_cast<const z64*>(G), ldg, k, N, Uz, ldu, gwork, st, 1, GATE_ALWAYS, stream, forced_u,
-                         nullptr, nullptr));
-    if (Rout)
-        FB_TRY(compose_r_enqueue(reinterpret_cast<z64*>(Rout), ldrout, k, reinterpret_cast<const z64*>(Rin), ldrin, Uz,
-                                 ldu, nullptr, 0, st, 0, stream));
+    const z64* Ri = reinterpret_cast<const z64*>(Rin);
+    z64* Ro = reinterpret_cast<z64*>(Rout);
+    // The composition's blocks read U while others write R, so where the two
+    // share memory the factor's own CTA forms the product.
+    const bool shared = Ro && Uz < Ro + ((int64_t)(k - 1) * ldrout + k) && Ro < Uz + ((int64_t)(k - 1) * ldu + k);
+    FB_TRY(potrf_launch(reinterpret_cast<const z64*>(G), ldg, k, N, Uz, ldu, gwork, st, 1, GATE_ALWAYS, stream, forced_u,
+                        nullptr, nullptr, Ri, ldrin, shared ? Ro : nullptr, ldrout));
+    if (Ro && !shared) FB_TRY(compose_r_enqueue(Ro, ldrout, k, Ri, ldrin, Uz, ldu, nullptr, 0, st, 0, stream));
     ChainStatus host{};
     FB_CUDA(cudaMemcpyAsync(&host, st, sizeof host, cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync");
     FB_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");

@@ -193,8 +193,9 @@ int fb_zgemm_right(fb_z128* dst, int64_t ldd, const fb_z128* A, int64_t lda,
  * with U^H U = G, reading G's upper triangle. When G is not positive
  * definite it factors G + s I with s = 11 N k eps(Float64) ||G||_F instead.
  * If Rin is non-NULL, Rout <- U * Rin (the R2 * R product of
- * src/panelblas.jl:133,136); Rout must not alias Rin. U and Rout are written
- * in full, zeros below the diagonal. Synchronizes `queue` and reports:
+ * src/panelblas.jl:133,136); Rout must not alias Rin, it may lie over U (which
+ * it then replaces). U and Rout are written in full, zeros below the diagonal.
+ * Synchronizes `queue` and reports:
  * *shifted = 1 if the shift was taken, *shift = s. Returns FB_ENOTSPD when
  * even G + s I fails. workspace: fb_zpotrf_workspace_size bytes. */
 int fb_zpotrf_workspace_size(int k, size_t* bytes);

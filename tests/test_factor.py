@@ -59,3 +59,26 @@ def test_a_failing_pivot_is_found_in_every_block(fb, backend):
         with pytest.raises(fb.NotPositiveDefinite):
             fb.kernels.cholesky_upper_device(backend, backend.todevice(np.asfortranarray(G)), 10, k,
                                              backend.alloc_device(np.complex128, (k, k)))
+
+
+@pytest.mark.parametrize("k", [1, 9, 64, 65, 160, 161, 200])
+@pytest.mark.parametrize("forced", [None, 2.0 ** -53])
+def test_r_may_take_the_place_of_u(fb, backend, k, forced):
+    # Only Rin must not alias Rout: R = U Rin written over U itself, or over
+    # memory that U's columns run through, holds what separate arrays hold.
+    # Two sums of at most k products in different orders: 4 k eps each.
+    rng = np.random.default_rng(200 + k)
+    G, Rin = gram(rng, k, 1e3), np.triu(randmatrix(rng, k, k))
+    dev = lambda a: backend.todevice(np.asfortranarray(a))
+    factor = lambda U, R: fb.kernels.cholesky_upper_device(backend, dev(G), 1000, k, U, dev(Rin), R, forced)
+    U, R = backend.alloc_device(np.complex128, (k, k)), backend.alloc_device(np.complex128, (k, k))
+    factor(U, R)
+    u, r = U.to_host(), R.to_host()
+    bound = 8 * k * EPS * np.linalg.norm(u) * np.linalg.norm(Rin)
+    same = backend.alloc_device(np.complex128, (k, k))
+    factor(same, same)
+    assert np.linalg.norm(same.to_host() - r) <= bound
+    both = backend.alloc_device(np.complex128, (k + 1, k))     # U from the first row on, R from the second
+    at = lambda row: fb.DeviceMatrix(both.ptr + 16 * row, (k, k), both.ld, np.dtype(np.complex128), both)
+    factor(at(0), at(1))
+    assert np.linalg.norm(both.to_host()[1:] - r) <= bound
