@@ -722,8 +722,18 @@ static GramShape gram_plan(int64_t rows, int kA, int kB, bool hermitian) {
     return gram_shape(rows, kA, kB, hermitian ? 1 : 0, gram_ctas_per_sm(rows, kA, kB, hermitian));
 }
 
+// The workspace of a split Gram: the split's own layout, whose partial tiles
+// share their memory with those of the FP64 kernels behind it.
+static size_t split_gram_workspace_bytes(const SplitShape& ss, const GramShape& sh) {
+    const SplitLayout L = split_layout(ss);
+    return std::max(L.total, L.partial + gram_workspace_bytes(sh));
+}
+
+// The scratch of fb_zgram_static.
+constexpr size_t GRAM_STATIC_SCRATCH_BYTES = (size_t)32 << 20;
+
 // Whether the Gram of this shape runs in the split form (fb_ozaki_gram.cu).
-// Two things draw the lines.
+// Three things draw the lines.
 // Accuracy: the slices' error relative to ||a_i|| ||b_j|| falls with the rows
 // (entries are cut at 2^-51 of their column's scale), that of the FP64 kernels
 // does not; the split form is taken where its is no larger. Gaussian entries,
@@ -743,19 +753,23 @@ static GramShape gram_plan(int64_t rows, int kA, int kB, bool hermitian) {
 //   36 blocks: 48 x 48, 1e5 rows 72 / 82, 4.1e5 rows 242 / 234;
 //   40 blocks (where the FP64 kernel has eight a warp) and more: 64 x 36, 6e4
 //   rows 82 / 61; 64 x 64, 1e5 rows 113 / 82.
+// Scratch: the split form's statistics and summed tiles come on top of the
+// partial tiles. Where they alone would take the Gram past what
+// fb_zgram_static holds (A === B with 321 to 384 columns, products of some 255
+// tiles and more), both entry points stay with the FP64 kernels, so that every
+// Gram that fits keeps fitting, with the same bits from either.
 static bool gram_takes_split(int64_t rows, int kA, int kB, bool hermitian) {
     if (rows > ((int64_t)1 << 30)) return false;   // the tile loads' 32-bit coordinates
-    if (hermitian) return kA > 40 && rows >= (kA > 48 ? 300000 : 500000);
-    const int a = kA < G_TILE ? kA : G_TILE, b = kB < G_TILE ? kB : G_TILE;
-    const int blocks = ((a + 7) / 8) * ((b + 7) / 8);
-    return blocks >= 36 && rows >= (blocks >= 40 ? 250000 : 400000);
-}
-
-// The workspace of a split Gram: the split's own layout, whose partial tiles
-// share their memory with those of the FP64 kernels behind it.
-static size_t split_gram_workspace_bytes(const SplitShape& ss, const GramShape& sh) {
-    const SplitLayout L = split_layout(ss);
-    return std::max(L.total, L.partial + gram_workspace_bytes(sh));
+    if (hermitian) {
+        if (kA <= 40 || rows < (kA > 48 ? 300000 : 500000)) return false;
+    } else {
+        const int a = kA < G_TILE ? kA : G_TILE, b = kB < G_TILE ? kB : G_TILE;
+        const int blocks = ((a + 7) / 8) * ((b + 7) / 8);
+        if (blocks < 36 || rows < (blocks >= 40 ? 250000 : 400000)) return false;
+    }
+    const GramShape sh = gram_plan(rows, kA, kB, hermitian);
+    return split_gram_workspace_bytes(split_shape(rows, kA, kB, hermitian), sh) <= GRAM_STATIC_SCRATCH_BYTES ||
+           gram_workspace_bytes(sh) > GRAM_STATIC_SCRATCH_BYTES;
 }
 
 static SplitGate split_gate(const SplitShape& ss, const void* workspace, bool strict) {
@@ -927,7 +941,6 @@ int ozaki_gram_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, int64_t r
 // GPU that loads the library holds these bytes until the process exits. The
 // partial tiles it holds are written by each call before that call reads
 // them, so nothing in it has to start at zero.
-constexpr size_t GRAM_STATIC_SCRATCH_BYTES = (size_t)32 << 20;
 static __device__ __align__(256) unsigned char g_gram_static_scratch[GRAM_STATIC_SCRATCH_BYTES];
 
 // The device address of g_gram_static_scratch on the current device. Host

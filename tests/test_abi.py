@@ -206,3 +206,22 @@ def test_static_gram_scratch_holds_every_gram_of_at_most_128_columns(fb):
                                  ctypes.byref(need))
                     worst = max(worst, need.value)
     assert worst <= 32 << 20
+
+
+@pytest.mark.parametrize("kA,kB,herm,line", [(321, 321, 1, 300_000), (384, 384, 1, 300_000), (1024, 1024, 0, 250_000),
+                                             (1000, 1400, 0, 250_000), (2048, 1024, 0, 250_000)])
+def test_the_split_form_never_takes_a_gram_past_the_static_scratch(fb, kA, kB, herm, line):
+    """Wide, tall Grams run in the split form from `line` rows on, whose scratch
+    is larger. One that fits fb_zgram_static's 32 MiB below the line fits it
+    above, where the partial tiles alone are no larger."""
+    if fb._lib.device_count() > 0:
+        pytest.skip("the sizes are stated for the 148 SMs the library assumes without a device")
+
+    def need(rows):
+        out = ctypes.c_size_t(0)
+        fb._lib.call("fb_zgram_workspace_size", ctypes.c_int64(rows), kA, kB, herm, ctypes.byref(out))
+        return out.value
+
+    assert need(line - 1) <= 32 << 20
+    for rows in (line, line + 1, 10 * line, 100 * line):
+        assert need(rows) <= 32 << 20

@@ -69,6 +69,18 @@ def test_static_scratch_matches_the_workspace_entry_point(fb, backend, rows, kA,
         np.testing.assert_array_equal(got.to_host(), expect.to_host())
 
 
+def test_static_scratch_takes_wide_tall_grams(fb, backend):
+    # Six tiles a side: the partial tiles fill the scratch all but 0.5 MiB.
+    rng = np.random.default_rng(11)
+    A = np.asfortranarray(randmatrix(rng, 300_000, 321))
+    Ad = backend.todevice(A)
+    expect, got = backend.alloc_device(np.complex128, (321, 321)), backend.alloc_device(np.complex128, (321, 321))
+    gram_with_workspace(fb, backend, expect, Ad, Ad, 1.0, 0.0)
+    gram_static(fb, got, Ad, Ad, 1.0, 0.0)
+    fb._lib.call("fb_sync_all")
+    np.testing.assert_array_equal(got.to_host(), expect.to_host())
+
+
 def test_static_scratch_call_allocates_no_device_memory(fb, backend):
     import torch
 
