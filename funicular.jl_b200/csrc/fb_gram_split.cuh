@@ -25,11 +25,11 @@ struct SplitShape {
 };
 
 // What a CTA reports about its chunk: per input column (A's 64, then B's) the
-// last scale exponent and the sum of squares.
+// last scale exponent and the sum of squares, and what is wrong with it.
 struct SplitStat {
     double sumsq[128];
     int E[128];
-    int invalid;
+    int flags;           // SPLIT_INVALID, SPLIT_INACCURATE
     int pad[3];
 };
 

@@ -95,6 +95,7 @@ struct Cfg {
     static constexpr int EPOCH_STAGES = (FULL ? 8192 : 12288) / ROWS;
     struct Stage {                                             // of the stage a group is working on
         uint32_t colmax[64 * SIDES];                           // slicers: high words of the column maxima
+        uint16_t colmin[64 * SIDES];                           // and the upper halves of those of the column minima
         int E[64 * SIDES], Eold[64 * SIDES];                   // decider: scales of this stage and the one before
         int fresh, epoch;
         int mma_fresh;                                         // fresh, kept by the slicers until the MMAs are issued
@@ -155,16 +156,23 @@ __device__ __forceinline__ void slice_words(const uint64_t (&y)[4], uint32_t (&w
     w[6] = __byte_perm(a01, a23, 0x5410) ^ 0x80808080u;  // byte 0
 }
 
-// The largest high word of |x| over eight values, taken as single-precision
-// magnitudes, which order like the words themselves and whose comparison
-// drops the sign for free. A word past single precision's range (|x| >= 2^1017,
-// Inf, NaN) propagates as a NaN, 0x7FFFFFFF.
-__device__ __forceinline__ uint32_t max_hi(const double (&v)[8]) {
-    float m = 0.0f;
+// The largest and the smallest high word over four complex values, each
+// counting by the larger of its parts, taken as single-precision magnitudes,
+// which order like the words themselves and whose comparison drops the sign for
+// free. A word past single precision's range (|x| >= 2^1017, Inf, NaN)
+// propagates to the largest as a NaN, 0x7FFFFFFF.
+__device__ __forceinline__ void range_hi(const double (&v)[8], uint32_t& largest, uint32_t& smallest) {
+    float m[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e)
-        asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(fabsf(__int_as_float(__double2hiint(v[e])))));
-    return (uint32_t)__float_as_int(m);
+    for (int e = 0; e < 4; ++e)
+        asm("max.NaN.f32 %0, %1, %2;" : "=f"(m[e])
+            : "f"(fabsf(__int_as_float(__double2hiint(v[2 * e])))),
+              "f"(fabsf(__int_as_float(__double2hiint(v[2 * e + 1])))));
+    float mx = m[0];
+#pragma unroll
+    for (int e = 1; e < 4; ++e) asm("max.NaN.f32 %0, %0, %1;" : "+f"(mx) : "f"(m[e]));
+    largest = (uint32_t)__float_as_int(mx);
+    smallest = (uint32_t)__float_as_int(fminf(fminf(m[0], m[1]), fminf(m[2], m[3])));
 }
 
 // What an operand's K rows are made of, from a complex entry (re, im).
@@ -393,9 +401,11 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 return true;
             };
             auto publish = [&](int s) {
+                uint32_t mn[NC];
 #pragma unroll
                 for (int n = 0; n < NC; ++n) {
-                    uint32_t mx = max_hi(v[n]);
+                    uint32_t mx;
+                    range_hi(v[n], mx, mn[n]);
                     if (mx == 0) {
 #pragma unroll
                         for (int e = 0; e < 8; ++e) mx |= __double2loint(v[n][e]) != 0 ? 1u : 0u;
@@ -403,6 +413,14 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                     mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
                     mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
                     if (i == 0) stage.colmax[64 * SIDE + m0 + 8 * n] = mx;
+                }
+                // Both columns' minima at once, their words' upper halves.
+                uint32_t low = __byte_perm(mn[0], mn[1], 0x7632);
+                low = __vminu2(low, __shfl_xor_sync(0xffffffffu, low, 1));
+                low = __vminu2(low, __shfl_xor_sync(0xffffffffu, low, 2));
+                if (i == 0) {
+                    stage.colmin[64 * SIDE + m0] = (uint16_t)low;
+                    stage.colmin[64 * SIDE + m0 + 8] = (uint16_t)(low >> 16);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&mx_full[g]);
@@ -532,8 +550,10 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         // Lane l decides input columns l, l + 32, ... (A's 0-63, then B's).
         // |x| < 2^E (1 - 2^-7) in terms of the high word of x; while the
         // scale is unset every normal number is past it.
-        constexpr int NC = C::COLUMNS / 32;
-        int E[NC];
+        // level[x][j] counts the stages whose smallest entry is 2^(E - 8 + j) or
+        // more, by the scale of the time; the levels move down as it grows.
+        constexpr int NC = C::COLUMNS / 32, LEVELS = 7;
+        int E[NC], level[NC][LEVELS] = {};
         uint32_t limit[NC];
         bool tiny[NC], bad = false;
 #pragma unroll
@@ -551,10 +571,12 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 break;
             }
             uint32_t mx[NC];
+            int low[NC];
             bool over[NC], mine = false;
 #pragma unroll
             for (int x = 0; x < NC; ++x) {
                 mx[x] = stage.colmax[32 * x + lane];
+                low[x] = (int)(stage.colmin[32 * x + lane] >> 4) - 1023;
                 over[x] = mx[x] >= limit[x];
                 if (mx[x] >= 0x7FF00000u) { bad = true; over[x] = false; }   // Inf, NaN or next to them
                 if (E[x] == SPLIT_E_UNSET && mx[x] != 0 && mx[x] < 0x00100000u) tiny[x] = true;
@@ -568,8 +590,12 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                     if (!over[x]) continue;
                     // The power of two above 1.3 times the maximum, and once
                     // more that while the maximum is that of 16 rows only.
-                    const int spare = E[x] == SPLIT_E_UNSET ? 1 : 0;
+                    const int spare = E[x] == SPLIT_E_UNSET ? 1 : 0, before = E[x];
                     E[x] = (int)((mx[x] + ROUND_UP) >> 20) - 1023 + 1 + spare;
+#pragma unroll 1
+                    for (int up = min(E[x] - before, LEVELS); up > 0; --up)
+#pragma unroll
+                        for (int j = 0; j < LEVELS; ++j) level[x][j] = j + 1 < LEVELS ? level[x][j + 1] : 0;
                     // The limit's exponent stays in range: a scale past it is
                     // refused afterwards by split_sum_kernel anyway.
                     limit[x] = ((uint32_t)min(max(E[x] - 1 + 1023, 1), 0x7FE) << 20) | 0xFC000u;
@@ -589,17 +615,23 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive(&sc_full[g]);
             if (++g == C::GROUPS) { g = 0; ph ^= 1u; }
+#pragma unroll
+            for (int x = 0; x < NC; ++x)
+#pragma unroll
+                for (int j = 0; j < LEVELS; ++j) level[x][j] += E[x] != SPLIT_E_UNSET && low[x] - (E[x] - 8) >= j;
         }
-        if (bad) *bad_flag = 1;
+        if (bad) atomicOr(bad_flag, SPLIT_INVALID);
 #pragma unroll
         for (int x = 0; x < NC; ++x) {
+            // Fewer than 5/8 of the stages within 2^-8 of the scale.
+            if (E[x] != SPLIT_E_UNSET && 8 * level[x][0] < 5 * nstages) atomicOr(bad_flag, SPLIT_INACCURATE);
             stat->E[32 * x + lane] = E[x] == SPLIT_E_UNSET && tiny[x] ? SPLIT_E_TINY : E[x];
         }
     }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    if (threadIdx.x == 0) stat->invalid = (*abort_flag || *bad_flag) ? 1 : 0;
+    if (threadIdx.x == 0) stat->flags = (*abort_flag ? SPLIT_INVALID : 0) | *bad_flag;
     if (warp == 0) umma::tmem_dealloc(taddr, TMEM_COLS);
     // The columns' sums of squares, over the four lanes of a column, then the
     // groups in order (the ring is free by now).
@@ -641,6 +673,20 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // A spike that dwarfs the rest of its column fails it, as do Inf and NaN, a
 // scale whose products could leave the FP64 range, and a wait that gave up:
 // the caller then computes the tile in FP64 instead.
+//
+// An error that is small against ||a_i|| ||a_j|| can still be all of an entry
+// to which only small parts of the columns contribute (rows graded one way in
+// one column and the other way in another, say). FP64 sums are off by little
+// against sum_r |a_ri| |a_rj|, and so the chunks report whether every column
+// has, in at least 5/8 of the stages, all its entries within 2^-8 of its
+// scale (entries count by the larger of their parts; a column that is zero
+// throughout a chunk is exact there). Any two columns then share a quarter of
+// the stages in which both have, so the sum is at least
+// n / 4 2^(E_i + E_j - 16) over a chunk's n rows. Rows alternating by 2^-5, the
+// two columns in opposite phase, pass: entries are then off by up to 2e-16 of
+// their sum at 3e5 rows, as FP64 sums are; alternating by 2^-48, refused, they
+// had no correct digit. Chunks of Gaussian rows pass with 9 of 10 stages or
+// more, whatever scale their first 16 rows set.
 constexpr int SUM_THREADS = 512;
 
 __global__ void __launch_bounds__(SUM_THREADS)
@@ -687,7 +733,7 @@ split_sum_kernel(SplitShape sh, int64_t rows, const double* __restrict__ partial
     double s = 0.0;
     const SplitStat* x = stats + (size_t)tile * sh.nchunks;
     for (int c = tid; c < sh.nchunks; c += SUM_THREADS)
-        if (x[c].invalid) mine |= SPLIT_INVALID;
+        mine |= x[c].flags;
     if (m < columns)
         for (int c0 = part; c0 < sh.nchunks; c0 += 40) {
             double v[10];
@@ -734,7 +780,9 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, int64_t rows, co
 
 }  // namespace split
 
-// One chunk per SM for the launch with fewer tiles, in whole stages.
+// One chunk per SM for the launch with fewer tiles, in whole stages; of long
+// chunks the last one is long too, since the verdict on a column is taken from
+// each chunk's stages.
 SplitShape split_shape(int64_t rows, int kA, int kB, bool hermitian) {
     SplitShape sh{};
     sh.nt_a = (kA + 63) / 64;
@@ -745,7 +793,9 @@ SplitShape split_shape(int64_t rows, int kA, int kB, bool hermitian) {
     if (hermitian && sh.nt_a > 1) smallest = std::min(sh.nt_a, sh.nt_a * (sh.nt_a - 1) / 2);
     const int64_t stages = (rows + SPLIT_STAGE_ROWS - 1) / SPLIT_STAGE_ROWS;
     const int64_t target = std::max<int64_t>(1, sm_count() / smallest);
-    sh.chunk_rows = std::max<int64_t>(1, (stages + target - 1) / target) * SPLIT_STAGE_ROWS;
+    int64_t per = std::max<int64_t>(1, (stages + target - 1) / target);
+    while (per >= 96 && stages % per != 0 && stages % per < 64) ++per;
+    sh.chunk_rows = per * SPLIT_STAGE_ROWS;
     sh.nchunks = (int)((rows + sh.chunk_rows - 1) / sh.chunk_rows);
     return sh;
 }

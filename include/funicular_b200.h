@@ -138,6 +138,11 @@ int fb_convert_copy(void* dst, int dst_type, int64_t ldd,
  * conjugate mirror, so the result is Hermitian to the bit. The reduction
  * order depends only on rows, kA, kB and the device, never on the caller's
  * pipelining, so repeated calls give identical bits.
+ * Accuracy: that of FP64 inner products, entry by entry: an error of a few eps
+ * sum_r |a_ri| |b_rj|, growing like the square root of the rows at most. Tall,
+ * wide products run on the integer tensor cores (see fb_zgram_tc) where the
+ * device finds that this holds, columns graded over their rows included in
+ * what it looks at, and on the FP64 tensor cores otherwise.
  * workspace must hold fb_zgram_workspace_size bytes of device memory. */
 int fb_zgram_workspace_size(int64_t rows, int kA, int kB, int hermitian, size_t* bytes);
 int fb_zgram(fb_z128* C, int64_t ldc,

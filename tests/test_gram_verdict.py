@@ -1,0 +1,112 @@
+"""What the device's verdict on the split Gram (fb_ozaki_gram.cu) accepts and
+refuses, read from the workspace, and the entries that come out either way,
+each against its own sum_r |a_ri| |b_rj| in extended precision.
+
+Accepted sums: each of the two terms of the verdict's bound is below
+2^-54 ||a|| ||b||, and the 148 chunk sums are added in runs of 19 and 8, so 8 eps
+||a|| ||b|| covers them (a lost slice costs 20 eps or more). Refused ones are FP64
+sums of N terms, which round as a random walk: 4 eps sqrt(N) of sum |a| |b|."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from conftest import randmatrix
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+PAIRS = [(0, 0), (0, 1), (1, 2), (3, 8), (5, 40), (17, 30), (20, 21), (35, 34)]
+
+
+def gram(fb, backend, A, B=None):
+    """G and the verdict of every output tile (the first words of the workspace)."""
+    vp = ctypes.c_void_p
+    Ad = backend.todevice(np.asfortranarray(A))
+    Bd = Ad if B is None else backend.todevice(np.asfortranarray(B))
+    need = ctypes.c_size_t(0)
+    fb._lib.call("fb_zgram_workspace_size", ctypes.c_int64(Ad.rows), Ad.cols, Bd.cols, int(B is None),
+                 ctypes.byref(need))
+    ws = backend.todevice(np.full((need.value // 16 + 1, 1), np.nan + 0j, order="F"))
+    C = backend.alloc_device(np.complex128, (Ad.cols, Bd.cols))
+    fb._lib.check(fb._lib.load().fb_zgram(vp(C.ptr), C.ld, vp(Ad.ptr), Ad.ld, vp(Bd.ptr), Bd.ld, Ad.rows, Ad.cols,
+                                          Bd.cols, fb._lib.z128(1.0), fb._lib.z128(0.0), vp(ws.ptr), need.value, None),
+                  "fb_zgram")
+    fb._lib.call("fb_sync_all")
+    na, nb = -(-Ad.cols // 64), -(-Bd.cols // 64)
+    words = ws.to_host().view(np.int32).ravel()
+    return C.to_host(), words[:na * (na + 1) // 2 if B is None else na * nb]
+
+
+def errors(G, A, B, pairs):
+    """Largest |G_ij - exact| over the pairs, against ||a|| ||b|| and against sum |a| |b|."""
+    L = np.longdouble
+    norm = size = 0.0
+    for i, j in pairs:
+        ar, ai, br, bi = (np.asarray(v, dtype=L) for v in (A[:, i].real, A[:, i].imag, B[:, j].real, B[:, j].imag))
+        d = np.hypot(float(G[i, j].real - ((ar * br).sum() + (ai * bi).sum())),
+                     float(G[i, j].imag - ((ar * bi).sum() - (ai * br).sum())))
+        norm = max(norm, d / (np.linalg.norm(A[:, i]) * np.linalg.norm(B[:, j])))
+        size = max(size, d / (np.abs(A[:, i]) @ np.abs(B[:, j])))
+    return norm, size
+
+
+def gaussian(rng, N, k):
+    return rng.standard_normal((N, k)) + 1j * rng.standard_normal((N, k))
+
+
+def flat(kind, rng, N, k):
+    r, j = np.arange(N)[:, None] / N, np.arange(1, k + 1)[None, :]
+    if kind == "gaussian":
+        return gaussian(rng, N, k)
+    if kind == "uniform":
+        return randmatrix(rng, N, k)
+    if kind == "waves":
+        return np.exp(2j * np.pi * j * r)
+    if kind == "modes":
+        return np.sin(np.pi * j * r) + 1j * np.cos(np.pi * j * r)
+    X = gaussian(rng, N, k)     # "zeros": a zero column, and one that starts late, on a chunk's first row
+    X[:, 3] = 0
+    X[:2032 * 70, 8] = 0
+    return X
+
+
+@pytest.mark.parametrize("kind", ["gaussian", "uniform", "waves", "modes", "zeros"])
+@pytest.mark.parametrize("N,kA,kB", [(300_000, 64, None), (250_007, 64, 64), (300_017, 130, None), (250_001, 100, 64)])
+def test_flat_columns_are_accepted(fb, backend, kind, N, kA, kB):
+    rng = np.random.default_rng(N + kA)
+    A = flat(kind, rng, N, kA)
+    B = A if kB is None else flat(kind, rng, N, kB)
+    G, verdict = gram(fb, backend, A, None if kB is None else B)
+    if kind != "zeros" or (N, kA, kB) == (300_000, 64, None):
+        assert not verdict.any()
+    pairs = [p for p in PAIRS + [(kA - 1, B.shape[1] - 2), (kA - 1, 2)] if 3 not in p]
+    assert errors(G, A, B, pairs)[0] <= 8 * EPS
+
+
+def graded(kind, rng, N, k, first):
+    X, r = gaussian(rng, N, k), np.arange(N)
+    odd = (np.arange(k) + first) % 2 == 1
+    low = {"halves": r < N // 2, "runs": r % 64 < 32, "rows": r % 2 == 0}.get(kind)
+    if low is not None:          # every other column small where the others are large
+        return X * np.where(low[:, None] ^ odd, 2.0 ** -48, 1.0)
+    if kind == "sparse":
+        return X * (rng.random((N, k)) < 0.05)
+    if kind == "spike":          # where the others are zero
+        X[77] = 0
+        X[77, 3] = 2.0 ** 60
+        return X
+    if kind == "range":
+        return X * 2.0 ** 460
+    raise AssertionError(kind)
+
+
+@pytest.mark.parametrize("kind", ["halves", "runs", "rows", "sparse", "spike", "range"])
+@pytest.mark.parametrize("N,kA,kB", [(300_000, 64, None), (250_007, 64, 48), (300_017, 70, None)])
+def test_columns_that_share_no_rows_at_their_scale_are_refused(fb, backend, kind, N, kA, kB):
+    rng = np.random.default_rng(N + kA)
+    A = graded(kind, rng, N, kA, 0)
+    B = A if kB is None else graded(kind, rng, N, kB, 0)
+    G, verdict = gram(fb, backend, A, None if kB is None else B)
+    assert verdict.any()
+    assert errors(G, A, B, PAIRS)[1] <= 4 * EPS * np.sqrt(N)
