@@ -662,11 +662,16 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 //
 // The verdict compares what the slices leave out with what the column weighs.
 // With scale 2^E an entry is off by at most 2^(E - 51) (V: 2^(E - 50)), which
-// reaches G_ij as an error of about 2^(E_j - 50) / sqrt(12) ||a_i||; the
-// products left out (three digit pairs a K row, digits of standard deviation
-// 74) add about sqrt(6 N) 74^2 2^(E_i + E_j - 70). Both stay below
-// 2^-54 ||a_i|| ||a_j||, under the rounding of the FP64 sums themselves, when
-//     ||a_j||^2 >= 4^E_j max(21.4, 0.21 sqrt(N)).
+// reaches G_ij as an error of about 2^(E_j - 50) / sqrt(12) ||a_i||. The
+// products left out, digits of standard deviation 74: in a full tile the six
+// pairs with t + u = 9 over 2 N K rows, sqrt(12 N) 74^2 2^(E_i + E_j - 70); in a
+// folded one three pairs of twice the weight, of which the mean of S_ij and
+// S_ji keeps 1 / sqrt(2): the same. Both stay below 2^-54 ||a_i|| ||a_j||,
+// under the rounding of the FP64 sums themselves, when
+//     ||a_j||^2 >= 4^E_j max(21.4, 0.29 sqrt(N)).
+// These are root mean squares of roundings that do not know of one another; a
+// column of equal entries rounds alike in every row and has been seen off by
+// 2e-15 of the entry (its FP64 sums: 8e-14).
 // The kernel knows ||a_j||^2 from the leading digits, whose rounding can raise
 // it by a third where they are small, so it checks 1.4 times that (N Gaussian
 // rows have at least about 2 N / 576).
@@ -758,7 +763,7 @@ split_sum_kernel(SplitShape sh, int64_t rows, const double* __restrict__ partial
         s = (red[tid] + red[128 + tid]) + (red[256 + tid] + red[384 + tid]);
         E = max(max(redE[tid], redE[128 + tid]), max(redE[256 + tid], redE[384 + tid]));
         if (E != SPLIT_E_UNSET &&
-            !(E >= -450 && E <= 450 && s >= fmax(30.0, 0.3 * sqrt((double)rows)) * pow2(2 * E)))
+            !(E >= -450 && E <= 450 && s >= fmax(30.0, 0.41 * sqrt((double)rows)) * pow2(2 * E)))
             mine |= SPLIT_INACCURATE;
     }
     if (mine) atomicOr(&flags, mine);

@@ -110,3 +110,19 @@ def test_columns_that_share_no_rows_at_their_scale_are_refused(fb, backend, kind
     G, verdict = gram(fb, backend, A, None if kB is None else B)
     assert verdict.any()
     assert errors(G, A, B, PAIRS)[1] <= 4 * EPS * np.sqrt(N)
+
+
+@pytest.mark.parametrize("modulus,accepted", [(0.82, False), (1.05, True)])
+@pytest.mark.parametrize("same", [True, False])
+def test_the_norm_a_scale_asks_for(fb, backend, modulus, accepted, same):
+    # What the slices leave out stays below 2^-54 ||a|| ||b|| from ||a||^2 =
+    # 0.29 sqrt(N) 4^E on, checked with 1.4 times that to spare (0.41). The
+    # entry of 20 sets 2^E = 32: modulus 0.82 has 0.36 sqrt(N) 4^E, 1.05 has 0.59.
+    rng = np.random.default_rng(6)
+    N, k = 300_000, 64
+    wave = lambda: np.exp(2j * np.pi * rng.random((N, k)))
+    A = wave()
+    A[:, 5] *= modulus
+    A[1_000, 5] = 20.0
+    G, verdict = gram(fb, backend, A, None if same else wave())
+    assert bool(verdict.any()) != accepted
