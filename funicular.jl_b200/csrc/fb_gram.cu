@@ -845,21 +845,33 @@ static int dmma_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_
     return FB_OK;
 }
 
-// The partial tiles of chunks [chunk0, chunk1).
-int gram_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
-                          bool hermitian, void* workspace, size_t workspace_bytes, cudaStream_t stream,
-                          const ChainStatus* st, int gate, int chunk0, int chunk1) {
+// The partial tiles of chunks [chunk0, chunk1). screened: see split_partials_enqueue.
+static int partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
+                            bool hermitian, void* workspace, size_t workspace_bytes, cudaStream_t stream,
+                            const ChainStatus* st, int gate, int chunk0, int chunk1, bool screened) {
     const size_t need = gram_workspace_size(rows, kA, kB, hermitian);
     if (workspace_bytes < need || workspace == nullptr) {
         set_error(FB_ENOMEM, "gram: workspace of %zu bytes is smaller than the %zu bytes this shape needs",
                   workspace_bytes, need);
         return FB_ENOMEM;
     }
-    if (gram_takes_split(rows, kA, kB, hermitian))
-        return split_partials_enqueue(A, lda, B, ldb, rows, kA, kB, split_shape(rows, kA, kB, hermitian), workspace,
-                                      stream, st, gate, chunk0, chunk1);
+    if (gram_takes_split(rows, kA, kB, hermitian)) {
+        const SplitShape ss = split_shape(rows, kA, kB, hermitian);
+        if (screened) FB_TRY(split_screen_enqueue(A, lda, B, ldb, rows, kA, ss, workspace, stream, st, gate));
+        return split_partials_enqueue(A, lda, B, ldb, rows, kA, kB, ss, workspace, stream, st, gate, chunk0, chunk1,
+                                      screened, false);
+    }
     return dmma_partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, static_cast<z64*>(workspace), stream, st,
                                  gate, chunk0, chunk1, SplitGate{});
+}
+
+// For rows that arrive piece by piece: no screen has seen them all yet, so the
+// partial tiles are computed whatever they hold.
+int gram_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
+                          bool hermitian, void* workspace, size_t workspace_bytes, cudaStream_t stream,
+                          const ChainStatus* st, int gate, int chunk0, int chunk1) {
+    return partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, workspace, workspace_bytes, stream, st, gate, chunk0,
+                            chunk1, false);
 }
 
 static int reduce_enqueue(z64* C, int64_t ldc, const GramShape& sh, int kA, int kB, const z64* partial, z64 alpha,
@@ -876,9 +888,9 @@ static int reduce_enqueue(z64* C, int64_t ldc, const GramShape& sh, int kA, int 
 // Gram: the sums and their verdict, the FP64 kernels over all rows (which
 // return at once when the verdict accepts the sums), and C from one or the
 // other.
-int gram_reduce_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
-                        int kB, bool hermitian, z64 alpha, z64 beta, void* workspace, cudaStream_t stream,
-                        const ChainStatus* st, int gate) {
+static int sum_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
+                       int kB, bool hermitian, z64 alpha, z64 beta, void* workspace, cudaStream_t stream,
+                       const ChainStatus* st, int gate, bool screened) {
     GramShape sh = gram_plan(rows, kA, kB, hermitian);
     if (hermitian && sh.nchunks > 0) sh.sdiag = folded_sdiag(sh, kA);
     z64* partial = static_cast<z64*>(workspace);
@@ -887,11 +899,20 @@ int gram_reduce_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z6
         const SplitShape ss = split_shape(rows, kA, kB, hermitian);
         split = split_gate(ss, workspace, false);
         partial = reinterpret_cast<z64*>(static_cast<char*>(workspace) + split_layout(ss).partial);
-        FB_TRY(split_sum_enqueue(rows, ss, workspace, stream, st, gate));
+        if (!screened) FB_TRY(split_screen_enqueue(A, lda, B, ldb, rows, kA, ss, workspace, stream, st, gate));
+        FB_TRY(split_sum_enqueue(rows, ss, workspace, stream, st, gate, true));
         FB_TRY(dmma_partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, partial, stream, st, gate, 0, sh.nchunks,
                                      split));
     }
     return reduce_enqueue(C, ldc, sh, kA, kB, partial, alpha, beta, split, stream, st, gate);
+}
+
+// After gram_partials_enqueue over all chunks. The screen runs here, so that
+// rows that came piece by piece give the bits of one call over all of them.
+int gram_reduce_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
+                        int kB, bool hermitian, z64 alpha, z64 beta, void* workspace, cudaStream_t stream,
+                        const ChainStatus* st, int gate) {
+    return sum_enqueue(C, ldc, A, lda, B, ldb, rows, kA, kB, hermitian, alpha, beta, workspace, stream, st, gate, false);
 }
 
 // Shared by fb_zgram and the orthonormalization chain.
@@ -902,10 +923,9 @@ int gram_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, const z64* B, i
     int64_t chunk_rows = 0;
     int nchunks = 0;
     gram_chunks(rows, kA, kB, hermitian, &chunk_rows, &nchunks);
-    FB_TRY(gram_partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, workspace, workspace_bytes, stream, st,
-                                 gate, 0, nchunks));
-    return gram_reduce_enqueue(C, ldc, A, lda, B, ldb, rows, kA, kB, hermitian, alpha, beta, workspace, stream, st,
-                               gate);
+    FB_TRY(partials_enqueue(A, lda, B, ldb, rows, kA, kB, hermitian, workspace, workspace_bytes, stream, st, gate, 0,
+                            nchunks, true));
+    return sum_enqueue(C, ldc, A, lda, B, ldb, rows, kA, kB, hermitian, alpha, beta, workspace, stream, st, gate, true);
 }
 
 // The tensor-core entry points: the split form whatever the shape (k <= 64),
@@ -930,8 +950,8 @@ int ozaki_gram_enqueue(z64* C, int64_t ldc, const z64* A, int64_t lda, int64_t r
         return FB_ENOMEM;
     }
     const SplitShape ss = split_shape(rows, k, k, true);
-    FB_TRY(split_partials_enqueue(A, lda, A, lda, rows, k, k, ss, workspace, stream, st, gate, 0, ss.nchunks));
-    FB_TRY(split_sum_enqueue(rows, ss, workspace, stream, st, gate));
+    FB_TRY(split_partials_enqueue(A, lda, A, lda, rows, k, k, ss, workspace, stream, st, gate, 0, ss.nchunks, false, true));
+    FB_TRY(split_sum_enqueue(rows, ss, workspace, stream, st, gate, false));
     return reduce_enqueue(C, ldc, gram_plan(rows, k, k, true), k, k, nullptr, alpha, beta,
                           split_gate(ss, workspace, true), stream, st, gate);
 }

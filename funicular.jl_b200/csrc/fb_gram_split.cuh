@@ -11,6 +11,7 @@ namespace fb {
 
 constexpr int SPLIT_STAGE_ROWS = 16;              // complex rows per stage; chunks are whole stages
 constexpr int SPLIT_TILE_DOUBLES = 128 * 64;      // a partial or summed tile, column n of it contiguous
+constexpr int SPLIT_SCREEN_PARTS = 4;             // blocks a column of the screen
 constexpr int SPLIT_E_UNSET = -4000;              // scale of a column that has only zeros so far
 constexpr int SPLIT_E_TINY = -3999;               // and of one that has nothing above the subnormals
 constexpr int SPLIT_INVALID = 1;                  // Inf, NaN or a wait that gave up: the sums mean nothing
@@ -20,6 +21,7 @@ struct SplitShape {
     int nt_a, nt_b;      // 64-column tiles of A and of B
     int hermitian;       // folded diagonal tiles first, then the tiles above the diagonal
     int ntiles;
+    int screened;        // columns the screen looks at: A's, and B's if it is another matrix
     int64_t chunk_rows;
     int nchunks;
 };
@@ -34,7 +36,7 @@ struct SplitStat {
 };
 
 struct SplitLayout {
-    size_t verdict, sums, stats, partial, total;  // byte offsets in the workspace
+    size_t verdict, refused, sums, stats, partial, total;  // byte offsets in the workspace
 };
 
 // Tile `x` of a launch over the folded or the full tiles.
@@ -55,12 +57,17 @@ __host__ __device__ inline void split_tile_of(const SplitShape& sh, bool full, i
 
 SplitShape split_shape(int64_t rows, int kA, int kB, bool hermitian);
 SplitLayout split_layout(const SplitShape& sh);
+// The screen over a sample of all rows: which columns go to the FP64 kernels.
+int split_screen_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
+                         const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st, int gate);
 // The partial tiles of chunks [chunk0, chunk1); each depends on its rows alone.
+// screened: nothing, where a screen that ran before refused a column. strict:
+// no FP64 kernels stand behind the sums.
 int split_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
                            const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st, int gate,
-                           int chunk0, int chunk1);
+                           int chunk0, int chunk1, bool screened, bool strict);
 // Sums the partial tiles of every chunk and writes each tile's verdict.
 int split_sum_enqueue(int64_t rows, const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st,
-                      int gate);
+                      int gate, bool screened);
 
 }  // namespace fb

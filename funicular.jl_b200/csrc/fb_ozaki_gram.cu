@@ -234,12 +234,109 @@ __device__ __noinline__ void drain_epoch(uint32_t tmem_lane, const int* EA, cons
     __threadfence_block();
 }
 
+// Whether the screen refused any column; by all threads of a block.
+__device__ __forceinline__ bool screened_off(const int* __restrict__ refused, const SplitShape& sh) {
+    int any = 0;
+    for (int c = threadIdx.x; c < SPLIT_SCREEN_PARTS * sh.screened; c += blockDim.x) any |= refused[c];
+    return __syncthreads_or(any) != 0;
+}
+
+// A look at a sample of every column before its products are formed: 64 rows of
+// every chunk, its first 16, its last 16 and two runs of 16 between them, by
+// SPLIT_SCREEN_PARTS blocks a column (A's, then those of B) that take every
+// SPLIT_SCREEN_PARTS-th chunk. What the verdict would refuse afterwards, or what the
+// slicing is slow on, goes to the FP64 kernels at once. A column is refused
+//   when a quarter of the runs have an entry under 2^-6 of their chunk's
+//   sampled maximum (the verdict asks for 5/8 of the stages within 2^-8 of a
+//   scale of 2.6 to 5.2 times that of the first stage);
+//   when two of a chunk's four runs have one under 2^-10 of it;
+//   when a chunk's later runs exceed its first by 4 or more: a scale set by
+//   the first 16 rows holds 2.6 times their maximum, and each time a column
+//   outgrows its scale the accumulators are drained;
+//   at numbers that are not finite or whose products could leave the range.
+// The choice of the runs depends on the shape alone. Gaussian columns pass with
+// a few runs in a hundred under the line and all but never a fourfold maximum.
+// Latency-bound, hence the four blocks a column: 6.3 us for 64 columns (one
+// block of 512 threads a column: 10). Without it a refused product paid for
+// both forms, and for a drain at every growth. Folded, 2e6 x 64, us, FP64 alone
+// 1075: columns in Gaussian envelopes 6530 -> 1087, heavy-tailed 3130 -> 1090,
+// sin(pi j x) 3190 -> 1090; 3e5 rows, FP64 alone 198: 1780, 1110, 1220 -> 218.
+// Accepted: 585 -> 592 and 133 -> 141.
+constexpr int SCREEN_THREADS = 256;
+
+__global__ void __launch_bounds__(SCREEN_THREADS)
+split_screen_kernel(const z64* __restrict__ A, int64_t lda, const z64* __restrict__ B, int64_t ldb, int64_t rows,
+                    SplitShape sh, int kA, int* __restrict__ refused, const ChainStatus* st, int gate) {
+    if (gated_off(st, gate)) return;
+    constexpr int WARPS = SCREEN_THREADS / 32, BATCH = 5;
+    const int c = blockIdx.x / SPLIT_SCREEN_PARTS, part = blockIdx.x % SPLIT_SCREEN_PARTS;
+    const int nchunks = (sh.nchunks - part + SPLIT_SCREEN_PARTS - 1) / SPLIT_SCREEN_PARTS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const z64* x = c < kA ? A + (int64_t)c * lda : B + (int64_t)(c - kA) * ldb;
+    __shared__ uint32_t most;
+    __shared__ int low, runs, grown;
+    if (threadIdx.x == 0) { most = 0; low = runs = grown = 0; }
+    __syncthreads();
+    uint32_t all = 0;
+    int wlow = 0, wruns = 0, wgrown = 0, wgraded = 0;
+    for (int k0 = warp; k0 < nchunks; k0 += BATCH * WARPS) {
+        z64 v[BATCH][2];
+#pragma unroll
+        for (int q = 0; q < BATCH; ++q) {
+            const int k = SPLIT_SCREEN_PARTS * min(k0 + q * WARPS, nchunks - 1) + part;
+            const int64_t row0 = (int64_t)k * sh.chunk_rows;
+            const int len = (int)min(rows - row0, sh.chunk_rows), last = max(len - SPLIT_STAGE_ROWS, 0);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                // Half a warp a run: the first and one in the first half, then
+                // one in the second half and the last.
+                const int r = 2 * h + (lane >> 4);
+                const uint32_t jump = __umulhi((uint32_t)(4 * k + r) * 2654435761u, (uint32_t)(last / 2));
+                const int off = r == 0 ? 0 : r == 3 ? last : (r - 1) * (last / 2) + (int)jump;
+                v[q][h] = x[row0 + min(off + (lane & 15), len - 1)];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < BATCH; ++q) {
+            if (k0 + q * WARPS >= nchunks) break;
+            uint32_t m[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                m[h] = max((uint32_t)__double2hiint(v[q][h].x) & 0x7FFFFFFFu,
+                           (uint32_t)__double2hiint(v[q][h].y) & 0x7FFFFFFFu);
+            const uint32_t first = __reduce_max_sync(0xffffffffu, lane < 16 ? m[0] : 0u);
+            const uint32_t top = __reduce_max_sync(0xffffffffu, max(m[0], m[1]));
+            if (top == 0) continue;   // a chunk of zeros is exact
+            const uint32_t line = top > (6u << 20) ? top - (6u << 20) : 1u;
+            const uint32_t b0 = __ballot_sync(0xffffffffu, m[0] < line), b1 = __ballot_sync(0xffffffffu, m[1] < line);
+            wlow += ((b0 & 0xFFFFu) != 0) + ((b0 >> 16) != 0) + ((b1 & 0xFFFFu) != 0) + ((b1 >> 16) != 0);
+            wruns += 4;
+            wgrown += top >= first + (2u << 20);
+            const uint32_t deep = top > (10u << 20) ? top - (10u << 20) : 1u;
+            const uint32_t d0 = __ballot_sync(0xffffffffu, m[0] < deep), d1 = __ballot_sync(0xffffffffu, m[1] < deep);
+            wgraded += ((d0 & 0xFFFFu) != 0) + ((d0 >> 16) != 0) + ((d1 & 0xFFFFu) != 0) + ((d1 >> 16) != 0) >= 2;
+            all = max(all, top);
+        }
+    }
+    if (lane == 0) {
+        atomicMax(&most, all);
+        atomicAdd(&low, wlow);
+        atomicAdd(&runs, wruns);
+        atomicAdd(&grown, wgrown + wgraded);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int e = (int)(most >> 20) - 1023;
+        refused[blockIdx.x] = most != 0 && (4 * low > runs || grown > 0 || e < -440 || e > 440);
+    }
+}
+
 template <bool FULL>
 __global__ void __launch_bounds__(Cfg<FULL>::THREADS, 1)
 split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int64_t rows,
                   SplitShape sh, double* __restrict__ partial, SplitStat* __restrict__ stats, const ChainStatus* st,
-                  int gate, int chunk0, int zero) {
+                  int gate, int chunk0, const int* __restrict__ refused, int give_up, int zero) {
     if (gated_off(st, gate)) return;
+    if (refused && screened_off(refused, sh)) return;
     using C = Cfg<FULL>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -562,6 +659,10 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             limit[x] = 0x00100000u;
             tiny[x] = false;
         }
+        // With the FP64 kernels behind it (give_up), a chunk whose scales keep
+        // growing is theirs: the rest of it passes with the scales it has.
+        const int most = 16 + nstages / 256;
+        bool gave_up = false;
         int g = 0, epoch = -1, epoch_start = 0;
         uint32_t ph = 0;
         for (int s = 0; s < nstages; ++s) {
@@ -583,7 +684,8 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 mine = mine || over[x];
                 stage.Eold[32 * x + lane] = E[x];
             }
-            const bool any_over = __any_sync(0xffffffffu, mine);
+            if (give_up && epoch >= most) gave_up = true;
+            const bool any_over = __any_sync(0xffffffffu, mine) && !gave_up;
             if (any_over) {
 #pragma unroll
                 for (int x = 0; x < NC; ++x) {
@@ -601,7 +703,7 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                     limit[x] = ((uint32_t)min(max(E[x] - 1 + 1023, 1), 0x7FE) << 20) | 0xFC000u;
                 }
             }
-            const bool fresh = s == 0 || any_over || s - epoch_start >= C::EPOCH_STAGES;
+            const bool fresh = s == 0 || any_over || (s - epoch_start >= C::EPOCH_STAGES && !gave_up);
             if (fresh) {
                 ++epoch;
                 epoch_start = s;
@@ -621,6 +723,7 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                 for (int j = 0; j < LEVELS; ++j) level[x][j] += E[x] != SPLIT_E_UNSET && low[x] - (E[x] - 8) >= j;
         }
         if (bad) atomicOr(bad_flag, SPLIT_INVALID);
+        if (gave_up) atomicOr(bad_flag, SPLIT_INACCURATE);
 #pragma unroll
         for (int x = 0; x < NC; ++x) {
             // Fewer than 5/8 of the stages within 2^-8 of the scale.
@@ -696,8 +799,13 @@ constexpr int SUM_THREADS = 512;
 
 __global__ void __launch_bounds__(SUM_THREADS)
 split_sum_kernel(SplitShape sh, int64_t rows, const double* __restrict__ partial, const SplitStat* __restrict__ stats,
-                 double* __restrict__ sums, int* __restrict__ verdict, const ChainStatus* st, int gate) {
+                 double* __restrict__ sums, int* __restrict__ verdict, const ChainStatus* st, int gate,
+                 const int* __restrict__ refused) {
     if (gated_off(st, gate)) return;
+    if (refused && screened_off(refused, sh)) {
+        if (blockIdx.x == 128 && threadIdx.x == 0) verdict[blockIdx.y] = SPLIT_INACCURATE;
+        return;
+    }
     __shared__ double red[SUM_THREADS];
     __shared__ int redE[SUM_THREADS];
     __shared__ int flags;
@@ -774,11 +882,11 @@ split_sum_kernel(SplitShape sh, int64_t rows, const double* __restrict__ partial
 template <bool FULL>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mb, int64_t rows, const SplitShape& sh, int ntiles,
                   double* partial, SplitStat* stats, cudaStream_t stream, const ChainStatus* st, int gate, int chunk0,
-                  int chunk1) {
+                  int chunk1, const int* refused, int give_up) {
     using C = Cfg<FULL>;
     FB_ALLOW_SMEM(split_gram_kernel<FULL>, C::SMEM);
     split_gram_kernel<FULL><<<dim3((unsigned)ntiles, (unsigned)(chunk1 - chunk0)), C::THREADS, C::SMEM, stream>>>(
-        ma, mb, rows, sh, partial, stats, st, gate, chunk0, 0);
+        ma, mb, rows, sh, partial, stats, st, gate, chunk0, refused, give_up, 0);
     FB_LAUNCHED("split_gram_kernel");
     return FB_OK;
 }
@@ -793,6 +901,7 @@ SplitShape split_shape(int64_t rows, int kA, int kB, bool hermitian) {
     sh.nt_a = (kA + 63) / 64;
     sh.nt_b = (kB + 63) / 64;
     sh.hermitian = hermitian ? 1 : 0;
+    sh.screened = hermitian ? kA : kA + kB;
     sh.ntiles = hermitian ? sh.nt_a * (sh.nt_a + 1) / 2 : sh.nt_a * sh.nt_b;
     int smallest = sh.ntiles;
     if (hermitian && sh.nt_a > 1) smallest = std::min(sh.nt_a, sh.nt_a * (sh.nt_a - 1) / 2);
@@ -809,16 +918,26 @@ SplitLayout split_layout(const SplitShape& sh) {
     SplitLayout L{};
     const size_t parts = (size_t)sh.ntiles * (size_t)(sh.nchunks > 0 ? sh.nchunks : 1);
     L.verdict = 0;
-    L.sums = align_up((size_t)sh.ntiles * sizeof(int), 256);
+    L.refused = align_up((size_t)sh.ntiles * sizeof(int), 256);
+    L.sums = L.refused + align_up((size_t)SPLIT_SCREEN_PARTS * sh.screened * sizeof(int), 256);
     L.stats = L.sums + (size_t)sh.ntiles * SPLIT_TILE_DOUBLES * sizeof(double);
     L.partial = align_up(L.stats + parts * sizeof(SplitStat), 256);
     L.total = L.partial + parts * SPLIT_TILE_DOUBLES * sizeof(double);
     return L;
 }
 
+int split_screen_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
+                         const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st, int gate) {
+    int* refused = reinterpret_cast<int*>(static_cast<char*>(workspace) + split_layout(sh).refused);
+    split::split_screen_kernel<<<SPLIT_SCREEN_PARTS * sh.screened, split::SCREEN_THREADS, 0, stream>>>(A, lda, B, ldb, rows, sh, kA, refused,
+                                                                                  st, gate);
+    FB_LAUNCHED("split_screen_kernel");
+    return FB_OK;
+}
+
 int split_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA, int kB,
                            const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st, int gate,
-                           int chunk0, int chunk1) {
+                           int chunk0, int chunk1, bool screened, bool strict) {
     if (chunk0 < 0) chunk0 = 0;
     if (chunk1 > sh.nchunks) chunk1 = sh.nchunks;
     if (chunk0 >= chunk1) return FB_OK;
@@ -830,21 +949,26 @@ int split_partials_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb,
     FB_TRY(encode_panel_map(&ma, A, rows, kA, lda, 64));
     if (sh.hermitian) mb = ma;
     else FB_TRY(encode_panel_map(&mb, B, rows, kB, ldb, 64));
+    const int* refused = screened ? reinterpret_cast<const int*>(ws + L.refused) : nullptr;
+    const int give_up = strict ? 0 : 1;
     const int full = sh.hermitian ? sh.ntiles - sh.nt_a : sh.ntiles;
     if (sh.hermitian)
-        FB_TRY(split::launch<false>(ma, mb, rows, sh, sh.nt_a, partial, stats, stream, st, gate, chunk0, chunk1));
+        FB_TRY(split::launch<false>(ma, mb, rows, sh, sh.nt_a, partial, stats, stream, st, gate, chunk0, chunk1, refused,
+                                    give_up));
     if (full > 0)
-        FB_TRY(split::launch<true>(ma, mb, rows, sh, full, partial, stats, stream, st, gate, chunk0, chunk1));
+        FB_TRY(split::launch<true>(ma, mb, rows, sh, full, partial, stats, stream, st, gate, chunk0, chunk1, refused,
+                                   give_up));
     return FB_OK;
 }
 
 int split_sum_enqueue(int64_t rows, const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st,
-                      int gate) {
+                      int gate, bool screened) {
     const SplitLayout L = split_layout(sh);
     char* ws = static_cast<char*>(workspace);
     split::split_sum_kernel<<<dim3(129, (unsigned)sh.ntiles), split::SUM_THREADS, 0, stream>>>(
         sh, rows, reinterpret_cast<const double*>(ws + L.partial), reinterpret_cast<const SplitStat*>(ws + L.stats),
-        reinterpret_cast<double*>(ws + L.sums), reinterpret_cast<int*>(ws + L.verdict), st, gate);
+        reinterpret_cast<double*>(ws + L.sums), reinterpret_cast<int*>(ws + L.verdict), st, gate,
+        screened ? reinterpret_cast<const int*>(ws + L.refused) : nullptr);
     FB_LAUNCHED("split_sum_kernel");
     return FB_OK;
 }

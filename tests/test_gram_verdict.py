@@ -20,7 +20,8 @@ PAIRS = [(0, 0), (0, 1), (1, 2), (3, 8), (5, 40), (17, 30), (20, 21), (35, 34)]
 
 
 def gram(fb, backend, A, B=None):
-    """G and the verdict of every output tile (the first words of the workspace)."""
+    """G, the verdict of every output tile (the first words of the workspace) and
+    what the screen refused (four words a column from the next 256 bytes on)."""
     vp = ctypes.c_void_p
     Ad = backend.todevice(np.asfortranarray(A))
     Bd = Ad if B is None else backend.todevice(np.asfortranarray(B))
@@ -35,7 +36,9 @@ def gram(fb, backend, A, B=None):
     fb._lib.call("fb_sync_all")
     na, nb = -(-Ad.cols // 64), -(-Bd.cols // 64)
     words = ws.to_host().view(np.int32).ravel()
-    return C.to_host(), words[:na * (na + 1) // 2 if B is None else na * nb]
+    tiles = na * (na + 1) // 2 if B is None else na * nb
+    screen = -(-tiles // 64) * 64
+    return C.to_host(), words[:tiles], words[screen:screen + 4 * (Ad.cols if B is None else Ad.cols + Bd.cols)]
 
 
 def errors(G, A, B, pairs):
@@ -77,9 +80,9 @@ def test_flat_columns_are_accepted(fb, backend, kind, N, kA, kB):
     rng = np.random.default_rng(N + kA)
     A = flat(kind, rng, N, kA)
     B = A if kB is None else flat(kind, rng, N, kB)
-    G, verdict = gram(fb, backend, A, None if kB is None else B)
+    G, verdict, screen = gram(fb, backend, A, None if kB is None else B)
     if kind != "zeros" or (N, kA, kB) == (300_000, 64, None):
-        assert not verdict.any()
+        assert not screen.any() and not verdict.any()
     pairs = [p for p in PAIRS + [(kA - 1, B.shape[1] - 2), (kA - 1, 2)] if 3 not in p]
     assert errors(G, A, B, pairs)[0] <= 8 * EPS
 
@@ -107,7 +110,7 @@ def test_columns_that_share_no_rows_at_their_scale_are_refused(fb, backend, kind
     rng = np.random.default_rng(N + kA)
     A = graded(kind, rng, N, kA, 0)
     B = A if kB is None else graded(kind, rng, N, kB, 0)
-    G, verdict = gram(fb, backend, A, None if kB is None else B)
+    G, verdict, _ = gram(fb, backend, A, None if kB is None else B)
     assert verdict.any()
     assert errors(G, A, B, PAIRS)[1] <= 4 * EPS * np.sqrt(N)
 
@@ -124,5 +127,53 @@ def test_the_norm_a_scale_asks_for(fb, backend, modulus, accepted, same):
     A = wave()
     A[:, 5] *= modulus
     A[1_000, 5] = 20.0
-    G, verdict = gram(fb, backend, A, None if same else wave())
+    G, verdict, _ = gram(fb, backend, A, None if same else wave())
     assert bool(verdict.any()) != accepted
+
+
+def uneven(kind, rng, N, k):
+    r, j = np.arange(N)[:, None] / N, np.arange(1, k + 1)[None, :]
+    if kind == "sines":
+        return np.sin(np.pi * j * r) * (1 + 0.5j)
+    if kind == "envelopes":
+        return gaussian(rng, N, k) * np.exp(-(r - j / (k + 1)) ** 2 / (2 * 0.02 ** 2))
+    if kind == "heavy tails":
+        return gaussian(rng, N, k) / np.sqrt(rng.random((N, k)))
+    if kind == "sparse":
+        return gaussian(rng, N, k) * (rng.random((N, k)) < 0.2)
+    X = gaussian(rng, N, k)      # "one": a single column of them all
+    X[:, k - 1] *= rng.random(N) < 0.2
+    return X
+
+
+@pytest.mark.parametrize("kind", ["sines", "envelopes", "heavy tails", "sparse", "one"])
+@pytest.mark.parametrize("N,kA,kB", [(300_000, 64, None), (250_007, 48, 64), (300_017, 70, None)])
+def test_what_slices_are_slow_on_is_refused_by_its_sample(fb, backend, kind, N, kA, kB):
+    rng = np.random.default_rng(N + kA)
+    A = uneven(kind, rng, N, kA)
+    B = A if kB is None else gaussian(rng, N, kB) if kind == "one" else uneven(kind, rng, N, kB)
+    G, verdict, screen = gram(fb, backend, A, None if kB is None else B)
+    assert screen.any() and verdict.all()
+    if kind == "one":
+        assert np.flatnonzero(screen)[0] >= 4 * (kA - 1)
+    assert errors(G, A, B, PAIRS)[1] <= 4 * EPS * np.sqrt(N)
+
+
+@pytest.mark.parametrize("spiked,accepted", [(8, True), (64, False)])
+@pytest.mark.parametrize("same", [True, False])
+def test_a_chunk_whose_scales_keep_growing_is_left_to_fp64(fb, backend, spiked, accepted, same):
+    # Entries of 20 among waves of modulus 1, each in another stage of one chunk
+    # and past the sampled rows: a new epoch each, 16 at most.
+    rng = np.random.default_rng(8)
+    N, k, chunk, rows = 300_000, 64, 5, 2032
+    wave = lambda: np.exp(2j * np.pi * rng.random((N, k)))
+    A, B = wave(), wave()
+    half = (rows - 16) // 2
+    sampled = {o + i for r in (1, 2) for i in range(16)
+               for o in [(r - 1) * half + (((4 * chunk + r) * 2654435761 % 2 ** 32) * half >> 32)]}
+    free = [s for s in range(17, rows - 32, 16) if s not in sampled]
+    for j in range(spiked):
+        A[chunk * rows + free[j], j] = 20.0
+    G, verdict, screen = gram(fb, backend, A, None if same else B)
+    assert not screen.any() and bool(verdict.any()) != accepted
+    assert errors(G, A, A if same else B, PAIRS)[1] <= 4 * EPS * np.sqrt(N)
