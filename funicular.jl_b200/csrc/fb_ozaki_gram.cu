@@ -253,6 +253,9 @@ __device__ __forceinline__ bool screened_off(const int* __restrict__ refused, co
 //   when a chunk's later runs exceed its first by 4 or more: a scale set by
 //   the first 16 rows holds 2.6 times their maximum, and each time a column
 //   outgrows its scale the accumulators are drained;
+//   when its real or its imaginary part stays under 2^-5 of the other: one sum of
+//   both parts carries Re and Im of a folded tile, and what is left out of it
+//   would show in the smaller of them (the Gram of real columns has no Im at all);
 //   at numbers that are not finite or whose products could leave the range.
 // The choice of the runs depends on the shape alone. Gaussian columns pass with
 // a few runs in a hundred under the line and all but never a fourfold maximum.
@@ -272,11 +275,11 @@ split_screen_kernel(const z64* __restrict__ A, int64_t lda, const z64* __restric
     const int c = blockIdx.x / SPLIT_SCREEN_PARTS, part = blockIdx.x % SPLIT_SCREEN_PARTS;
     const int nchunks = (sh.nchunks - part + SPLIT_SCREEN_PARTS - 1) / SPLIT_SCREEN_PARTS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const z64* x = c < kA ? A + (int64_t)c * lda : B + (int64_t)(c - kA) * ldb;
-    __shared__ uint32_t most;
+    __shared__ uint32_t most[2];
     __shared__ int low, runs, grown;
-    if (threadIdx.x == 0) { most = 0; low = runs = grown = 0; }
+    if (threadIdx.x == 0) { most[0] = most[1] = 0; low = runs = grown = 0; }
     __syncthreads();
-    uint32_t all = 0;
+    uint32_t all[2] = {0, 0};     // the largest real and imaginary part
     int wlow = 0, wruns = 0, wgrown = 0, wgraded = 0;
     for (int k0 = warp; k0 < nchunks; k0 += BATCH * WARPS) {
         z64 v[BATCH][2];
@@ -300,9 +303,13 @@ split_screen_kernel(const z64* __restrict__ A, int64_t lda, const z64* __restric
             if (k0 + q * WARPS >= nchunks) break;
             uint32_t m[2];
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                m[h] = max((uint32_t)__double2hiint(v[q][h].x) & 0x7FFFFFFFu,
-                           (uint32_t)__double2hiint(v[q][h].y) & 0x7FFFFFFFu);
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t re = (uint32_t)__double2hiint(v[q][h].x) & 0x7FFFFFFFu;
+                const uint32_t im = (uint32_t)__double2hiint(v[q][h].y) & 0x7FFFFFFFu;
+                m[h] = max(re, im);
+                all[0] = max(all[0], re);
+                all[1] = max(all[1], im);
+            }
             const uint32_t first = __reduce_max_sync(0xffffffffu, lane < 16 ? m[0] : 0u);
             const uint32_t top = __reduce_max_sync(0xffffffffu, max(m[0], m[1]));
             if (top == 0) continue;   // a chunk of zeros is exact
@@ -314,19 +321,20 @@ split_screen_kernel(const z64* __restrict__ A, int64_t lda, const z64* __restric
             const uint32_t deep = top > (10u << 20) ? top - (10u << 20) : 1u;
             const uint32_t d0 = __ballot_sync(0xffffffffu, m[0] < deep), d1 = __ballot_sync(0xffffffffu, m[1] < deep);
             wgraded += ((d0 & 0xFFFFu) != 0) + ((d0 >> 16) != 0) + ((d1 & 0xFFFFu) != 0) + ((d1 >> 16) != 0) >= 2;
-            all = max(all, top);
         }
     }
+    for (int p = 0; p < 2; ++p) all[p] = __reduce_max_sync(0xffffffffu, all[p]);
     if (lane == 0) {
-        atomicMax(&most, all);
+        for (int p = 0; p < 2; ++p) atomicMax(&most[p], all[p]);
         atomicAdd(&low, wlow);
         atomicAdd(&runs, wruns);
         atomicAdd(&grown, wgrown + wgraded);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        const int e = (int)(most >> 20) - 1023;
-        refused[blockIdx.x] = most != 0 && (4 * low > runs || grown > 0 || e < -440 || e > 440);
+        const uint32_t top = max(most[0], most[1]), other = min(most[0], most[1]);
+        const int e = (int)(top >> 20) - 1023;
+        refused[blockIdx.x] = top != 0 && (4 * low > runs || grown > 0 || other + (5u << 20) < top || e < -440 || e > 440);
     }
 }
 

@@ -177,3 +177,30 @@ def test_a_chunk_whose_scales_keep_growing_is_left_to_fp64(fb, backend, spiked, 
     G, verdict, screen = gram(fb, backend, A, None if same else B)
     assert not screen.any() and bool(verdict.any()) != accepted
     assert errors(G, A, A if same else B, PAIRS)[1] <= 4 * EPS * np.sqrt(N)
+
+
+@pytest.mark.parametrize("N,kA,kB", [(300_000, 64, None), (300_017, 130, None), (250_001, 64, 48)])
+def test_the_gram_of_real_columns_is_real(fb, backend, N, kA, kB):
+    rng = np.random.default_rng(N + kA)
+    real = lambda k: (0.5 + rng.random((N, k))) * rng.choice([-1.0, 1.0], (N, k)) + 0j
+    A = real(kA)
+    B = A if kB is None else real(kB)
+    G, _, _ = gram(fb, backend, A, None if kB is None else B)
+    assert not G.imag.any()
+    assert errors(G, A, B, PAIRS)[1] <= 4 * EPS * np.sqrt(N)
+
+
+@pytest.mark.parametrize("small", [2.0 ** -20, 2.0 ** -40])
+def test_a_small_imaginary_part_keeps_its_digits(fb, backend, small):
+    # Im G_ij sums re_i im_j - im_i re_j: 2 N terms, against their own size.
+    rng = np.random.default_rng(12)
+    N, k = 300_000, 64
+    A = 0.5 + rng.random((N, k)) + 1j * small * (0.5 + rng.random((N, k)))
+    G, _, _ = gram(fb, backend, A)
+    L = np.longdouble
+    for i, j in PAIRS + [(0, 63), (9, 60)]:
+        if i // 8 == j // 8:     # the folded 8 x 8 diagonal blocks of the FP64 form carry Re + Im
+            continue
+        ar, ai, br, bi = (np.asarray(v, dtype=L) for v in (A[:, i].real, A[:, i].imag, A[:, j].real, A[:, j].imag))
+        exact, size = (ar * bi).sum() - (ai * br).sum(), float((ar * bi).sum() + (ai * br).sum())
+        assert abs(float(L(G[i, j].imag) - exact)) <= 4 * EPS * np.sqrt(2 * N) * size
