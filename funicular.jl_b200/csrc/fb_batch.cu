@@ -213,7 +213,7 @@ struct GramSet {
 // & 3) + 0/1), an off-diagonal block Re then Im (4 doubles).
 template <int NB, int G0>
 __device__ __forceinline__ void gram_kstep(const unsigned char* p, int odelta, unsigned long long flip,
-                                           double (&acc)[GramSet<NB, G0>::NACC]) {
+                                           double (&acc)[GramSet<NB, G0>::NACC], uint32_t& seen) {
     using S = GramSet<NB, G0>;
     constexpr int BLK = 8 * pb_col_bytes(NB);   // bytes from one 8-column block to the next
     double own[S::NO];
@@ -221,6 +221,9 @@ __device__ __forceinline__ void gram_kstep(const unsigned char* p, int odelta, u
     for (int b = 0; b < S::NO; ++b) own[b] = *reinterpret_cast<const double*>(p + (S::R0 + b) * BLK);
     const double aim0 = __longlong_as_double(
         __double_as_longlong(*reinterpret_cast<const double*>(p + S::R0 * BLK + odelta)) ^ flip);
+#pragma unroll
+    for (int b = 0; b < S::NO; ++b) mark_loaded(seen, own[b]);
+    mark_loaded(seen, aim0);
     dmma_884(acc[0], acc[1], own[0] + aim0, own[0]);
 #pragma unroll
     for (int j = 0; j < S::OFF0; ++j) {
@@ -232,6 +235,7 @@ __device__ __forceinline__ void gram_kstep(const unsigned char* p, int odelta, u
         const double are1 = own[D1];
         const double aim1 = __longlong_as_double(
             __double_as_longlong(*reinterpret_cast<const double*>(p + S::R1 * BLK + odelta)) ^ flip);
+        mark_loaded(seen, aim1);
         dmma_884(acc[S::B1], acc[S::B1 + 1], are1 + aim1, are1);
 #pragma unroll
         for (int j = 0; j < S::OFF1; ++j) {
@@ -251,10 +255,12 @@ struct GramCtx {
     z64* out;           // this chunk's partial: npairs blocks of 64 entries
     bool ok;            // every stage arrived
     int bad_site;       // the wait that gave up, if one did
+    int zero;           // 0, which the compiler does not know (mark_loaded)
 };
 
 // Waits for each stage of the chunk in turn, lets `work` multiply it, and
-// hands the slot back. The k-steps of the chunk (SR / 2 a stage) are dealt to the
+// hands the slot back, through an address that depends on all it read, which
+// work returns marked (mark_loaded). The k-steps of the chunk (SR / 2 a stage) are dealt to the
 // WPG warps of a set in turn, h, h + WPG, ..., across stage boundaries; work
 // gets the stage and its first k-step for this warp. A stage whose wait gave
 // up is skipped (ok = false), but the loop still runs to the end so every
@@ -282,9 +288,10 @@ __device__ __forceinline__ void gram_stages(GramCtx& c, uint32_t& full_par, int 
             fence_proxy_async_all();
             compute_sync();
         }
-        if (got) work(base, q0, (valid + 7) / 8 * 4);
+        uint32_t seen = 0;
+        if (got) seen = work(base, q0, (valid + 7) / 8 * 4);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&c.empty[slot]);
+        if (lane == 0) mbar_arrive(&c.empty[slot + (seen & c.zero)]);
         if (++slot == c.nslots) slot = 0;
         q0 = (q0 + SR / 2 * WPG - SR / 2) % WPG;
     }
@@ -307,8 +314,10 @@ __device__ void gram_warp(GramCtx& c, uint32_t& full_par) {
     for (int i = 0; i < S::NACC; ++i) acc[i] = 0.0;
     gram_stages<WPG, SR>(c, full_par, h, [&](const unsigned char* base, int q0, int nq) {
         const unsigned char* p = base + lane_off;
+        uint32_t seen = 0;
 #pragma unroll (NB <= 4 ? 4 : 2)
-        for (int q = q0; q < nq; q += WPG) gram_kstep<NB, G0>(p + (q >> 2) * 128 + (q & 3) * 16, odelta, flip, acc);
+        for (int q = q0; q < nq; q += WPG) gram_kstep<NB, G0>(p + (q >> 2) * 128 + (q & 3) * 16, odelta, flip, acc, seen);
+        return seen;
     });
     // The ring is free once every multiplying warp is past its last stage.
     double* comb = reinterpret_cast<double*>(c.ring);
@@ -777,7 +786,8 @@ struct PbRing {
 
 // The ring of a job over the rows of `chunk` (stage height and slot count by
 // the instance's width).
-__device__ GramCtx ring_ctx(const PbInst& I, int chunk, unsigned char* smem, const PbRing& ring, bool solve) {
+__device__ GramCtx ring_ctx(const PbInst& I, int chunk, unsigned char* smem, const PbRing& ring, bool solve,
+                            int zero) {
     const int kp = pb_kp(I.k);
     const bool small = I.k <= PB_STAGED_SOLVE_KMAX;
     GramCtx c;
@@ -794,6 +804,7 @@ __device__ GramCtx ring_ctx(const PbInst& I, int chunk, unsigned char* smem, con
     c.out = nullptr;
     c.ok = true;
     c.bad_site = 0;
+    c.zero = zero;
     return c;
 }
 
@@ -824,7 +835,7 @@ __device__ bool gram_job(const PbArgs& a, const PbInst& I, int pass, int chunk, 
     __syncthreads();
     if (!s_skip) {
         const int k = I.k;
-        GramCtx c = ring_ctx(I, chunk, smem, ring, false);
+        GramCtx c = ring_ctx(I, chunk, smem, ring, false, a.zero);
         c.out = reinterpret_cast<z64*>(I.scratch + pb_layout(k, I.nchunks).partial) + (size_t)chunk * pb_npairs(k) * 64;
         // Padding columns past k read as zero: no copy writes them.
         if (k < c.kp) {
@@ -902,7 +913,7 @@ __device__ void solve_job(const PbArgs& a, const PbInst& I, int slot, int pass, 
             for (int e = tid; e < n / 2; e += blockDim.x) reinterpret_cast<double2*>(frag)[e] = __ldcg(src + e);
             cached = key;
         }
-        GramCtx c = ring_ctx(I, chunk, smem, ring, true);
+        GramCtx c = ring_ctx(I, chunk, smem, ring, true, a.zero);
         if (path == PATH_INVERSE && k <= PB_STAGED_SOLVE_KMAX) {
             fence_proxy_async_all();
             __syncthreads();

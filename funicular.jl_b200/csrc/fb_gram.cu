@@ -253,6 +253,10 @@ gram_dmma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             if (!mbar_wait(&full[b], phase)) { ok = false; break; }
             const unsigned char* sa = smem + (size_t)b * ln.stage_bytes;
             const unsigned char* sbb = ln.diag ? sa : sa + GS_BOXES * box_a;
+            // This loop stays rolled. Every product of a box then issues, with
+            // its operands arrived, before the loop is left, and so before the
+            // slot is given back below: no mark_loaded here (marking the values
+            // cost 6 %, the sums 1 to 3).
 #pragma unroll 1
             for (int g = 0; g < GS_BOXES; ++g) {
                 const unsigned char* ba = sa + g * box_a;

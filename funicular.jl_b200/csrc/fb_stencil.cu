@@ -118,6 +118,7 @@ laplace7_tiled_kernel(const __grid_constant__ CUtensorMap tm, z64* __restrict__ 
     cur = point(1, 0);
     uint32_t seen = 0;
     mark_loaded(seen, below.x);
+    mark_loaded(seen, cur.x);
     __syncwarp();
     if (tx == 0) mbar_arrive(&empty[seen & zero]);
     int b = 1, nb = 2;
@@ -132,6 +133,7 @@ laplace7_tiled_kernel(const __grid_constant__ CUtensorMap tm, z64* __restrict__ 
         mark_loaded(seen, r.x);
         mark_loaded(seen, d.x);
         mark_loaded(seen, u.x);
+        mark_loaded(seen, above.x);
         __syncwarp();
         if (tx == 0) mbar_arrive(&empty[b + (seen & zero)]);
         if (!ok) sx = __longlong_as_double(0x7ff8000000000000ll);   // a plane never came: no silent wrong answer
