@@ -29,7 +29,6 @@
 
 namespace fb {
 
-constexpr int TR_THREADS = 256;
 constexpr int TR_PREP_THREADS = 512;
 
 // Substitution for rows in [first, rows) step `stride`: the fallback.
