@@ -86,6 +86,30 @@ def alg_flops(N, k):
     return 16 * N * k * k  # 2 passes x (Hermitian Gram 4Nk^2 + TRSM 4Nk^2)
 
 
+def gram_in_slices(N, kA, kB, hermitian):
+    """Whether the library forms this Gram of Gaussian-like columns on the
+    integer tensor cores (gram_takes_split in csrc/fb_gram.cu, up to the 320
+    columns timed here): its FP64 flops then bound nothing."""
+    if hermitian:
+        return kA > 40 and N >= (300_000 if kA > 48 else 500_000)
+    blocks = -(-min(kA, 64) // 8) * -(-min(kB, 64) // 8)
+    return blocks >= 36 and N >= (250_000 if blocks >= 40 else 400_000)
+
+
+def gram_bound_ms(N, kA, kB, hermitian, hbm_gbs, fp64_tflops):
+    """The slower of reading the operands once and, where they run in FP64,
+    the products."""
+    read = 16 * N * (kA if hermitian else kA + kB) / (hbm_gbs * 1e6)
+    flops = 0 if gram_in_slices(N, kA, kB, hermitian) else (4 if hermitian else 8) * N * kA * kB
+    return max(read, flops / (fp64_tflops * 1e9))
+
+
+def step_bound_ms(N, k, hbm_gbs, fp64_tflops):
+    """Two passes of a Gram and a solve, one after the other, each at its own bound."""
+    solve = max(32 * N * k / (hbm_gbs * 1e6), 4 * N * k * k / (fp64_tflops * 1e9))
+    return 2 * (gram_bound_ms(N, k, k, True, hbm_gbs, fp64_tflops) + solve)
+
+
 def workload_config(N, k, extra=None):
     cfg = {
         "workload": f"cholqr2! device-resident, N={N}, k={k}, panel width {W_PANEL}, ComplexF64, "
@@ -452,7 +476,7 @@ def run_c1(args, fb, backend, torch, device, world, max_over_ranks, barrier, hbm
         pairs.append((a, b))
     pairs[-1][1].synchronize()
     ms = max_over_ranks(sum(a.elapsed_time(b) for a, b in pairs)) / args.steps
-    roof_ms = max(alg_bytes(N, k) / (hbm_peak * 1e9), alg_flops(N, k) / (fp64_peak * 1e12)) * 1e3
+    roof_ms = step_bound_ms(N, k, hbm_peak, fp64_peak)
     record = {
         "workload": f"cholqr2! of PanelMatrix{{ComplexF64}} N={N}, k={k}, panel width {w}, copied from "
                     f"GhostPanels seed {C1_SEED:#x} (device fill)",
@@ -466,7 +490,7 @@ def run_c1(args, fb, backend, torch, device, world, max_over_ranks, barrier, hbm
     return record, (A, Q, R)
 
 
-def run_wide(args, fb, backend, torch, device, world, max_over_ranks, barrier, fp64_peak):
+def run_wide(args, fb, backend, torch, device, world, max_over_ranks, barrier, hbm_peak, fp64_peak):
     """The wide configuration: plain FP64 cholqr2! at N = args.wide_N (10^7),
     k = 128, on Y = U diag(s) V^H with condition numbers 1e4 and 1e7 (s
     log-spaced). The triangular solves go by 64-column blocks. Each kappa: one
@@ -500,10 +524,10 @@ def run_wide(args, fb, backend, torch, device, world, max_over_ranks, barrier, f
         b.record(stream)
         b.synchronize()
         ms = max_over_ranks(a.elapsed_time(b) / args.steps)
-        bound_ms = alg_flops(N, k) / (fp64_peak * 1e12) * 1e3
+        bound_ms = step_bound_ms(N, k, hbm_peak, fp64_peak)
         out["runs"].append({"kappa": kappa, "passes": passes, "ms_per_step": ms,
                             "value": whole_job_gbs(alg_bytes(N, k), world, ms), "unit": UNIT,
-                            "tflops": alg_flops(N, k) / (ms * 1e-3) / 1e12, "fp64_roofline_frac": bound_ms / ms,
+                            "tflops": alg_flops(N, k) / (ms * 1e-3) / 1e12, "ms_roofline": bound_ms, "frac": bound_ms / ms,
                             "orthogonality_fro": orth, "orthogonality_fro_cublas": orth_cublas,
                             "reconstruction_rel": recon})
         del Yt, Y
@@ -718,7 +742,7 @@ def run_project(args, fb, backend, torch, device, world, max_over_ranks, barrier
     ms_gram = timed(lambda: fb.kernels.gram_accumulate(backend, S, Q, Z, 1.0, 0.0))
     ms_both = timed(lambda: (G.apply(backend, Z, Q), fb.kernels.gram_accumulate(backend, S, Q, Z, 1.0, 0.0)))
     flops, nbytes = 8 * N * k * k, 32 * N * k
-    roof_ms = max(nbytes / (hbm_peak * 1e9), flops / (fp64_peak * 1e12)) * 1e3
+    roof_ms = gram_bound_ms(N, k, k, False, hbm_peak, fp64_peak)
     # End to end through the public API.
     Qh = np.asfortranarray(Q.to_host())
     del Q, Z
@@ -1140,12 +1164,11 @@ def run_ours(args):
         "peak_source": "cuBLAS ZGEMM 4096^3 measured in this run (FP64 has no entry in MEASURED_PEAKS.json)",
         "per_launch": f"4 N k^2 = {kernel_flops:.3e} flops per launch",
     }
-    step_flops_bound = alg_flops(N, k) / (fp64_peak * 1e12) * 1e3
-    step_bytes_bound = alg_bytes(N, k) / (hbm_peak * 1e9) * 1e3
+    step_ms = step_bound_ms(N, k, hbm_peak, fp64_peak)
     step_roofline = {
-        "ms_fp64_bound": step_flops_bound, "ms_hbm_bound": step_bytes_bound,
-        "ms_roofline": max(step_flops_bound, step_bytes_bound), "ms_measured": ms_step,
-        "frac": max(step_flops_bound, step_bytes_bound) / ms_step,
+        "ms_gram_bound": gram_bound_ms(N, k, k, True, hbm_peak, fp64_peak),
+        "gram_bound": "hbm" if gram_in_slices(N, k, k, True) else "fp64 or hbm",
+        "ms_roofline": step_ms, "ms_measured": ms_step, "frac": step_ms / ms_step,
         "achieved_tflops": alg_flops(N, k) / (ms_step * 1e-3) / 1e12,
         "hbm_peak_gbs": hbm_peak, "hbm_peak_source": hbm_source, "fp64_peak_tflops": fp64_peak,
     }
@@ -1160,7 +1183,7 @@ def run_ours(args):
 
     c1, c1_outputs = section(run_c1, hbm_peak, fp64_peak) if args.c1_N > 0 else (None, None)
     batched = section(run_batched, hbm_peak, fp64_peak) if args.batch > 0 else None
-    wide = section(run_wide, fp64_peak) if args.wide_N > 0 else None
+    wide = section(run_wide, hbm_peak, fp64_peak) if args.wide_N > 0 else None
     if wide is not None and args.e2e_steps > 0:
         wide["storage"] = section(run_wide_storage)
     range_finder = section(run_range_finder) if args.rf_k > 0 else None
