@@ -7,11 +7,15 @@ kernels:
 
 - the Gram's row-chunk count (its tile shape along the rows), a shift of the
   built-in one-wave count held in the library's own table
-  (fb_tune_set_gram_chunks), which every Gram launch of that class reads:
-  the FP64 Gram of gram_accumulate!, of both cholqr2! forms' FP64 passes, of
-  the batch and of the pullbacks;
+  (fb_tune_set_gram_chunks), which every FP64 Gram launch of that class
+  reads: those of gram_accumulate!, of cholqr2!, of the stream lanes and of the
+  pullbacks. Where the library forms the Gram on the integer tensor cores
+  (tall products of more than 40 columns) the chunks are its own, the
+  candidates time alike and the built-in count stays;
 - the form of the device-resident cholqr2! ("fp64" or "tc", k <= 64), read
-  by kernels.cholqr2_resident(form="auto");
+  by kernels.cholqr2_resident(form="auto"). At those sizes the two differ by
+  the check on the integer sums and the FP64 kernels behind it only, some 20 us
+  a pass;
 - the number of stream lanes a batch of cholqr2! instances is spread over
   (fb_tune_set_batch_lanes), timed on the caller's own batch.
 

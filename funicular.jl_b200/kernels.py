@@ -175,8 +175,11 @@ def cholqr2_resident(backend, Y: DeviceMatrix, R: DeviceMatrix, wait: bool = Tru
     """cholqr2! (src/panelblas.jl:130-139) on a matrix already in device
     memory: Y becomes Q in place and R (k x k) is written. With wait=True the
     call returns (passes, shifts) and raises if a Gram matrix stayed
-    indefinite; with wait=False it only enqueues. form="tc" computes the Gram
-    matrices on the integer tensor cores (k <= 64); form="shifted3" is the
+    indefinite; with wait=False it only enqueues. form="fp64" leaves it to the
+    library how a Gram is formed: on the integer tensor cores where it is tall
+    and wide and the device finds the result as accurate as FP64 sums, in FP64
+    otherwise. form="tc" takes the integer tensor cores for every Gram
+    (k <= 64), with no FP64 kernels behind them; form="shifted3" is the
     shifted CholeskyQR3 (pass 1 shifted by 11 (N k + k (k+1)) u ||G||_F with
     u = unit_roundoff, three passes); form="auto" takes the form the
     autotuner chose for this shape ("fp64" when untuned)."""
