@@ -781,8 +781,8 @@ split_gram_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // under the rounding of the FP64 sums themselves, when
 //     ||a_j||^2 >= 4^E_j max(21.4, 0.29 sqrt(N)).
 // These are root mean squares of roundings that do not know of one another; a
-// column of equal entries rounds alike in every row and has been seen off by
-// 2e-15 of the entry (its FP64 sums: 8e-14).
+// column of equal entries rounds alike in every row and is off by up to 4e-15
+// of the entry (its FP64 sums: 1e-13 at 3e5 rows, 1.5e-12 at 4e6).
 // The kernel knows ||a_j||^2 from the leading digits, whose rounding can raise
 // it by a third where they are small, so it checks 1.4 times that (N Gaussian
 // rows have at least about 2 N / 576).
