@@ -937,8 +937,8 @@ SplitLayout split_layout(const SplitShape& sh) {
 int split_screen_enqueue(const z64* A, int64_t lda, const z64* B, int64_t ldb, int64_t rows, int kA,
                          const SplitShape& sh, void* workspace, cudaStream_t stream, const ChainStatus* st, int gate) {
     int* refused = reinterpret_cast<int*>(static_cast<char*>(workspace) + split_layout(sh).refused);
-    split::split_screen_kernel<<<SPLIT_SCREEN_PARTS * sh.screened, split::SCREEN_THREADS, 0, stream>>>(A, lda, B, ldb, rows, sh, kA, refused,
-                                                                                  st, gate);
+    split::split_screen_kernel<<<SPLIT_SCREEN_PARTS * sh.screened, split::SCREEN_THREADS, 0, stream>>>(
+        A, lda, B, ldb, rows, sh, kA, refused, st, gate);
     FB_LAUNCHED("split_screen_kernel");
     return FB_OK;
 }
